@@ -956,6 +956,52 @@ int dq_tile_plan_dump(const char* json, size_t len, int tile_qubits, int fusion_
     });
 }
 
+int dq_rotation_plan_dump(const char* json, size_t len, int tile_qubits, char** out_text) {
+    return guard([&] {
+        need(json, "json");
+        need(out_text, "out_text");
+        uint64_t n = 0, ncb = 0;
+        auto ops = compile_json(json, len, &n, &ncb);
+        for (auto& op : ops)
+            if (!tileable(op)) fail(kValueError, "circuit has operations a tile pass cannot apply");
+        TilePlanOptions o;
+        o.m = tile_qubits;
+        o.beam = kPlanBeam;
+        o.keep_raw = true;
+        std::vector<double2> pool;
+        auto passes = plan_tiles(ops, 0, ops.size(), int(n), o, &pool);
+        std::string s = "{\"n\":" + std::to_string(n) + ",\"passes\":[";
+        auto list = [&](const char* name, auto begin, auto end) {
+            s += std::string(",\"") + name + "\":[";
+            for (auto i = begin; i != end; ++i) s += (i == begin ? "" : ",") + std::to_string(*i);
+            s += "]";
+        };
+        for (size_t pi = 0; pi < passes.size(); pi++) {
+            const TilePass& p = passes[pi];
+            RotProgram r;
+            const bool ok = build_rotation_pass(p.raw, p.qubits, int(n), r);
+            s += std::string(pi ? ",{" : "{") + "\"ok\":" + (ok ? "true" : "false") +
+                 ",\"raw\":" + std::to_string(p.raw_ops) + ",\"data\":" + std::to_string(r.data) + ",\"phases\":" + std::to_string(r.nphases) +
+                 ",\"rotations\":" + std::to_string(r.rotations) + ",\"tables\":" + std::to_string(r.tables) +
+                 ",\"slot_phases\":" + std::to_string(r.slot_phases) + ",\"out_const\":" +
+                 std::to_string(r.out_const) + ",\"sign_local\":" + std::to_string(r.sign_local) +
+                 ",\"sign_outer\":" + std::to_string(r.sign_outer) + ",\"sign_const\":" + std::to_string(r.sign_const);
+            list("qubits", p.qubits.begin(), p.qubits.end());
+            list("out_dir", r.out_dir, r.out_dir + r.m);
+            list("out_outer", r.out_outer, r.out_outer + kRotMaxOuter);
+            std::vector<uint32_t> flat;
+            for (const uint4& w : r.words) flat.insert(flat.end(), {w.x, w.y, w.z, w.w});
+            list("words", flat.begin(), flat.end());
+            s += "}";
+        }
+        s += "]}";
+        char* out = static_cast<char*>(std::malloc(s.size() + 1));
+        if (!out) throw std::bad_alloc();
+        std::memcpy(out, s.c_str(), s.size() + 1);
+        *out_text = out;
+    });
+}
+
 int dq_fused_plan_dump(const char* json, size_t len, char** out_text) {
     return guard([&] {
         need(json, "json");

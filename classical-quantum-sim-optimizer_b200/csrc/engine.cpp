@@ -356,7 +356,7 @@ double Executor::step_bytes(size_t i, const k::Batch& b) const {
     const Step& s = steps_[i];
     const double S = b.c64 ? 8.0 : 16.0;
     const double full = S * double(uint64_t(1) << b.n) * double(b.W);
-    if (s.pass >= 0 || s.fused >= 0) return 2.0 * full;
+    if (s.pass >= 0 || s.fused >= 0 || s.rot >= 0) return 2.0 * full;
     switch (s.type) {
         case Operation::One:
         case Operation::X: return 2.0 * full / double(uint64_t(1) << s.controls.size());
@@ -390,6 +390,10 @@ void Executor::arith_flops(const k::Batch& b, double* cuda_core, double* tensor)
         if (s.fused >= 0) {
             const FusedPass& p = fused_[size_t(s.fused)];
             tc += double(p.nblocks) * (amps / double(1 << kFusedM)) * 3.0 * 2.0 * 128.0 * 64.0 * 64.0;
+            continue;
+        }
+        if (s.rot >= 0) {
+            cc += amps * rots_[size_t(s.rot)].program.flops_per_amp;
             continue;
         }
         if (s.pass >= 0) {
@@ -531,18 +535,53 @@ void Executor::lower_segment(const std::vector<Operation>& ops, size_t begin, si
         }
         return;
     }
+    const bool rotations = cfg_.rotations && !cfg_.c64 && !cfg_.model;
+    o.keep_raw = rotations;
     std::vector<TilePass> ps = plan_tiles(ops, begin, end, cfg_.n, o, &pool_host_);
-    for (auto& p : ps) {
-        p.op_begin = int(tile_ops_host_.size());
-        tile_ops_host_.insert(tile_ops_host_.end(), p.ops.begin(), p.ops.end());
-        attach_phases(p);
+    if (!rotations) {
+        for (auto& p : ps) add_tile_pass(std::move(p));
+        return;
+    }
+    std::vector<RotProgram> programs(ps.size());
+    std::vector<char> ok(ps.size(), 0);
+    parallel_for(ps.size(), [&](size_t i) {
+        ok[i] = char(build_rotation_pass(ps[i].raw, ps[i].qubits, cfg_.n, programs[i]));
+    });
+    for (size_t i = 0; i < ps.size(); i++) {
+        TilePass& p = ps[i];
+        if (!ok[i]) {
+            lower_pass_ops(p.raw, p.qubits, cfg_.n, cfg_.fuse, pool_host_, p.ops);
+            p.raw.clear();
+            add_tile_pass(std::move(p));
+            continue;
+        }
+        RotStep r;
+        r.qubits = p.qubits;
+        r.raw_ops = p.raw_ops;
+        r.program = std::move(programs[i]);
+        if (r.program.words.size() > size_t(kRotParamWords)) {
+            r.words_at = rot_words_host_.size();
+            rot_words_host_.insert(rot_words_host_.end(), r.program.words.begin(), r.program.words.end());
+        }
         Step s;
-        s.pass = int(passes_.size());
+        s.rot = int(rots_.size());
         s.type = Operation::Dense;
         s.category = 1;
-        passes_.push_back(std::move(p));
+        rots_.push_back(std::move(r));
         steps_.push_back(std::move(s));
     }
+}
+
+void Executor::add_tile_pass(TilePass&& p) {
+    p.op_begin = int(tile_ops_host_.size());
+    tile_ops_host_.insert(tile_ops_host_.end(), p.ops.begin(), p.ops.end());
+    attach_phases(p);
+    Step s;
+    s.pass = int(passes_.size());
+    s.type = Operation::Dense;
+    s.category = 1;
+    passes_.push_back(std::move(p));
+    steps_.push_back(std::move(s));
 }
 
 void Executor::attach_phases(TilePass& p) {
@@ -652,6 +691,13 @@ void Executor::record_costs(const k::Batch& b, std::vector<float>& X, std::vecto
 size_t Executor::raw_ops_in_passes() const {
     size_t t = 0;
     for (auto& p : passes_) t += size_t(p.raw_ops);
+    for (auto& r : rots_) t += size_t(r.raw_ops);
+    return t;
+}
+
+size_t Executor::tile_ops() const {
+    size_t t = tile_ops_host_.size();
+    for (auto& r : rots_) t += size_t(r.program.rotations + r.program.tables + r.program.slot_phases);
     return t;
 }
 
@@ -747,6 +793,12 @@ void Executor::upload(cudaStream_t stream) {
                                    cudaMemcpyHostToDevice, stream),
                    "upload tile phases");
     }
+    if (!rot_words_host_.empty()) {
+        rot_words_.alloc(rot_words_host_.size() * sizeof(uint4), "rotation passes");
+        cuda_check(cudaMemcpyAsync(rot_words_.p, rot_words_host_.data(), rot_words_host_.size() * sizeof(uint4),
+                                   cudaMemcpyHostToDevice, stream),
+                   "upload rotation passes");
+    }
     if (!fused_blocks_host_.empty()) {
         fused_blocks_.alloc(fused_blocks_host_.size() * sizeof(FusedBlock), "fused block descriptors");
         upool_.alloc(upool_host_.size() * sizeof(uint16_t), "fused block gate images");
@@ -759,6 +811,16 @@ void Executor::upload(cudaStream_t stream) {
     }
     uploaded_ = true;
 }
+
+namespace {
+// A profiled pass counts as one many-qubit call (execution.rs:297-347).
+void finish_tile_step(ProfileAcc* profile, cudaStream_t stream, std::chrono::steady_clock::time_point t0) {
+    if (!profile) return;
+    cuda_check(cudaStreamSynchronize(stream), "stream synchronize");
+    profile->nq_calls++;
+    profile->nq_time += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+}
+}  // namespace
 
 void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, bool normalize, bool from_basis) {
     upload(b.stream);
@@ -818,9 +880,17 @@ void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, b
             }
             continue;
         }
-        if (s.pass >= 0) {
-            const TilePass& p = passes_[size_t(s.pass)];
+        if (s.pass >= 0 || s.rot >= 0) {
             if (rec) rec->begin(kcTile, step_bytes(si, b));
+            if (s.rot >= 0) {
+                const RotStep& r = rots_[size_t(s.rot)];
+                k::rotation_pass(b, r.qubits, r.program,
+                                 rot_words_.p ? rot_words_.as<uint4>() + r.words_at : nullptr, from_basis && si == 0);
+                if (rec) rec->end();
+                finish_tile_step(profile, b.stream, t0);
+                continue;
+            }
+            const TilePass& p = passes_[size_t(s.pass)];
             const int m = int(p.qubits.size());
             if (p.nphases > 0)
                 k::tile_pass_phased(b, p, p.nphases, phase_blocks_[size_t(p.phase_block)],
@@ -829,11 +899,7 @@ void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, b
                 k::tile_pass(b, nullptr, m, tile_ops_.as<TileOp>() + p.op_begin, int(p.ops.size()),
                              pool_.as<double2>(), p);
             if (rec) rec->end();
-            if (profile) {
-                cuda_check(cudaStreamSynchronize(b.stream), "stream synchronize");
-                profile->nq_calls++;
-                profile->nq_time += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-            }
+            finish_tile_step(profile, b.stream, t0);
             continue;
         }
         if (rec) {

@@ -12,6 +12,7 @@
 #include "compile.hpp"
 #include "kernels.hpp"
 #include "phased.hpp"
+#include "rotations.hpp"
 #include "tile.hpp"
 
 namespace dq {
@@ -136,6 +137,9 @@ struct ExecConfig {
     // tile-op cost model keep one operation per sweep, the form that model's
     // per-operation costs were recorded on.
     bool phased = true;
+    // complex128 passes run as Pauli rotations (rotations.hpp) wherever every
+    // operation of the pass has that form; the others in register phases.
+    bool rotations = false;
 };
 
 // How the fused plan of a segment was chosen: the portfolio's caps, the hand
@@ -161,11 +165,11 @@ class Executor {
     // of the norm, ~1e-7); for callers that only sample, which divides by the
     // total probability anyway.
     // `from_basis`: every state of the batch is |0...0> on entry; a first step
-    // that is a fused pass then builds its input tiles itself (the caller
-    // need not write the state first: starts_with_fused_pass()).
+    // that is a fused or a rotation pass then builds its input tiles itself
+    // (the caller need not write the state first: builds_basis()).
     void run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec = nullptr, bool normalize = true,
              bool from_basis = false);
-    bool starts_with_fused_pass() const { return !steps_.empty() && steps_[0].fused >= 0; }
+    bool builds_basis() const { return !steps_.empty() && (steps_[0].fused >= 0 || steps_[0].rot >= 0); }
     // Uploads the matrix pools and sizes the scratch a run over batches like
     // `b` needs, so that later runs allocate nothing and copy nothing from the
     // host (they can then be captured into a CUDA graph).
@@ -179,12 +183,12 @@ class Executor {
     // f16 tensor-core FLOPs the fused blocks issue.
     void arith_flops(const k::Batch& b, double* cuda_core, double* tensor) const;
 
-    size_t passes() const { return passes_.size() + fused_.size(); }
+    size_t passes() const { return passes_.size() + fused_.size() + rots_.size(); }
     size_t fused_blocks() const { return fused_blocks_host_.size(); }
     size_t raw_ops_in_passes() const;
     const std::vector<int>& chosen_widths() const { return widths_; }
     const std::vector<FusedPlanChoice>& fused_choices() const { return fused_choices_; }
-    size_t tile_ops() const { return tile_ops_host_.size(); }
+    size_t tile_ops() const;
     // Times every pass (CUDA events), shares each pass's time among its
     // operations by their clock64 cycles or equally among its tensor-core
     // blocks, and appends (features, log picoseconds per tile) samples.  Fused
@@ -196,6 +200,7 @@ class Executor {
     struct Step {
         int pass = -1;   // >= 0: a tile pass (index into passes_)
         int fused = -1;  // >= 0: a tensor-core fused pass (index into fused_)
+        int rot = -1;    // >= 0: a rotation pass (index into rots_)
         Operation::Type type;
         int target = 0, a = 0, b = 0;
         std::vector<k::Ctl> controls;
@@ -218,6 +223,15 @@ class Executor {
     std::vector<uint16_t> upool_host_;
     std::vector<std::vector<uint4>> phase_blocks_;  // per phased pass (host copies: launch arguments)
     std::vector<uint4> phase_words_host_;           // the same blocks back to back (device copy)
+    struct RotStep {
+        std::vector<int> qubits;
+        RotProgram program;
+        size_t words_at = 0;  // of its words in rot_words_host_ (programs larger than a launch argument)
+        int raw_ops = 0;
+    };
+    std::vector<RotStep> rots_;
+    std::vector<uint4> rot_words_host_;
+    DevMem rot_words_;
     DevMem pool_, tile_ops_, fused_blocks_, upool_, norm_tiles_, norm_states_, phase_words_;
     bool uploaded_ = false;
     ExecConfig cfg_;
@@ -226,6 +240,7 @@ class Executor {
     void upload(cudaStream_t stream);
     void lower(const Operation& op, std::vector<Condition>& conds);
     void lower_segment(const std::vector<Operation>& ops, size_t begin, size_t end);
+    void add_tile_pass(TilePass&& p);
     void attach_phases(TilePass& p);
 };
 

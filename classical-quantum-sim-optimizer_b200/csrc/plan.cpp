@@ -115,8 +115,8 @@ double Plan::run(bool record) {
     cuda_check(cudaEventCreate(&b), "cudaEventCreate");
     cuda_check(cudaEventRecord(a, s), "cudaEventRecord");
     k::Batch bt = st_.view(s, 1);
-    // |0...0>: written here, or built by a first fused pass in its tiles.
-    const bool built = ex_->starts_with_fused_pass();
+    // |0...0>: written here, or built by the first pass in its tiles.
+    const bool built = ex_->builds_basis();
     if (!built) k::init_basis(bt);
     cuda_check(cudaMemsetAsync(st_.cbits.p, 0, size_t(st_.cwords) * 8, s), "clear cbits");
     cuda_check(cudaMemsetAsync(st_.draws.p, 0, 8, s), "clear draws");
@@ -213,7 +213,16 @@ void Plan::record_costs(std::vector<float>& X, std::vector<float>& y) {
     std::lock_guard<std::mutex> lk(dev_->mu);
     dev_->activate();
     k::Batch bt = st_.view(dev_->stream, 1);
-    ex_->record_costs(bt, X, y);
+    // The model learns the cost of fused tile operations, which the default
+    // complex128 passes no longer are.
+    ExecConfig c = exec_config(opt_, n_);
+    if (!c.rotations) {
+        ex_->record_costs(bt, X, y);
+        return;
+    }
+    c.rotations = false;
+    Executor tiles(ops_, 0, (terminal_ && cdf_.p) ? prefix_end_ : ops_.size(), c);
+    tiles.record_costs(bt, X, y);
 }
 
 void Plan::samples(uint64_t* out) const {

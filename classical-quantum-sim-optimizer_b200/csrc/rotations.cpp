@@ -1,0 +1,1007 @@
+// Host planner of Pauli-rotation passes: gates -> relabellings, phases and
+// rotations -> phases of four register directions.
+#include "rotations.hpp"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+namespace dq {
+
+namespace {
+
+constexpr long double kPiL = 3.14159265358979323846264338327950288L;
+constexpr double kPi = double(kPiL);
+constexpr double kUnitaryTol = 1e-12;
+constexpr double kAngleTol = 2.3e-16;  // a quarter turn to the rounding of its angle
+constexpr int kMaxDiagQubits = 6;
+
+int parity64(uint64_t x) { return __builtin_parityll(x); }
+
+struct Item {
+    bool rot = false;
+    bool imag = false;   // rotation without the factor i (mu & v even)
+    uint32_t v = 0;      // rotation: direction (tile-local place bits)
+    uint64_t mask = 0;   // parity mask over place bits (tile-local below m, tile index above)
+    double t = 0.0;      // rotation: signed tangent
+    double a = 0.0;      // phase: angle
+    long double b = 0.0; // phase: logarithm of its modulus (factors e^(+-(b + ia)))
+};
+
+struct Unsupported {};
+
+double norm2(cplx z) { return z.re * z.re + z.im * z.im; }
+double arg(cplx z) { return std::atan2(z.im, z.re); }
+
+bool commute(const Item& x, const Item& y) {
+    if (!x.rot && !y.rot) return true;
+    int p = 0;
+    if (y.rot) p ^= parity64(x.mask & y.v);
+    if (x.rot) p ^= parity64(y.mask & x.v);
+    return p == 0;
+}
+
+// The gates of a pass as items, with the frame that relabels places.
+class Lowering {
+  public:
+    Lowering(const std::vector<int>& tile, int n) : m_(int(tile.size())) {
+        mask_.resize(size_t(n));
+        cons_.assign(size_t(n), 0);
+        dir_.assign(size_t(n), 0);
+        int outer = 0;
+        for (int q = 0, l = 0; q < n; q++) {
+            if (l < m_ && tile[size_t(l)] == q) {
+                mask_[size_t(q)] = uint64_t(1) << l;
+                dir_[size_t(q)] = 1u << l;
+                l++;
+            } else {
+                mask_[size_t(q)] = uint64_t(1) << (m_ + outer++);
+            }
+        }
+    }
+
+    void add(const Operation& op) {
+        switch (op.type) {
+            case Operation::One: one(op.target, op.m, op.controls); break;
+            case Operation::X: x(op.target, op.controls); break;
+            case Operation::Swap: swap(op.a, op.b, op.controls); break;
+            case Operation::Diagonal: diagonal(op); break;
+            case Operation::Dense: dense(op); break;
+            default: throw Unsupported{};
+        }
+    }
+
+    std::vector<Item> items;
+    // Sums hundreds of angles: a 64-bit mantissa keeps its rounding below the amplitudes'.
+    long double global = 0.0;  // phase of the whole state
+    uint64_t sign = 0;         // Z^sign still to be applied
+
+    const std::vector<uint64_t>& masks() const { return mask_; }
+    const std::vector<int>& consts() const { return cons_; }
+    const std::vector<uint32_t>& dirs() const { return dir_; }
+
+  private:
+    int m_;
+    std::vector<uint64_t> mask_;
+    std::vector<int> cons_;
+    std::vector<uint32_t> dir_;
+    std::vector<size_t> open_;  // phases that every later rotation commutes with
+
+    // exp(i a Z^mask (-1)^cons)
+    void phase(uint64_t mask, int cons, double a) {
+        if (cons) a = -a;
+        if (mask == 0) {
+            global += a;
+            return;
+        }
+        const double r = std::nearbyint(a / kPi);
+        a = double((long double)(a) - (long double)(r) * kPiL);
+        if (std::fmod(std::fabs(r), 2.0) == 1.0) global += kPiL;
+        if (a == 0.0) return;
+        if (std::fabs(std::fabs(a) - kPi / 2) <= kAngleTol) {  // +-i Z^mask
+            global += a > 0 ? kPiL / 2 : -kPiL / 2;
+            sign ^= mask;
+            return;
+        }
+        for (size_t i : open_)
+            if (items[i].mask == mask) {
+                items[i].a += a;
+                return;
+            }
+        Item it;
+        it.mask = mask;
+        it.a = a;
+        open_.push_back(items.size());
+        items.push_back(it);
+    }
+
+    // exp(-i theta/2 P) with (c, s) = (cos, sin)(theta/2), P the product over the
+    // qubits of X (bit of xs), Z (of zs) or Y (both).
+    void rotation(const std::vector<uint64_t>& xs, const std::vector<uint64_t>& zs, double c, double s) {
+        uint32_t v = 0;
+        uint64_t mask = 0;
+        int cons = 0, ny = 0;
+        for (uint64_t q : xs) {
+            if (dir_[size_t(q)] == 0) throw Unsupported{};  // a rotated qubit outside the tile
+            v ^= dir_[size_t(q)];
+        }
+        for (uint64_t q : zs) {
+            mask ^= mask_[size_t(q)];
+            cons ^= cons_[size_t(q)];
+            if (std::find(xs.begin(), xs.end(), q) != xs.end()) ny++;
+        }
+        const bool imag = ny % 2 == 0;
+        if ((ny / 2) % 2) cons ^= 1;  // i^ny = +-1 or +-i
+        if (c < 0) {
+            global += kPiL;
+            c = -c;
+            s = -s;
+        }
+        if (s == 0.0) return;
+        if (cons) s = -s;  // from here P = (i) X^v Z^mask
+        if (std::fabs(s) > c) {
+            // c - i s P = (-i P) (s + i c P): rotate by the complement, then apply P
+            // (the phases and rotations before see the place, so P comes last).
+            double c2 = s, s2 = -c;
+            if (c2 < 0) {
+                global += kPiL;
+                c2 = -c2;
+                s2 = -s2;
+            }
+            if (s2 != 0.0) emit(v, mask, imag, c2, s2);
+            if (imag) global -= kPiL / 2;
+            sign ^= mask;
+            for (size_t q = 0; q < mask_.size(); q++) cons_[q] ^= parity64(mask_[q] & v);
+            return;
+        }
+        emit(v, mask, imag, c, s);
+    }
+
+    void emit(uint32_t v, uint64_t mask, bool imag, double c, double s) {
+        Item it;
+        it.rot = true;
+        it.imag = imag;
+        it.v = v;
+        it.mask = mask;
+        it.t = s / c;
+        if (parity64(sign & v)) it.t = -it.t;
+        open_.erase(std::remove_if(open_.begin(), open_.end(),
+                                   [&](size_t i) { return parity64(items[i].mask & v) != 0; }),
+                    open_.end());
+        items.push_back(it);
+    }
+
+    // Phases phi[j] by the qubits' values (qubits[0] the MSB of j).
+    void phases(const std::vector<uint64_t>& qubits, std::vector<double> phi) {
+        const size_t k = qubits.size();
+        if (k > size_t(kMaxDiagQubits)) throw Unsupported{};
+        const size_t D = size_t(1) << k;
+        for (size_t h = 1; h < D; h <<= 1)
+            for (size_t i = 0; i < D; i++)
+                if (!(i & h)) {
+                    const double x = phi[i], y = phi[i | h];
+                    phi[i] = x + y;
+                    phi[i | h] = x - y;
+                }
+        for (size_t S = 0; S < D; S++) {
+            uint64_t mask = 0;
+            int cons = 0;
+            for (size_t b = 0; b < k; b++)
+                if ((S >> (k - 1 - b)) & 1) {
+                    mask ^= mask_[size_t(qubits[b])];
+                    cons ^= cons_[size_t(qubits[b])];
+                }
+            const double a = phi[S] / double(D);
+            if (a != 0.0) phase(mask, cons, a);
+        }
+    }
+
+    static void pattern(const std::vector<Control>& controls, std::vector<uint64_t>& qubits, size_t& index) {
+        index = 0;
+        for (const Control& c : controls) {
+            qubits.push_back(c.qubit);
+            index = (index << 1) | size_t(c.value);
+        }
+    }
+
+    // -1 where every control holds and `target` is 1.
+    void controlled_z(const std::vector<Control>& controls, uint64_t target) {
+        std::vector<uint64_t> q;
+        size_t j;
+        pattern(controls, q, j);
+        q.push_back(target);
+        std::vector<double> phi(size_t(1) << q.size(), 0.0);
+        phi[(j << 1) | 1] = kPi;
+        phases(q, phi);
+    }
+
+    void one(uint64_t target, const Mat2& u, const std::vector<Control>& controls) {
+        // u = e^{i alpha} RZ(beta) RY(theta) RZ(gamma)
+        const double c = std::sqrt(norm2(u[0][0])), s = std::sqrt(norm2(u[1][0]));
+        const double dev[] = {std::fabs(c * c + s * s - 1.0), std::fabs(norm2(u[0][1]) + norm2(u[1][1]) - 1.0),
+                              std::fabs(u[0][0].re * u[0][1].re + u[0][0].im * u[0][1].im + u[1][0].re * u[1][1].re +
+                                        u[1][0].im * u[1][1].im),
+                              std::fabs(u[0][0].re * u[0][1].im - u[0][0].im * u[0][1].re + u[1][0].re * u[1][1].im -
+                                        u[1][0].im * u[1][1].re)};
+        for (double d : dev)
+            if (!(d <= kUnitaryTol)) throw Unsupported{};
+        // Arguments of u00, u10 and u11; the fourth entry's follows from
+        // unitarity, so the smaller pair gives one argument only.
+        double A, B, D;
+        if (c >= s) {
+            A = arg(u[0][0]);
+            D = arg(u[1][1]);
+            B = s > 0 ? arg(u[1][0]) : A;
+        } else {
+            B = arg(u[1][0]);
+            const double C = arg(-u[0][1]);
+            A = c > 0 ? arg(u[0][0]) : B;
+            D = B + C - A;
+        }
+        double beta = B - A, gamma = D - B, alpha = A + (beta + gamma) / 2;
+        if (controls.empty()) {
+            global += alpha;
+            // RZ(-+pi/2) RY(theta) RZ(+-pi/2) = RX(+-theta)
+            const double turns = std::nearbyint((beta + gamma) / (2 * kPi));
+            const double quarter = std::fabs(std::remainder(beta, 2 * kPi));
+            if (s > 0 && std::fabs(beta + gamma - turns * 2 * kPi) <= 4 * kAngleTol &&
+                std::fabs(quarter - kPi / 2) <= 4 * kAngleTol) {
+                // RZ(gamma) = RZ(-beta) (-1)^turns; beta = +-pi/2 up to whole turns, which cancel in the pair.
+                if (std::fmod(std::fabs(turns), 2.0) == 1.0) global += kPiL;
+                rotation({target}, {}, c, std::remainder(beta, 2 * kPi) < 0 ? s : -s);
+                return;
+            }
+            phase(mask_[size_t(target)], cons_[size_t(target)], -gamma / 2);
+            rotation({target}, {target}, c, s);
+            phase(mask_[size_t(target)], cons_[size_t(target)], -beta / 2);
+            return;
+        }
+        std::vector<uint64_t> q;
+        size_t j;
+        pattern(controls, q, j);
+        const size_t nc = q.size();
+        std::vector<uint64_t> qt = q;
+        qt.push_back(target);
+        auto crz = [&](double angle) {
+            std::vector<double> phi(size_t(2) << nc, 0.0);
+            phi[j << 1] = -angle / 2;
+            phi[(j << 1) | 1] = angle / 2;
+            phases(qt, phi);
+        };
+        const double half = std::atan2(s, c) / 2;  // theta / 4
+        crz(gamma);
+        controlled_z(controls, target);
+        rotation({target}, {target}, std::cos(half), -std::sin(half));
+        controlled_z(controls, target);
+        rotation({target}, {target}, std::cos(half), std::sin(half));
+        crz(beta);
+        std::vector<double> phi(size_t(1) << nc, 0.0);
+        phi[j] = alpha;
+        phases(q, phi);
+    }
+
+    void cx(uint64_t c, bool value, uint64_t t) {
+        if (dir_[size_t(t)] == 0) throw Unsupported{};
+        mask_[size_t(t)] ^= mask_[size_t(c)];
+        cons_[size_t(t)] ^= cons_[size_t(c)] ^ (value ? 0 : 1);
+        if (dir_[size_t(c)]) dir_[size_t(c)] ^= dir_[size_t(t)];
+    }
+
+    void x(uint64_t target, const std::vector<Control>& controls) {
+        if (dir_[size_t(target)] == 0) throw Unsupported{};
+        if (controls.empty()) {
+            cons_[size_t(target)] ^= 1;
+        } else if (controls.size() == 1) {
+            cx(controls[0].qubit, controls[0].value, target);
+        } else {
+            const double r = std::sqrt(0.5);
+            auto h = [&] {  // H = RY(pi/2) Z
+                phase(mask_[size_t(target)], cons_[size_t(target)], -kPi / 2);  // -i Z
+                global += kPiL / 2;
+                rotation({target}, {target}, r, r);
+            };
+            h();
+            controlled_z(controls, target);
+            h();
+        }
+    }
+
+    void swap(uint64_t a, uint64_t b, const std::vector<Control>& controls) {
+        if (controls.empty()) {
+            if (dir_[size_t(a)] == 0 || dir_[size_t(b)] == 0) throw Unsupported{};
+            std::swap(mask_[size_t(a)], mask_[size_t(b)]);
+            std::swap(cons_[size_t(a)], cons_[size_t(b)]);
+            std::swap(dir_[size_t(a)], dir_[size_t(b)]);
+            return;
+        }
+        cx(b, true, a);
+        std::vector<Control> both = controls;
+        both.push_back({a, true});
+        x(b, both);
+        cx(b, true, a);
+    }
+
+    void diagonal(const Operation& op) {
+        std::vector<double> phi;
+        for (cplx d : op.values) {
+            if (!(std::fabs(norm2(d) - 1.0) <= kUnitaryTol)) throw Unsupported{};
+            phi.push_back(arg(d));
+        }
+        phases(op.qubits, phi);
+    }
+
+    // A one-qubit matrix, or cos I - i sin P for a two-qubit Pauli matrix P.
+    void dense(const Operation& op) {
+        if (op.qubits.size() == 1) {
+            Mat2 u;
+            for (int r = 0; r < 2; r++)
+                for (int c = 0; c < 2; c++) u[size_t(r)][size_t(c)] = op.values[size_t(2 * r + c)];
+            one(op.qubits[0], u, {});
+            return;
+        }
+        if (op.qubits.size() != 2) throw Unsupported{};
+        const uint64_t hi = op.qubits[0], lo = op.qubits[1];
+        for (int X = 1; X < 4; X++)      // bit 1: hi, bit 0: lo
+            for (int Z = 0; Z < 4; Z++) {
+                // P|j> = i^ny (-1)^{Z.j} |j ^ X>; entry (j ^ X, j) of the matrix is -i s times that.
+                const int ny = __builtin_popcount(unsigned(X & Z));
+                const double c = op.values[0].re;
+                auto factor = [&](int j) {  // -i i^ny (-1)^{Z.j}
+                    cplx f(0, -1);
+                    for (int y = 0; y < ny; y++) f = f * cplx(0, 1);
+                    return __builtin_parity(unsigned(Z & j)) ? -f : f;
+                };
+                const cplx f0 = factor(0), e0 = op.values[size_t(X * 4)];
+                const double s = e0.re * f0.re + e0.im * f0.im;
+                bool ok = std::fabs(c * c + s * s - 1.0) <= kUnitaryTol;
+                for (int r = 0; r < 4 && ok; r++)
+                    for (int j = 0; j < 4 && ok; j++) {
+                        cplx want(0);
+                        if (r == j) want = cplx(c);
+                        if (r == (j ^ X)) want = factor(j) * cplx(s);
+                        const cplx got = op.values[size_t(r * 4 + j)];
+                        ok = std::fabs(got.re - want.re) <= 1e-15 && std::fabs(got.im - want.im) <= 1e-15;
+                    }
+                if (!ok) continue;
+                std::vector<uint64_t> xs, zs;
+                if (X & 2) xs.push_back(hi);
+                if (X & 1) xs.push_back(lo);
+                if (Z & 2) zs.push_back(hi);
+                if (Z & 1) zs.push_back(lo);
+                rotation(xs, zs, c, s);
+                return;
+            }
+        throw Unsupported{};
+    }
+};
+
+// A subspace of places in echelon form (each vector's top bit in no other).
+struct Span {
+    uint32_t basis[kRotRegBits] = {};
+    int dim = 0;
+    uint32_t reduce(uint32_t v) const {
+        for (int i = 0; i < dim; i++)
+            if (v & (uint32_t(1) << (31 - __builtin_clz(basis[i])))) v ^= basis[i];
+        return v;
+    }
+    bool add(uint32_t v) {
+        v = reduce(v);
+        if (!v || dim == kRotRegBits) return false;
+        const uint32_t top = uint32_t(1) << (31 - __builtin_clz(v));
+        for (int i = 0; i < dim; i++)
+            if (basis[i] & top) basis[i] ^= v;
+        basis[dim++] = v;
+        return true;
+    }
+};
+
+constexpr long double kMaxOwed = 200.0L;  // rotations may leave amplitudes e^200 too large before a table
+constexpr int kWindow = 128;  // items a phase chooses among
+struct Bits {
+    uint64_t w[2] = {0, 0};
+    void set(int i) { w[i >> 6] |= uint64_t(1) << (i & 63); }
+    bool get(int i) const { return (w[i >> 6] >> (i & 63)) & 1; }
+    bool within(const Bits& o) const { return !(w[0] & ~o.w[0]) && !(w[1] & ~o.w[1]); }
+};
+
+uint4 word(uint32_t x, uint32_t y, uint32_t z, uint32_t w) { return make_uint4(x, y, z, w); }
+uint4 word(double a, double b) {
+    uint4 u;
+    double d[2] = {a, b};
+    std::memcpy(&u, d, sizeof u);
+    return u;
+}
+
+class Scheduler {
+  public:
+    Scheduler(std::vector<Item> items, int m, Lowering& lw, RotProgram& out)
+        : items_(std::move(items)), m_(m), lw_(lw), out_(out) {}
+
+    void run() {
+        for (size_t i = 0; i < items_.size(); i++)
+            if (items_[i].rot || items_[i].a != 0.0) active_.push_back(int(i));
+        struct Ph {
+            uint4 head[3];
+            std::vector<uint4> steps, rots;
+        };
+        std::vector<Ph> phases;
+        do {
+            Ph p;
+            one_phase(p.head);
+            pack(p.steps, p.rots);
+            phases.push_back(std::move(p));
+        } while (!active_.empty());
+        size_t step_at = phases.size() * 3, rot_at = step_at;
+        for (const Ph& p : phases) rot_at += p.steps.size();
+        out_.words.clear();
+        for (Ph& p : phases) {
+            p.head[0].x = uint32_t(step_at);
+            p.head[0].y = uint32_t(p.steps.size());
+            p.head[2].y = uint32_t(rot_at);
+            out_.words.insert(out_.words.end(), p.head, p.head + 3);
+            step_at += p.steps.size();
+            rot_at += p.rots.size();
+        }
+        for (const Ph& p : phases) out_.words.insert(out_.words.end(), p.steps.begin(), p.steps.end());
+        for (const Ph& p : phases) out_.words.insert(out_.words.end(), p.rots.begin(), p.rots.end());
+        out_.data = int(out_.words.size());
+        out_.words.insert(out_.words.end(), tables_.begin(), tables_.end());
+        // The kernel fetches a step and a rotation ahead.
+        out_.words.insert(out_.words.end(), 2, make_uint4(0, 0, 0, 0));
+        out_.nphases = int(phases.size());
+    }
+
+  private:
+    std::vector<Item> items_;
+    int m_;
+    Lowering& lw_;
+    RotProgram& out_;
+    std::vector<int> active_;  // items not applied yet, in order
+    double fma_ = 0;
+
+    // One part of a step, in the order the kernel applies a step's parts.
+    struct Part {
+        int place = 0;     // 0-3: rotation on register bit `place`; 4: other rotations; 5: table; 6: slot phases or moduli
+        uint32_t d = 0, kind = 0, signs = 0, mask = 0, data = 0, count = 0;
+        double t = 0.0, u = 0.0;
+    };
+    std::vector<Part> parts_;
+
+    // Consecutive parts share a step as long as their places ascend: a step's
+    // fixed cost (its branches fetch instructions the other warps are not
+    // running) is about that of a rotation.
+    void pack(std::vector<uint4>& steps, std::vector<uint4>& rots) {
+        int last = 99;
+        for (const Part& p : parts_) {
+            if (p.place <= last) steps.push_back(make_uint4(0, 0, 0, 0));
+            last = p.place;
+            uint4& s = steps.back();
+            if (p.place <= 4) {
+                s.x |= p.place < 4 ? (p.kind + 1) << (2 * p.place) : (p.d | p.kind << 4) << 8;
+                rots.push_back(word(p.t, p.u));
+                if (p.kind != kRotPlain) rots.push_back(make_uint4(p.signs, p.mask, 0, 0));
+            } else if (p.place == 5) {
+                s.x |= kRotTable;
+                s.y = p.data;
+            } else {
+                s.x |= p.kind;
+                s.z = p.data;
+                s.w = p.count | p.signs << 16;
+            }
+        }
+        parts_.clear();
+    }
+
+    void one_phase(uint4 head[3]) {
+        const int W = int(std::min<size_t>(active_.size(), size_t(kWindow)));
+        std::vector<const Item*> it(static_cast<size_t>(W));
+        for (int i = 0; i < W; i++) it[size_t(i)] = &items_[size_t(active_[size_t(i)])];
+        std::vector<Bits> pred(static_cast<size_t>(W));
+        for (int j = 0; j < W; j++)
+            for (int i = 0; i < j; i++)
+                if (!commute(*it[size_t(i)], *it[size_t(j)])) pred[size_t(j)].set(i);
+        auto closure = [&](const Span& V, Bits& exec) {
+            int rots = 0;
+            exec = Bits{};
+            for (int i = 0; i < W; i++) {
+                const Item& x = *it[size_t(i)];
+                if (!pred[size_t(i)].within(exec)) continue;
+                if (x.rot) {
+                    if (V.reduce(x.v)) continue;
+                    rots++;
+                }
+                exec.set(i);
+            }
+            return rots;
+        };
+        // Directions one at a time: the one that lets the most rotations in,
+        // among those of the first rotations that only lack their direction.
+        Span V;
+        Bits exec;
+        closure(V, exec);
+        while (V.dim < kRotRegBits) {
+            std::vector<uint32_t> cand;
+            for (int i = 0; i < W && cand.size() < 8; i++) {
+                const Item& x = *it[size_t(i)];
+                if (!x.rot || exec.get(i) || !pred[size_t(i)].within(exec)) continue;
+                const uint32_t v = V.reduce(x.v);
+                if (v && std::find(cand.begin(), cand.end(), v) == cand.end()) cand.push_back(v);
+            }
+            if (cand.empty()) break;
+            int best = -1;
+            Span bestV;
+            Bits bestE;
+            for (uint32_t v : cand) {
+                Span T = V;
+                T.add(v);
+                Bits e;
+                const int r = closure(T, e);
+                if (r > best) {
+                    best = r;
+                    bestV = T;
+                    bestE = e;
+                }
+            }
+            V = bestV;
+            exec = bestE;
+        }
+        for (int b = m_ - 1; b >= 0 && V.dim < kRotRegBits; b--) V.add(1u << b);
+        closure(V, exec);
+        bool last = int(active_.size()) == W;
+        for (int i = 0; i < W && last; i++)
+            if (it[size_t(i)]->rot && !exec.get(i)) last = false;
+
+        // Order: rotations as far as they go, then the phases that hold the
+        // next ones back, and so on.  `flush[f]` comes before the rotations of group f.
+        std::vector<std::vector<int>> groups, flush;
+        Bits done;
+        while (true) {
+            std::vector<int> g;
+            for (int i = 0; i < W; i++)
+                if (it[size_t(i)]->rot && exec.get(i) && !done.get(i) && pred[size_t(i)].within(done)) {
+                    done.set(i);
+                    g.push_back(i);
+                }
+            groups.push_back(g);
+            std::vector<int> need;
+            for (int j = 0; j < W; j++) {
+                if (!it[size_t(j)]->rot || !exec.get(j) || done.get(j)) continue;
+                // Held back by phases only?
+                bool only = true;
+                for (int i = 0; i < j && only; i++)
+                    if (pred[size_t(j)].get(i) && !done.get(i) && it[size_t(i)]->rot) only = false;
+                if (!only) continue;
+                for (int i = 0; i < j; i++)
+                    if (pred[size_t(j)].get(i) && !done.get(i) && std::find(need.begin(), need.end(), i) == need.end())
+                        need.push_back(i);
+            }
+            if (need.empty()) break;
+            std::vector<int> ready;
+            for (int i : need)
+                if (pred[size_t(i)].within(done)) ready.push_back(i);
+            for (int i : ready) done.set(i);
+            flush.push_back(ready);
+        }
+        // V's basis: the directions of the first rotations, whose signs then
+        // follow their own register bit where they commute.
+        uint32_t basis[kRotRegBits];
+        {
+            Span got;
+            auto want = [&](uint32_t v) {
+                const int at = got.dim;
+                if (got.add(v)) basis[at] = v;
+            };
+            for (auto& g : groups)
+                for (int i : g) want(it[size_t(i)]->v);
+            for (int j = 0; j < kRotRegBits; j++) want(V.basis[j]);
+        }
+        // After the last rotation every phase left; also those of a window without rotations.
+        std::vector<int> tail;
+        if (last || groups[0].empty())
+            for (int i = 0; i < W; i++)
+                if (!it[size_t(i)]->rot && !done.get(i) && pred[size_t(i)].within(done)) tail.push_back(i);
+
+        // The slots' places: the complement of V in which the parities of up to
+        // four of those phases vanish (their factors then depend on the
+        // register entry alone).
+        const uint64_t local = (uint64_t(1) << m_) - 1;
+        uint32_t M[kRotRegBits], R[kRotRegBits];  // masks and their parities on V's basis
+        int nm = 0;
+        auto on_V = [&](uint64_t mask) {
+            uint32_t r = 0;
+            for (int j = 0; j < kRotRegBits; j++) r |= uint32_t(parity64(mask & basis[j])) << j;
+            return r;
+        };
+        uint32_t ech[kRotRegBits] = {};
+        auto take = [&](uint64_t mask) {
+            if (nm == kRotRegBits) return;
+            uint32_t r = on_V(mask), red = r;
+            for (int j = 0; j < kRotRegBits; j++)  // ech[j]: a vector whose top bit is j
+                if (ech[kRotRegBits - 1 - j] && ((red >> (kRotRegBits - 1 - j)) & 1)) red ^= ech[kRotRegBits - 1 - j];
+            if (!red) return;
+            ech[31 - __builtin_clz(red)] = red;
+            M[nm] = uint32_t(mask & local);
+            R[nm++] = r;
+        };
+        for (auto& f : flush)
+            for (int i : f)
+                if (!(it[size_t(i)]->mask & ~local)) take(it[size_t(i)]->mask);
+        for (int i : tail)
+            if (!(it[size_t(i)]->mask & ~local)) take(it[size_t(i)]->mask);
+        for (int i = 0; i < W; i++)
+            if (!it[size_t(i)]->rot && pred[size_t(i)].within(done) && !(it[size_t(i)]->mask & ~local))
+                take(it[size_t(i)]->mask);
+        for (int b = 0; b < m_; b++) take(uint64_t(1) << b);
+        // Place p shifted within its coset so that every M vanishes: solve
+        // sum_j x_j R[i]_j = M[i].p for x (R is invertible).
+        uint32_t inv[kRotRegBits] = {};  // bit i of inv[j]: x_j takes M[i].p
+        {
+            uint32_t rows[kRotRegBits], id[kRotRegBits];
+            for (int i = 0; i < kRotRegBits; i++) {
+                rows[i] = R[i];
+                id[i] = 1u << i;
+            }
+            for (int c = 0; c < kRotRegBits; c++) {
+                int p = c;
+                while (p < kRotRegBits && !((rows[p] >> c) & 1)) p++;
+                std::swap(rows[c], rows[p]);
+                std::swap(id[c], id[p]);
+                for (int i = 0; i < kRotRegBits; i++)
+                    if (i != c && ((rows[i] >> c) & 1)) {
+                        rows[i] ^= rows[c];
+                        id[i] ^= id[c];
+                    }
+            }
+            for (int j = 0; j < kRotRegBits; j++) inv[j] = id[j];
+        }
+        auto project = [&](uint32_t p) {
+            uint32_t mp = 0;
+            for (int i = 0; i < kRotRegBits; i++) mp |= uint32_t(__builtin_parity(M[i] & p)) << i;
+            for (int j = 0; j < kRotRegBits; j++)
+                if (__builtin_parity(inv[j] & mp)) p ^= basis[j];
+            return p;
+        };
+        // A basis of that complement; the first three (lanes 0-7 of a 16-byte
+        // shared-memory wavefront) on distinct bank groups where it has such vectors.
+        std::vector<uint32_t> U;
+        {
+            std::vector<uint32_t> red;
+            auto independent = [&](uint32_t p, bool keep) {
+                for (uint32_t r : red)
+                    if (p & (uint32_t(1) << (31 - __builtin_clz(r)))) p ^= r;
+                if (!p) return false;
+                if (keep) {
+                    const uint32_t top = uint32_t(1) << (31 - __builtin_clz(p));
+                    for (uint32_t& r : red)
+                        if (r & top) r ^= p;
+                    red.push_back(p);
+                }
+                return true;
+            };
+            std::vector<uint32_t> unit;
+            for (int b = 0; b < m_; b++) unit.push_back(project(1u << b));
+            std::vector<uint32_t> pool = unit;
+            for (int i = 0; i < m_; i++)
+                for (int j = 0; j < i; j++) pool.push_back(unit[size_t(i)] ^ unit[size_t(j)]);
+            uint32_t banks[3] = {}, nb = 0;
+            for (uint32_t p : pool) {
+                if (nb == 3 || int(U.size()) == m_ - kRotRegBits) break;
+                uint32_t l = rot_swizzle(p) & 7u;
+                for (uint32_t i = 0; i < nb; i++)
+                    if (l & (1u << (31 - __builtin_clz(banks[i])))) l ^= banks[i];
+                if (!p || !l || !independent(p, true)) continue;
+                const uint32_t top = 1u << (31 - __builtin_clz(l));
+                for (uint32_t i = 0; i < nb; i++)
+                    if (banks[i] & top) banks[i] ^= l;
+                banks[nb++] = l;
+                U.push_back(p);
+            }
+            for (uint32_t p : unit)
+                if (int(U.size()) < m_ - kRotRegBits && p && independent(p, true)) U.push_back(p);
+        }
+        auto slots = [&](uint64_t mask) {  // kernel parity mask
+            uint32_t s = 0;
+            for (size_t i = 0; i < U.size(); i++) s |= uint32_t(parity64(mask & U[i])) << i;
+            return s | uint32_t(mask >> m_) << kRotSlotBits;
+        };
+        auto signs = [&](uint32_t r) {
+            uint32_t s = 0;
+            for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) s |= uint32_t(__builtin_parity(r & v)) << v;
+            return s;
+        };
+        auto direction = [&](uint32_t v) {  // v on the basis
+            uint32_t d = 0, best = 0;
+            for (d = 1; d < uint32_t(kRotEntries); d++) {
+                uint32_t x = 0;
+                for (int j = 0; j < kRotRegBits; j++)
+                    if ((d >> j) & 1) x ^= basis[j];
+                if (x == v) best = d;
+            }
+            return best;
+        };
+
+        // Emission.  pend[j]: logarithm of the factor still owed by the entries
+        // with register bit j clear (the others owe its negative).
+        long double pend[kRotRegBits] = {};
+        auto emit_table = [&](const long double A[kRotEntries], long double B[kRotEntries], double G) {
+            Part part;
+            part.place = 5;
+            part.data = uint32_t(tables_.size());
+            parts_.push_back(part);
+            for (int v = 0; v < kRotEntries; v++) {
+                B[v] += uniform_;
+                for (int j = 0; j < kRotRegBits; j++) B[v] += (v >> j) & 1 ? -pend[j] : pend[j];
+                const double a = double(A[v] + G), S = std::exp(double(B[v]));
+                tables_.push_back(word(S * std::cos(a), S * std::sin(a)));
+            }
+            for (long double& p : pend) p = 0.0;
+            uniform_ = 0.0;
+            out_.tables++;
+            fma_ += 6.0;
+        };
+        // Rotations of a group in an order that fills steps: places ascending,
+        // earlier ones that do not commute first.
+        for (auto& g : groups) {
+            std::vector<int> left = g, order;
+            int at = -1;
+            while (!left.empty()) {
+                size_t pick = left.size();
+                int place = 99;
+                for (size_t i = 0; i < left.size(); i++) {
+                    bool free = true;
+                    for (size_t j = 0; j < i && free; j++) free = !pred[size_t(left[i])].get(left[j]);
+                    if (!free) continue;
+                    const uint32_t d = direction(it[size_t(left[i])]->v);
+                    const int p = (d & (d - 1)) == 0 && !it[size_t(left[i])]->imag ? __builtin_ctz(d) : 4;
+                    if (p > at && p < place) {
+                        place = p;
+                        pick = i;
+                    }
+                }
+                if (pick == left.size()) {
+                    at = -1;
+                    continue;
+                }
+                at = place;
+                order.push_back(left[pick]);
+                left.erase(left.begin() + long(pick));
+            }
+            g = order;
+        }
+        auto emit_flush = [&](std::vector<int> f, bool final) {
+            // Phases that need no slot parity come along for nothing.
+            bool free_table = final;
+            for (int i : f) free_table = free_table || slots(it[size_t(i)]->mask) == 0;
+            if (free_table)
+                for (int i = 0; i < W; i++)
+                    if (!it[size_t(i)]->rot && !done.get(i) && pred[size_t(i)].within(applied_) &&
+                        slots(it[size_t(i)]->mask) == 0 && std::find(f.begin(), f.end(), i) == f.end()) {
+                        f.push_back(i);
+                        done.set(i);
+                    }
+            std::vector<std::pair<uint32_t, std::vector<int>>> by;  // register parity -> phases
+            long double A[kRotEntries] = {}, B[kRotEntries] = {};
+            bool table = false;
+            for (int i : f) {
+                const Item& x = *it[size_t(i)];
+                if (applied_.get(i)) continue;
+                applied_.set(i);
+                const uint32_t r = on_V(x.mask);
+                if (slots(x.mask) == 0) {
+                    table = true;
+                    for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) {
+                        const bool neg = __builtin_parity(r & v);
+                        A[v] += neg ? -x.a : x.a;
+                        B[v] += neg ? -x.b : x.b;
+                    }
+                    continue;
+                }
+                auto b = std::find_if(by.begin(), by.end(), [&](auto& e) { return e.first == r; });
+                if (b == by.end()) {
+                    by.push_back({r, {}});
+                    b = by.end() - 1;
+                }
+                b->second.push_back(i);
+            }
+            double G = 0.0;
+            if (final) {
+                G = double(std::remainder(lw_.global, 2 * kPiL));
+                table = table || G != 0.0;
+                for (long double p : pend) table = table || p != 0.0;
+                table = table || uniform_ != 0.0;
+            }
+            if (table) emit_table(A, B, G);
+            for (auto& b : by) {
+                const std::vector<int>& terms = b.second;
+                auto part_of = [&](uint32_t kind, const std::vector<int>& t) {
+                    Part part;
+                    part.place = 6;
+                    part.kind = kind;
+                    part.signs = signs(b.first);
+                    part.data = uint32_t(tables_.size());
+                    part.count = uint32_t(t.size());
+                    parts_.push_back(part);
+                    for (size_t i = 0; i < t.size(); i += 4) {
+                        uint32_t m4[4] = {};
+                        for (size_t j = i; j < std::min(t.size(), i + 4); j++) m4[j - i] = slots(it[size_t(t[j])]->mask);
+                        tables_.push_back(word(m4[0], m4[1], m4[2], m4[3]));
+                    }
+                };
+                std::vector<int> angles, moduli;
+                for (int i : terms) {
+                    if (it[size_t(i)]->a != 0.0) angles.push_back(i);
+                    if (it[size_t(i)]->b != 0.0) moduli.push_back(i);
+                }
+                if (!angles.empty()) {
+                    part_of(kRotSlots, angles);
+                    for (int i : angles) tables_.push_back(word(std::cos(it[size_t(i)]->a), std::sin(it[size_t(i)]->a)));
+                    out_.slot_phases++;
+                    fma_ += 6.0 + 6.0 * double(angles.size()) / kRotEntries;
+                }
+                if (!moduli.empty()) {
+                    part_of(kRotSlotModuli, moduli);
+                    for (int i : moduli) {
+                        const long double x = it[size_t(i)]->b;
+                        tables_.push_back(word(double(std::exp(x)), double(std::exp(-x))));
+                    }
+                    out_.slot_phases++;
+                    fma_ += 2.0 + 2.0 * double(moduli.size()) / kRotEntries;
+                }
+            }
+        };
+        // The coordinate functional of register bit j: a mask that vanishes on the slots.
+        auto functional = [&](int j) {
+            uint64_t f = 0;
+            for (int i = 0; i < kRotRegBits; i++)
+                if ((inv[j] >> i) & 1) f ^= M[i];
+            return f;
+        };
+        applied_ = Bits{};
+        // The next table after each group (groups.size(): none in this phase).
+        std::vector<size_t> table_at(groups.size() + 1, groups.size());
+        for (size_t g = groups.size(); g-- > 0;) {
+            bool table = g + 1 == groups.size() && last;
+            if (g < flush.size())
+                for (int i : flush[g]) table = table || slots(it[size_t(i)]->mask) == 0;
+            table_at[g] = table ? g : table_at[g + 1];
+        }
+        for (size_t g = 0; g < groups.size(); g++) {
+            for (size_t gi = 0; gi < groups[g].size(); gi++) {
+                const int i = groups[g][gi];
+                const Item& x = *it[size_t(i)];
+                const uint32_t d = direction(x.v), r = on_V(x.mask);
+                const int low = __builtin_ctz(d);
+                // In place where a table comes before the next rotation that mixes
+                // this register bit, or where the factors owed can join a phase
+                // that waits with the same mask.
+                bool in_place = table_at[g] < groups.size();
+                for (size_t h = g; h < groups.size() && h <= table_at[g] && in_place; h++)
+                    for (size_t hi = h == g ? gi + 1 : 0; hi < groups[h].size() && in_place; hi++)
+                        in_place = !((direction(it[size_t(groups[h][hi])]->v) >> low) & 1);
+                if (!in_place && table_at[g] == groups.size()) {
+                    const uint64_t f = functional(low);
+                    for (int j = 0; j < W && !in_place; j++)
+                        in_place = !it[size_t(j)]->rot && !done.get(j) && it[size_t(j)]->mask == f &&
+                                   pred[size_t(j)].within(done);
+                    for (size_t h = g; h < groups.size() && in_place; h++)
+                        for (size_t hi = h == g ? gi + 1 : 0; hi < groups[h].size() && in_place; hi++)
+                            in_place = !((direction(it[size_t(groups[h][hi])]->v) >> low) & 1);
+                }
+                const long double lost = 0.5L * std::log1p((long double)(x.t) * x.t);
+                Part part;
+                part.place = (d & (d - 1)) == 0 && !x.imag ? low : 4;
+                part.d = d;
+                part.kind = x.imag ? kRotImag : !in_place ? kRotKept
+                            : part.place < 4 && r == (1u << low) && slots(x.mask) == 0 ? kRotPlain : kRotSigned;
+                part.signs = signs(r);
+                part.mask = slots(x.mask);
+                part.t = x.t;
+                part.u = x.t / (1.0 + x.t * x.t);
+                if (part.kind == kRotKept) {
+                    part.u = 1.0 + x.t * x.t;
+                    uniform_ -= lost;
+                } else {
+                    for (int j = 0; j < kRotRegBits; j++)
+                        if (((d >> j) & 1) && pend[j] != 0.0) {
+                            long double A[kRotEntries] = {}, B[kRotEntries] = {};
+                            emit_table(A, B, 0.0);
+                            break;
+                        }
+                    pend[low] -= lost;
+                }
+                parts_.push_back(part);
+                applied_.set(i);
+                out_.rotations++;
+                fma_ += 4.0;
+            }
+            if (g < flush.size()) emit_flush(flush[g], false);
+        }
+        if (last || !tail.empty()) emit_flush(tail, last);
+        if (!last && uniform_ < -kMaxOwed) {  // a circuit without phases: keep the amplitudes in range
+            long double A[kRotEntries] = {}, B[kRotEntries] = {};
+            emit_table(A, B, 0.0);
+        }
+        // Factors still owed become phases of the register bits' parities (the
+        // coordinate functionals), for later phases of the pass.
+        std::vector<Item> owed;
+        for (int j = 0; j < kRotRegBits; j++) {
+            if (pend[j] == 0.0) continue;
+            Item f;
+            f.mask = functional(j);
+            f.b = pend[j];
+            owed.push_back(f);
+        }
+        head[0] = word(0, 0, rot_swizzle(basis[0]) | rot_swizzle(basis[1]) << 16,
+                       rot_swizzle(basis[2]) | rot_swizzle(basis[3]) << 16);
+        uint32_t b[12] = {};
+        for (size_t i = 0; i < U.size(); i++) b[i] = rot_swizzle(U[i]);
+        head[1] = word(b[0] | b[1] << 16, b[2] | b[3] << 16, b[4] | b[5] << 16, b[6] | b[7] << 16);
+        head[2] = word(b[8], 0, 0, 0);
+        std::vector<int> left;
+        for (const Item& f : owed) {
+            // Joined with a phase of the same mask that is ready, else first in line.
+            bool joined = false;
+            for (int i = 0; i < W && !joined; i++) {
+                Item& x = items_[size_t(active_[size_t(i)])];
+                if (x.rot || applied_.get(i) || x.mask != f.mask || !pred[size_t(i)].within(applied_)) continue;
+                x.b += f.b;
+                joined = true;
+            }
+            if (joined) continue;
+            left.push_back(int(items_.size()));
+            items_.push_back(f);
+        }
+        for (int i = 0; i < int(active_.size()); i++)
+            if (i >= W || !applied_.get(i)) left.push_back(active_[size_t(i)]);
+        active_ = std::move(left);
+        out_.flops_per_amp = fma_;
+    }
+
+    Bits applied_;
+    long double uniform_ = 0.0;  // logarithm of a factor all amplitudes are owed
+    std::vector<uint4> tables_;  // data of the tables and slot phases
+};
+
+}  // namespace
+
+bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<int>& tile_qubits, int n,
+                         RotProgram& out) {
+    const int m = int(tile_qubits.size());
+    if (m < kRotMinTile || m > kRotMaxTile || n - m > kRotMaxOuter) return false;
+    Lowering lw(tile_qubits, n);
+    try {
+        for (const Operation& op : ops) lw.add(op);
+    } catch (const Unsupported&) {
+        return false;
+    }
+    out = RotProgram{};
+    out.m = m;
+    Scheduler s(lw.items, m, lw, out);
+    s.run();
+    // Place of tile index e: sum over q of (e_q ^ const_q ^ outer part) v_q.
+    uint32_t c = 0;
+    for (int q = 0; q < m; q++) {
+        const size_t g = size_t(tile_qubits[size_t(q)]);
+        const uint32_t v = lw.dirs()[g];
+        out.out_dir[q] = uint16_t(rot_swizzle(v));
+        if (lw.consts()[g]) c ^= v;
+        for (int j = 0; j < n - m; j++)
+            if ((lw.masks()[g] >> (m + j)) & 1) out.out_outer[j] = uint16_t(out.out_outer[j] ^ rot_swizzle(v));
+        if (parity64(lw.sign & v)) out.sign_local |= 1u << q;
+    }
+    out.out_const = uint16_t(rot_swizzle(c));
+    // sign . p over p(e): on e through sign.v_q, on the tile index through its
+    // own bits and through the places' outer part.
+    out.sign_const = parity64(lw.sign & c);
+    for (int j = 0; j < n - m; j++) {
+        int bit = int((lw.sign >> (m + j)) & 1);
+        for (int q = 0; q < m; q++) {
+            const size_t g = size_t(tile_qubits[size_t(q)]);
+            if ((lw.masks()[g] >> (m + j)) & 1) bit ^= parity64(lw.sign & lw.dirs()[g]);
+        }
+        if (bit) out.sign_outer |= 1u << j;
+    }
+    return true;
+}
+
+}  // namespace dq

@@ -142,6 +142,9 @@ ExecConfig exec_config(const Options& o, uint64_t n, bool force_per_gate, const 
     // complex64 runs its tile passes as fused 5-qubit tensor-core blocks unless a
     // CUDA-core tile shape or a narrower fusion width is asked for.
     c.fused = c.c64 && c.tiled && (o.fusion_width == 5 || (o.fusion_width == 0 && o.tile_qubits == 0));
+    // The default complex128 passes are Pauli rotations; an explicit fusion
+    // width asks for fused matrices of that width.
+    c.rotations = !c.c64 && o.fusion_width == 0;
     c.n = int(n);
     return c;
 }
@@ -321,8 +324,8 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
                     }
                 } ev_guard{ev};
                 cuda_check(cudaEventRecord(ev[0], s), "cudaEventRecord");
-                // |0...0>: written here, or built by a first fused pass in its tiles.
-                const bool built = ex->starts_with_fused_pass();
+                // |0...0>: written here, or built by the first pass in its tiles.
+                const bool built = ex->builds_basis();
                 if (!built) k::init_basis(b);
                 ex->run(b, nullptr, nullptr, /*normalize=*/false, /*from_basis=*/built);  // the sampler divides by the total
                 cuda_check(cudaEventRecord(ev[1], s), "cudaEventRecord");
@@ -430,10 +433,10 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
     if (cache_prefix) {
         prefix.allocate(int(n), 1, ncb, c64);
         k::Batch pb = prefix.view(s, 1);
-        k::init_basis(pb);
         reset_bookkeeping(prefix, 1, {seed}, s);
         Executor pre(ops, 0, prefix_end, exec_config(opt_, n));
-        pre.run(pb, nullptr);
+        if (!pre.builds_basis()) k::init_basis(pb);
+        pre.run(pb, nullptr, nullptr, true, pre.builds_basis());
     }
     StateBatch st;
     st.allocate(int(n), workers, ncb, c64);
@@ -494,12 +497,12 @@ std::unique_ptr<Result> Simulator::simulate(const char* json, size_t len) {
     res->n = n;
     res->state.allocate(int(n), 1, ncb, opt_.precision == Precision::C64);
     k::Batch b = res->state.view(s, 1);
-    k::init_basis(b);
     reset_bookkeeping(res->state, 1, {seed}, s);
     // Profiling times each reference operation, so it runs the per-gate form.
     Executor ex(plan, 0, plan.size(), exec_config(opt_, n, opt_.profile));
     ProfileAcc acc;
-    ex.run(b, opt_.profile ? &acc : nullptr);
+    if (!ex.builds_basis()) k::init_basis(b);
+    ex.run(b, opt_.profile ? &acc : nullptr, nullptr, true, ex.builds_basis());
     check_err_flag(res->state, s);
     std::vector<uint64_t> hbits(res->state.cwords);
     cuda_check(cudaMemcpyAsync(hbits.data(), res->state.cbits.p, hbits.size() * 8, cudaMemcpyDeviceToHost, s),

@@ -16,6 +16,7 @@ this engine; their names exist and raise ``NotImplementedError``.
 from __future__ import annotations
 
 import ctypes
+import json
 import os
 from pathlib import Path
 
@@ -930,6 +931,18 @@ def tile_plan_dump(circuit_json, tile_qubits=12, fusion_width=2):
         return _json.loads(out.value.decode("utf-8"))
     finally:
         _string_free(ctypes.cast(out, ctypes.c_void_p))
+
+
+_rotation_plan_dump = _sig("dq_rotation_plan_dump", [ctypes.c_char_p, ctypes.c_size_t, ctypes.c_int,
+                                                     ctypes.POINTER(ctypes.c_char_p)])
+
+
+def rotation_plan_dump(circuit_json, tile_qubits=12):
+    """Host-only: the complex128 rotation passes of a unitary circuit (for tests and inspection)."""
+    text = circuit_json.encode("utf-8") if isinstance(circuit_json, str) else circuit_json
+    out = ctypes.c_char_p()
+    _check(_rotation_plan_dump(text, len(text), int(tile_qubits), ctypes.byref(out)))
+    return json.loads(_take_text(out))
 
 
 _fused_plan_dump = _sig("dq_fused_plan_dump", [ctypes.c_char_p, ctypes.c_size_t, ctypes.POINTER(ctypes.c_char_p)])
