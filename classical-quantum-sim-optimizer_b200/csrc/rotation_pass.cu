@@ -331,15 +331,28 @@ __global__ void __launch_bounds__(kRotThreads, 1)
     rotation_body(s, n, p, pack, total_tiles, basis, DevWords{w, w + p.data});
 }
 
+// CTAs of the kernel that are resident at once on the current device, asked of
+// the runtime when the shape differs from this thread's last launch.
 template <typename Kernel>
-unsigned rotation_grid(Kernel kernel, int threads, size_t smem, uint64_t ctas) {
+uint64_t resident_ctas(Kernel kernel, int threads, size_t smem) {
+    struct Shape {
+        const void* kernel = nullptr;
+        int dev = -1, threads = 0;
+        size_t smem = 0;
+        uint64_t ctas = 0;
+    };
+    static thread_local Shape last;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const void* id = reinterpret_cast<const void*>(kernel);
+    if (last.kernel == id && last.dev == dev && last.threads == threads && last.smem >= smem) return last.ctas;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, int(cudaSharedmemCarveoutMaxShared));
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
+    int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-    return unsigned(std::min<uint64_t>(ctas, uint64_t(std::max(sms, 1)) * uint64_t(std::max(per_sm, 1))));
+    last = {id, dev, threads, smem, uint64_t(std::max(sms, 1)) * uint64_t(std::max(per_sm, 1))};
+    return last.ctas;
 }
 
 }  // namespace
@@ -384,11 +397,13 @@ void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const Ro
     if (as_argument) {
         static thread_local RotWords args;
         std::memcpy(args.w, r.words.data(), r.words.size() * sizeof(uint4));
-        k_rotations_arg<<<rotation_grid(k_rotations_arg, threads, smem, ctas), unsigned(threads), smem, b.stream>>>(
+        k_rotations_arg<<<unsigned(std::min(ctas, resident_ctas(k_rotations_arg, threads, smem))), unsigned(threads), smem,
+                          b.stream>>>(
             static_cast<double2*>(b.amps), b.n, pack, total, basis ? 1 : 0, p, args);
     } else {
         if (!words_dev) fail(kValueError, "rotation pass without its device words");
-        k_rotations_dev<<<rotation_grid(k_rotations_dev, threads, smem, ctas), unsigned(threads), smem, b.stream>>>(
+        k_rotations_dev<<<unsigned(std::min(ctas, resident_ctas(k_rotations_dev, threads, smem))), unsigned(threads), smem,
+                          b.stream>>>(
             static_cast<double2*>(b.amps), b.n, pack, total, basis ? 1 : 0, p, words_dev);
     }
     const cudaError_t e = cudaGetLastError();

@@ -11,7 +11,9 @@ namespace dq {
 namespace {
 
 constexpr long double kPiL = 3.14159265358979323846264338327950288L;
-constexpr double kPi = double(kPiL);
+// Angles and moduli are kept with 64-bit mantissas: what the gates' entries say
+// is then lost only where a factor is rounded for the kernel.
+using ld = long double;
 constexpr double kUnitaryTol = 1e-12;
 constexpr double kAngleTol = 2.3e-16;  // a quarter turn to the rounding of its angle
 constexpr int kMaxDiagQubits = 6;
@@ -24,14 +26,15 @@ struct Item {
     uint32_t v = 0;      // rotation: direction (tile-local place bits)
     uint64_t mask = 0;   // parity mask over place bits (tile-local below m, tile index above)
     double t = 0.0;      // rotation: signed tangent
-    double a = 0.0;      // phase: angle
-    long double b = 0.0; // phase: logarithm of its modulus (factors e^(+-(b + ia)))
+    ld a = 0.0;          // phase: angle
+    ld b = 0.0;          // phase: logarithm of its modulus (factors e^(+-(b + ia)))
 };
 
 struct Unsupported {};
 
 double norm2(cplx z) { return z.re * z.re + z.im * z.im; }
-double arg(cplx z) { return std::atan2(z.im, z.re); }
+ld arg(cplx z) { return std::atan2(ld(z.im), ld(z.re)); }
+ld modulus(cplx z) { return std::sqrt(ld(z.re) * z.re + ld(z.im) * z.im); }
 
 bool commute(const Item& x, const Item& y) {
     if (!x.rot && !y.rot) return true;
@@ -73,7 +76,8 @@ class Lowering {
 
     std::vector<Item> items;
     // Sums hundreds of angles: a 64-bit mantissa keeps its rounding below the amplitudes'.
-    long double global = 0.0;  // phase of the whole state
+    ld global = 0.0;           // phase of the whole state
+    ld norm = 0.0;             // logarithm of a modulus of the whole state
     uint64_t sign = 0;         // Z^sign still to be applied
 
     const std::vector<uint64_t>& masks() const { return mask_; }
@@ -88,17 +92,17 @@ class Lowering {
     std::vector<size_t> open_;  // phases that every later rotation commutes with
 
     // exp(i a Z^mask (-1)^cons)
-    void phase(uint64_t mask, int cons, double a) {
+    void phase(uint64_t mask, int cons, ld a) {
         if (cons) a = -a;
         if (mask == 0) {
             global += a;
             return;
         }
-        const double r = std::nearbyint(a / kPi);
-        a = double((long double)(a) - (long double)(r) * kPiL);
-        if (std::fmod(std::fabs(r), 2.0) == 1.0) global += kPiL;
+        const ld r = std::nearbyint(a / kPiL);
+        a -= r * kPiL;
+        if (std::fmod(std::fabs(r), 2.0L) == 1.0L) global += kPiL;
         if (a == 0.0) return;
-        if (std::fabs(std::fabs(a) - kPi / 2) <= kAngleTol) {  // +-i Z^mask
+        if (std::fabs(std::fabs(a) - kPiL / 2) <= kAngleTol) {  // +-i Z^mask
             global += a > 0 ? kPiL / 2 : -kPiL / 2;
             sign ^= mask;
             return;
@@ -117,7 +121,7 @@ class Lowering {
 
     // exp(-i theta/2 P) with (c, s) = (cos, sin)(theta/2), P the product over the
     // qubits of X (bit of xs), Z (of zs) or Y (both).
-    void rotation(const std::vector<uint64_t>& xs, const std::vector<uint64_t>& zs, double c, double s) {
+    void rotation(const std::vector<uint64_t>& xs, const std::vector<uint64_t>& zs, ld c, ld s) {
         uint32_t v = 0;
         uint64_t mask = 0;
         int cons = 0, ny = 0;
@@ -142,7 +146,7 @@ class Lowering {
         if (std::fabs(s) > c) {
             // c - i s P = (-i P) (s + i c P): rotate by the complement, then apply P
             // (the phases and rotations before see the place, so P comes last).
-            double c2 = s, s2 = -c;
+            ld c2 = s, s2 = -c;
             if (c2 < 0) {
                 global += kPiL;
                 c2 = -c2;
@@ -157,13 +161,14 @@ class Lowering {
         emit(v, mask, imag, c, s);
     }
 
-    void emit(uint32_t v, uint64_t mask, bool imag, double c, double s) {
+    void emit(uint32_t v, uint64_t mask, bool imag, ld c, ld s) {
         Item it;
         it.rot = true;
         it.imag = imag;
         it.v = v;
         it.mask = mask;
-        it.t = s / c;
+        it.t = double(s / c);
+        norm += 0.5L * std::log(c * c + s * s);  // the entries' own rounding
         if (parity64(sign & v)) it.t = -it.t;
         open_.erase(std::remove_if(open_.begin(), open_.end(),
                                    [&](size_t i) { return parity64(items[i].mask & v) != 0; }),
@@ -172,14 +177,14 @@ class Lowering {
     }
 
     // Phases phi[j] by the qubits' values (qubits[0] the MSB of j).
-    void phases(const std::vector<uint64_t>& qubits, std::vector<double> phi) {
+    void phases(const std::vector<uint64_t>& qubits, std::vector<ld> phi) {
         const size_t k = qubits.size();
         if (k > size_t(kMaxDiagQubits)) throw Unsupported{};
         const size_t D = size_t(1) << k;
         for (size_t h = 1; h < D; h <<= 1)
             for (size_t i = 0; i < D; i++)
                 if (!(i & h)) {
-                    const double x = phi[i], y = phi[i | h];
+                    const ld x = phi[i], y = phi[i | h];
                     phi[i] = x + y;
                     phi[i | h] = x - y;
                 }
@@ -191,8 +196,9 @@ class Lowering {
                     mask ^= mask_[size_t(qubits[b])];
                     cons ^= cons_[size_t(qubits[b])];
                 }
-            const double a = phi[S] / double(D);
-            if (a != 0.0) phase(mask, cons, a);
+            // (phases that cancel leave the rounding of their sum)
+            const ld a = phi[S] / ld(D);
+            if (std::fabs(a) > 1e-18L) phase(mask, cons, a);
         }
     }
 
@@ -210,15 +216,15 @@ class Lowering {
         size_t j;
         pattern(controls, q, j);
         q.push_back(target);
-        std::vector<double> phi(size_t(1) << q.size(), 0.0);
-        phi[(j << 1) | 1] = kPi;
+        std::vector<ld> phi(size_t(1) << q.size(), 0.0);
+        phi[(j << 1) | 1] = kPiL;
         phases(q, phi);
     }
 
     void one(uint64_t target, const Mat2& u, const std::vector<Control>& controls) {
         // u = e^{i alpha} RZ(beta) RY(theta) RZ(gamma)
-        const double c = std::sqrt(norm2(u[0][0])), s = std::sqrt(norm2(u[1][0]));
-        const double dev[] = {std::fabs(c * c + s * s - 1.0), std::fabs(norm2(u[0][1]) + norm2(u[1][1]) - 1.0),
+        const ld c = modulus(u[0][0]), s = modulus(u[1][0]);
+        const double dev[] = {std::fabs(double(c * c + s * s - 1.0L)), std::fabs(norm2(u[0][1]) + norm2(u[1][1]) - 1.0),
                               std::fabs(u[0][0].re * u[0][1].re + u[0][0].im * u[0][1].im + u[1][0].re * u[1][1].re +
                                         u[1][0].im * u[1][1].im),
                               std::fabs(u[0][0].re * u[0][1].im - u[0][0].im * u[0][1].re + u[1][0].re * u[1][1].im -
@@ -227,28 +233,28 @@ class Lowering {
             if (!(d <= kUnitaryTol)) throw Unsupported{};
         // Arguments of u00, u10 and u11; the fourth entry's follows from
         // unitarity, so the smaller pair gives one argument only.
-        double A, B, D;
+        ld A, B, D;
         if (c >= s) {
             A = arg(u[0][0]);
             D = arg(u[1][1]);
             B = s > 0 ? arg(u[1][0]) : A;
         } else {
             B = arg(u[1][0]);
-            const double C = arg(-u[0][1]);
+            const ld C = arg(-u[0][1]);
             A = c > 0 ? arg(u[0][0]) : B;
             D = B + C - A;
         }
-        double beta = B - A, gamma = D - B, alpha = A + (beta + gamma) / 2;
+        const ld beta = B - A, gamma = D - B, alpha = A + (beta + gamma) / 2;
         if (controls.empty()) {
             global += alpha;
             // RZ(-+pi/2) RY(theta) RZ(+-pi/2) = RX(+-theta)
-            const double turns = std::nearbyint((beta + gamma) / (2 * kPi));
-            const double quarter = std::fabs(std::remainder(beta, 2 * kPi));
-            if (s > 0 && std::fabs(beta + gamma - turns * 2 * kPi) <= 4 * kAngleTol &&
-                std::fabs(quarter - kPi / 2) <= 4 * kAngleTol) {
+            const ld turns = std::nearbyint((beta + gamma) / (2 * kPiL));
+            const ld quarter = std::fabs(std::remainder(beta, 2 * kPiL));
+            if (s > 0 && std::fabs(beta + gamma - turns * 2 * kPiL) <= kAngleTol &&
+                std::fabs(quarter - kPiL / 2) <= kAngleTol) {
                 // RZ(gamma) = RZ(-beta) (-1)^turns; beta = +-pi/2 up to whole turns, which cancel in the pair.
-                if (std::fmod(std::fabs(turns), 2.0) == 1.0) global += kPiL;
-                rotation({target}, {}, c, std::remainder(beta, 2 * kPi) < 0 ? s : -s);
+                if (std::fmod(std::fabs(turns), 2.0L) == 1.0L) global += kPiL;
+                rotation({target}, {}, c, std::remainder(beta, 2 * kPiL) < 0 ? s : -s);
                 return;
             }
             phase(mask_[size_t(target)], cons_[size_t(target)], -gamma / 2);
@@ -262,20 +268,20 @@ class Lowering {
         const size_t nc = q.size();
         std::vector<uint64_t> qt = q;
         qt.push_back(target);
-        auto crz = [&](double angle) {
-            std::vector<double> phi(size_t(2) << nc, 0.0);
+        auto crz = [&](ld angle) {
+            std::vector<ld> phi(size_t(2) << nc, 0.0);
             phi[j << 1] = -angle / 2;
             phi[(j << 1) | 1] = angle / 2;
             phases(qt, phi);
         };
-        const double half = std::atan2(s, c) / 2;  // theta / 4
+        const ld half = std::atan2(s, c) / 2;  // theta / 4
         crz(gamma);
         controlled_z(controls, target);
         rotation({target}, {target}, std::cos(half), -std::sin(half));
         controlled_z(controls, target);
         rotation({target}, {target}, std::cos(half), std::sin(half));
         crz(beta);
-        std::vector<double> phi(size_t(1) << nc, 0.0);
+        std::vector<ld> phi(size_t(1) << nc, 0.0);
         phi[j] = alpha;
         phases(q, phi);
     }
@@ -294,9 +300,9 @@ class Lowering {
         } else if (controls.size() == 1) {
             cx(controls[0].qubit, controls[0].value, target);
         } else {
-            const double r = std::sqrt(0.5);
+            const ld r = std::sqrt(0.5L);
             auto h = [&] {  // H = RY(pi/2) Z
-                phase(mask_[size_t(target)], cons_[size_t(target)], -kPi / 2);  // -i Z
+                phase(mask_[size_t(target)], cons_[size_t(target)], -kPiL / 2);  // -i Z
                 global += kPiL / 2;
                 rotation({target}, {target}, r, r);
             };
@@ -322,7 +328,7 @@ class Lowering {
     }
 
     void diagonal(const Operation& op) {
-        std::vector<double> phi;
+        std::vector<ld> phi;
         for (cplx d : op.values) {
             if (!(std::fabs(norm2(d) - 1.0) <= kUnitaryTol)) throw Unsupported{};
             phi.push_back(arg(d));
@@ -395,7 +401,7 @@ struct Span {
     }
 };
 
-constexpr long double kMaxOwed = 200.0L;  // rotations may leave amplitudes e^200 too large before a table
+constexpr ld kMaxOwed = 200.0L;  // rotations may leave amplitudes e^200 too large before a table
 constexpr int kWindow = 128;  // items a phase chooses among
 struct Bits {
     uint64_t w[2] = {0, 0};
@@ -410,6 +416,29 @@ uint4 word(double a, double b) {
     double d[2] = {a, b};
     std::memcpy(&u, d, sizeof u);
     return u;
+}
+
+// S e^{ia} as doubles.  Entries recur (a CZ's are e^{+-i pi/4}), so the rounding
+// of their modulus would add up: of the nearest pairs the one closest in modulus.
+// `off` gains the logarithm of the modulus, and the angle, by which it misses.
+uint4 factor_word(ld S, ld a, ld off[2]) {
+    const ld re = S * std::cos(a), im = S * std::sin(a);
+    const double x = double(re), y = double(im);
+    double best[2] = {x, y};
+    ld miss = std::fabs(ld(x) * x + ld(y) * y - S * S);
+    const double tries[4][2] = {{std::nextafter(x, 4.0 * x), y}, {std::nextafter(x, 0.0), y},
+                                {x, std::nextafter(y, 4.0 * y)}, {x, std::nextafter(y, 0.0)}};
+    for (const auto& t : tries) {
+        const ld m = std::fabs(ld(t[0]) * t[0] + ld(t[1]) * t[1] - S * S);
+        if (m < miss) {
+            miss = m;
+            best[0] = t[0];
+            best[1] = t[1];
+        }
+    }
+    off[0] += ((best[0] - re) * re + (best[1] - im) * im) / (S * S);
+    off[1] += ((best[1] - im) * re - (best[0] - re) * im) / (S * S);
+    return word(best[0], best[1]);
 }
 
 class Scheduler {
@@ -597,7 +626,7 @@ class Scheduler {
         }
         // After the last rotation every phase left; also those of a window without rotations.
         std::vector<int> tail;
-        if (last || groups[0].empty())
+        if (last || std::all_of(groups.begin(), groups.end(), [](const std::vector<int>& g) { return g.empty(); }))
             for (int i = 0; i < W; i++)
                 if (!it[size_t(i)]->rot && !done.get(i) && pred[size_t(i)].within(done)) tail.push_back(i);
 
@@ -722,20 +751,22 @@ class Scheduler {
 
         // Emission.  pend[j]: logarithm of the factor still owed by the entries
         // with register bit j clear (the others owe its negative).
-        long double pend[kRotRegBits] = {};
-        auto emit_table = [&](const long double A[kRotEntries], long double B[kRotEntries], double G) {
+        ld pend[kRotRegBits] = {};
+        auto emit_table = [&](const ld A[kRotEntries], ld B[kRotEntries], ld G) {
             Part part;
             part.place = 5;
             part.data = uint32_t(tables_.size());
             parts_.push_back(part);
+            ld off[2] = {};
             for (int v = 0; v < kRotEntries; v++) {
                 B[v] += uniform_;
                 for (int j = 0; j < kRotRegBits; j++) B[v] += (v >> j) & 1 ? -pend[j] : pend[j];
-                const double a = double(A[v] + G), S = std::exp(double(B[v]));
-                tables_.push_back(word(S * std::cos(a), S * std::sin(a)));
+                tables_.push_back(factor_word(std::exp(B[v]), std::remainder(A[v] + G, 2 * kPiL), off));
             }
-            for (long double& p : pend) p = 0.0;
-            uniform_ = 0.0;
+            for (ld& p : pend) p = 0.0;
+            // What the table misses on average is owed to the next ones.
+            uniform_ = -off[0] / kRotEntries;
+            lw_.global -= off[1] / kRotEntries;
             out_.tables++;
             fma_ += 6.0;
         };
@@ -780,7 +811,7 @@ class Scheduler {
                         done.set(i);
                     }
             std::vector<std::pair<uint32_t, std::vector<int>>> by;  // register parity -> phases
-            long double A[kRotEntries] = {}, B[kRotEntries] = {};
+            ld A[kRotEntries] = {}, B[kRotEntries] = {};
             bool table = false;
             for (int i : f) {
                 const Item& x = *it[size_t(i)];
@@ -803,11 +834,12 @@ class Scheduler {
                 }
                 b->second.push_back(i);
             }
-            double G = 0.0;
+            ld G = 0.0;
             if (final) {
-                G = double(std::remainder(lw_.global, 2 * kPiL));
+                G = std::remainder(lw_.global, 2 * kPiL);
+                uniform_ += lw_.norm;
                 table = table || G != 0.0;
-                for (long double p : pend) table = table || p != 0.0;
+                for (ld p : pend) table = table || p != 0.0;
                 table = table || uniform_ != 0.0;
             }
             if (table) emit_table(A, B, G);
@@ -834,14 +866,16 @@ class Scheduler {
                 }
                 if (!angles.empty()) {
                     part_of(kRotSlots, angles);
-                    for (int i : angles) tables_.push_back(word(std::cos(it[size_t(i)]->a), std::sin(it[size_t(i)]->a)));
+                    ld off[2] = {};
+                    for (int i : angles) tables_.push_back(factor_word(1.0L, it[size_t(i)]->a, off));
+                    uniform_ -= off[0];
                     out_.slot_phases++;
                     fma_ += 6.0 + 6.0 * double(angles.size()) / kRotEntries;
                 }
                 if (!moduli.empty()) {
                     part_of(kRotSlotModuli, moduli);
                     for (int i : moduli) {
-                        const long double x = it[size_t(i)]->b;
+                        const ld x = it[size_t(i)]->b;
                         tables_.push_back(word(double(std::exp(x)), double(std::exp(-x))));
                     }
                     out_.slot_phases++;
@@ -887,7 +921,7 @@ class Scheduler {
                         for (size_t hi = h == g ? gi + 1 : 0; hi < groups[h].size() && in_place; hi++)
                             in_place = !((direction(it[size_t(groups[h][hi])]->v) >> low) & 1);
                 }
-                const long double lost = 0.5L * std::log1p((long double)(x.t) * x.t);
+                const ld lost = 0.5L * std::log1p(ld(x.t) * x.t);
                 Part part;
                 part.place = (d & (d - 1)) == 0 && !x.imag ? low : 4;
                 part.d = d;
@@ -896,14 +930,14 @@ class Scheduler {
                 part.signs = signs(r);
                 part.mask = slots(x.mask);
                 part.t = x.t;
-                part.u = x.t / (1.0 + x.t * x.t);
+                part.u = double(ld(x.t) / (1.0L + ld(x.t) * x.t));
                 if (part.kind == kRotKept) {
-                    part.u = 1.0 + x.t * x.t;
+                    part.u = double(1.0L + ld(x.t) * x.t);
                     uniform_ -= lost;
                 } else {
                     for (int j = 0; j < kRotRegBits; j++)
                         if (((d >> j) & 1) && pend[j] != 0.0) {
-                            long double A[kRotEntries] = {}, B[kRotEntries] = {};
+                            ld A[kRotEntries] = {}, B[kRotEntries] = {};
                             emit_table(A, B, 0.0);
                             break;
                         }
@@ -918,7 +952,7 @@ class Scheduler {
         }
         if (last || !tail.empty()) emit_flush(tail, last);
         if (!last && uniform_ < -kMaxOwed) {  // a circuit without phases: keep the amplitudes in range
-            long double A[kRotEntries] = {}, B[kRotEntries] = {};
+            ld A[kRotEntries] = {}, B[kRotEntries] = {};
             emit_table(A, B, 0.0);
         }
         // Factors still owed become phases of the register bits' parities (the
@@ -958,7 +992,7 @@ class Scheduler {
     }
 
     Bits applied_;
-    long double uniform_ = 0.0;  // logarithm of a factor all amplitudes are owed
+    ld uniform_ = 0.0;  // logarithm of a factor all amplitudes are owed
     std::vector<uint4> tables_;  // data of the tables and slot phases
 };
 

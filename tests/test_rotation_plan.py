@@ -1,0 +1,206 @@
+"""complex128 rotation passes (csrc/rotations.cpp, csrc/rotation_pass.cu).
+
+On the CPU a numpy replay of each pass's program, step by step as the kernel
+runs it, against the oracle, over every gate kind the form takes, tile sizes
+and circuit families; on the GPU the default complex128 path where it can go
+wrong (smallest and largest tiles, tiles sharing a CTA, programs too large for
+a launch argument, several trajectories).
+"""
+
+import struct
+
+import numpy as np
+import pytest
+
+from helpers import Circuit, brickwork, hea, inst, qft, random_circuit
+from oracle import oracle as o
+
+import dqsim
+from dqsim import _core, workloads
+
+PLAIN, SIGNED, KEPT, IMAG = range(4)
+TABLE, SLOTS, MODULI = 1 << 16, 1 << 17, 1 << 18
+SLOT_BITS = 9
+
+
+def parity(x):
+    x = np.asarray(x, dtype=np.uint64).copy()
+    for s in (32, 16, 8, 4, 2, 1):
+        x ^= x >> np.uint64(s)
+    return (x & np.uint64(1)).astype(np.int64)
+
+
+def sign(x):
+    return 1 - 2 * parity(x)
+
+
+def linear(x, vectors):
+    """XOR of vectors[b] over the set bits b of x."""
+    x = np.asarray(x, dtype=np.int64)
+    out = np.zeros_like(x)
+    for b, v in enumerate(vectors):
+        out ^= ((x >> b) & 1) * int(v)
+    return out
+
+
+def deposit(x, positions):
+    return linear(x, [1 << p for p in positions])
+
+
+def swizzle(p):
+    return p ^ (((p >> 3) ^ (p >> 6) ^ (p >> 9) ^ (p >> 12)) & 7)
+
+
+def pair(word):
+    return struct.unpack("<dd", struct.pack("<IIII", *word))
+
+
+def rotate(a, d, kind, t, u, signs):
+    low = d & -d
+    for v in range(16):
+        if v & low:
+            continue
+        s = -1 if (signs >> v) & 1 else 1
+        assert kind != PLAIN or s == 1
+        x, y = a[:, :, v], a[:, :, v ^ d]
+        if kind == KEPT:
+            x -= s * t * y
+            y *= u
+            y += s * t * x
+        elif kind == IMAG:
+            x -= 1j * s * t * y
+            y -= 1j * s * u * x
+        else:
+            x -= s * t * y
+            y += s * u * x
+
+
+def run_phase(a, words, data, head, index):
+    at = head[2][1]
+    for step in words[head[0][0]:head[0][0] + head[0][1]]:
+        todo = [(1 << j, ((step[0] >> (2 * j)) & 3) - 1) for j in range(4) if (step[0] >> (2 * j)) & 3]
+        if (step[0] >> 8) & 15:
+            todo.append(((step[0] >> 8) & 15, (step[0] >> 12) & 3))
+        for d, kind in todo:
+            t, u = pair(words[at])
+            at, signs, f = at + 1, 0, 1
+            if kind != PLAIN:
+                signs, mask = words[at][:2]
+                at, f = at + 1, sign(mask & index)
+            rotate(a, d, kind, t * f, u if kind == KEPT else u * f, signs)
+        if step[0] & TABLE:
+            a *= np.array([complex(*pair(w)) for w in words[data + step[1]:data + step[1] + 16]])
+        if step[0] & (SLOTS | MODULI):
+            n, signs = step[3] & 0xFFFF, step[3] >> 16
+            first = data + step[2]
+            plus = np.ones(index.shape, dtype=np.complex128)
+            minus = plus.copy()
+            for i in range(n):
+                s = sign(words[first + i // 4][i % 4] & index)
+                x, y = pair(words[first + (n + 3) // 4 + i])
+                if step[0] & SLOTS:
+                    plus *= x + 1j * y * s
+                    minus *= x - 1j * y * s
+                else:
+                    plus *= np.where(s < 0, y, x)
+                    minus *= np.where(s < 0, x, y)
+            for v in range(16):
+                a[:, :, v] *= minus if (signs >> v) & 1 else plus
+
+
+def replay(plan):
+    n = plan["n"]
+    state = np.zeros(1 << n, dtype=np.complex128)
+    state[0] = 1.0
+    for p in plan["passes"]:
+        tile = p["qubits"]
+        m = len(tile)
+        words = [tuple(int(x) for x in w) for w in np.array(p["words"], dtype=np.uint32).reshape(-1, 4)]
+        outer = np.arange(1 << (n - m))
+        index = deposit(outer, [q for q in range(n) if q not in tile])[:, None] | deposit(np.arange(1 << m), tile)
+        places = np.empty((outer.size, 1 << m), dtype=np.complex128)
+        places[:, swizzle(np.arange(1 << m))] = state[index]
+        slot = np.arange(1 << (m - 4))
+        for ph in range(p["phases"]):
+            head = words[3 * ph:3 * ph + 3]
+            halves = [h for w in (head[0][2:], head[1], head[2][:1]) for x in w for h in (x & 0xFFFF, x >> 16)]
+            full = linear(slot, halves[4:4 + m - 4])[:, None] ^ linear(np.arange(16), halves[:4])[None, :]
+            assert np.array_equal(np.sort(full.ravel()), np.arange(1 << m))  # every place once
+            a = places[:, full]
+            run_phase(a, words, p["data"], head, slot[None, :] | outer[:, None] << SLOT_BITS)
+            places[:, full] = a
+        e = np.arange(1 << m)
+        at = linear(e, p["out_dir"])[None, :] ^ p["out_const"] ^ linear(outer, p["out_outer"][:n - m])[:, None]
+        flips = parity(p["sign_local"] & e)[None, :] ^ parity(p["sign_outer"] & outer)[:, None] ^ p["sign_const"]
+        state[index] = np.take_along_axis(places, at, axis=1) * (1 - 2 * flips)
+    return state
+
+
+def oracle_state(circuit):
+    return o.OracleSimulator(seed=1).simulate(circuit).statevector
+
+
+def layers(n, depth):
+    return workloads.TransportCircuit(n, workloads.benchmark_layers(n, depth))
+
+
+@pytest.mark.parametrize("tile", [5, 8, 10])
+@pytest.mark.parametrize("maker", [lambda: brickwork(9, 8, seed=1, measure=False), lambda: qft(10, seed=3),
+                                   lambda: hea(10, 6, seed=4), lambda: layers(9, 8)])
+def test_rotation_passes_reproduce_the_oracle(maker, tile):
+    c = maker()
+    plan = _core.rotation_plan_dump(c.model_dump_json(), tile)
+    assert all(p["ok"] for p in plan["passes"])
+    np.testing.assert_allclose(replay(plan), oracle_state(c), atol=1e-13, rtol=0)
+
+
+def kinds():
+    """One instruction of every kind that random circuits draw."""
+    found = {}
+    for seed in range(40):
+        for g in random_circuit(seed, 6, 60):
+            found.setdefault((g["kind"], g.get("name")), g)
+    return sorted(found.items(), key=str)
+
+
+@pytest.mark.parametrize("name,gate", kinds(), ids=lambda x: str(x) if isinstance(x, tuple) else "")
+def test_every_gate_kind_between_entangling_layers(name, gate):
+    before = [inst("u3", qubit=q, theta=0.3 + q, phi=0.2 * q, lam=1.1 * q) for q in range(6)]
+    before += [inst("cx", control=q, target=q + 1) for q in range(5)]
+    after = [inst("u3", qubit=q, theta=1.3 * q, phi=0.4, lam=-0.7 * q) for q in range(6)]
+    c = Circuit(6, before + [gate] + after)
+    try:
+        plan = _core.rotation_plan_dump(c.model_dump_json(), 6)
+    except ValueError:
+        assert name[0] == "rc3x"  # wider than any tile operation
+        return
+    if not all(p["ok"] for p in plan["passes"]):
+        assert name[0] in ("rccx", "gate")  # dense matrices that are no Pauli rotation run in register phases
+        return
+    np.testing.assert_allclose(replay(plan), oracle_state(c), atol=1e-14, rtol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,tile", [(5, 5), (6, 5), (9, 5), (9, 9), (13, 13), (14, 13), (15, 12), (16, 0)])
+def test_rotation_kernel_against_the_oracle(n, tile):
+    for c in (brickwork(n, 7, seed=n, measure=False), qft(n, seed=n), hea(n, 5, seed=n), layers(n, 4)):
+        sim = dqsim.StatevectorSimulator(seed=1, tile_qubits=tile)
+        assert np.max(np.abs(sim.simulate(c).statevector - oracle_state(c))) <= 1e-12
+
+
+@pytest.mark.gpu
+def test_rotation_programs_larger_than_a_launch_argument():
+    c = brickwork(11, 120, seed=2, measure=False)  # one pass holds every operation
+    words = [len(p["words"]) // 4 for p in _core.rotation_plan_dump(c.model_dump_json(), 12)["passes"]]
+    assert min(words) > 1980
+    assert np.max(np.abs(dqsim.StatevectorSimulator(seed=1).simulate(c).statevector - oracle_state(c))) <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [5, 7, 10, 13])
+def test_rotation_passes_in_trajectories(n):
+    """Batches of states (tiles of several states to a CTA, ragged counts) with seeded counts equal to the oracle's."""
+    ins = workloads.benchmark_layers(n, 2) + [inst("measure", qubit=0, cbit=0)] + workloads.benchmark_layers(n, 2)
+    c = Circuit(n, ins + [inst("measure", qubit=q, cbit=q) for q in range(n)], n)
+    got = dqsim.StatevectorSimulator(seed=3).simulate_shots(c, shots=67)
+    assert got == o.OracleSimulator(seed=3).simulate_shots(c, shots=67)
