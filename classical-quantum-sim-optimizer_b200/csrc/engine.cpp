@@ -137,6 +137,16 @@ cudaMemPool_t g_pools[kMaxPoolDevices] = {};
 // Live Device objects per ordinal: the pool is shared by every simulator (and
 // result) on a device, so only the last one to go returns its cache.
 std::map<int, int> g_devices_live;
+// Devices whose kept block an allocation that runs short may take back.  Held
+// while a block is dropped, so that no Device goes meanwhile.
+std::mutex g_blocks_mu;
+std::vector<std::pair<int, Device*>> g_block_devices;
+
+void drop_blocks(int dev) {
+    std::lock_guard<std::mutex> l(g_blocks_mu);
+    for (auto& d : g_block_devices)
+        if (d.first == dev) d.second->drop_block();
+}
 
 cudaMemPool_t engine_pool(int dev) {
     std::lock_guard<std::mutex> l(g_devices_mu);
@@ -170,6 +180,7 @@ void trim_pool(bool sync_device) {
         std::lock_guard<std::mutex> l(g_devices_mu);
         pool = g_pools[dev];
     }
+    if (sync_device) drop_blocks(dev);
     if (!pool) return;
     if (sync_device) cudaDeviceSynchronize();
     cudaMemPoolTrimTo(pool, 0);
@@ -207,18 +218,39 @@ void DevMem::alloc_on(size_t b, cudaStream_t s, const char* what) {
     cuda_check(e, what);
     bytes = b;
     stream = s;
+    device = dev;
+}
+
+void DevMem::alloc_cached(size_t b, Device& d, const char* what) {
+    release();
+    if (b == 0) b = 16;
+    p = d.take_block(b);
+    if (p)
+        bytes = b;
+    else
+        alloc(b, what);
+    home = &d;
 }
 
 void DevMem::release() {
     if (p) {
-        if (stream)
+        if (stream) {
+            // (results and executors may go on a thread whose current device is another)
+            int now = device;
+            cudaGetDevice(&now);
+            if (now != device) cudaSetDevice(device);
             cudaFreeAsync(p, stream);
-        else
+            if (now != device) cudaSetDevice(now);
+        } else if (home) {
+            home->keep_block(p, bytes);
+        } else {
             cudaFree(p);
+        }
     }
     p = nullptr;
     bytes = 0;
     stream = nullptr;
+    home = nullptr;
 }
 
 Device::Device(int ord) : ordinal(ord) {
@@ -230,13 +262,55 @@ Device::Device(int ord) : ordinal(ord) {
     cuda_check(cudaSetDevice(ord), "cudaSetDevice");
     cuda_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
     engine_pool(ord);
-    std::lock_guard<std::mutex> l(g_devices_mu);
-    g_devices_live[ord]++;
+    {
+        std::lock_guard<std::mutex> l(g_devices_mu);
+        g_devices_live[ord]++;
+    }
+    std::lock_guard<std::mutex> l(g_blocks_mu);
+    g_block_devices.emplace_back(ord, this);
+}
+
+void* Device::take_block(size_t bytes) {
+    std::lock_guard<std::mutex> l(block_mu_);
+    if (!block_ || block_bytes_ != bytes) return nullptr;
+    void* p = block_;
+    block_ = nullptr;
+    return p;
+}
+
+void Device::keep_block(void* p, size_t bytes) {
+    void* old = nullptr;
+    {
+        std::lock_guard<std::mutex> l(block_mu_);
+        old = block_;
+        block_ = p;
+        block_bytes_ = bytes;
+    }
+    if (old) cudaFree(old);
+}
+
+void Device::drop_block() {
+    void* old = nullptr;
+    {
+        std::lock_guard<std::mutex> l(block_mu_);
+        old = block_;
+        block_ = nullptr;
+    }
+    if (old) cudaFree(old);
 }
 
 Device::~Device() {
     if (stream) {
+        {
+            std::lock_guard<std::mutex> l(g_blocks_mu);
+            for (size_t i = 0; i < g_block_devices.size(); i++)
+                if (g_block_devices[i].second == this) {
+                    g_block_devices.erase(g_block_devices.begin() + long(i));
+                    break;
+                }
+        }
         cudaSetDevice(ordinal);
+        drop_block();
         cudaStreamSynchronize(stream);
         cudaStreamDestroy(stream);
         bool last = false;
@@ -254,6 +328,11 @@ void Device::activate() const { cuda_check(cudaSetDevice(ordinal), "cudaSetDevic
 
 void Device::sync() { cuda_check(cudaStreamSynchronize(stream), "stream synchronize"); }
 
+void StateBatch::allocate(int n_, uint64_t W_, uint64_t ncb_, bool c64_, Device& d) {
+    amps.alloc_cached((size_t(W_) << n_) * (c64_ ? 8 : 16), d, "the statevector");
+    allocate(n_, W_, ncb_, c64_, d.stream);
+}
+
 void StateBatch::allocate(int n_, uint64_t W_, uint64_t ncb_, bool c64_, cudaStream_t pool_stream) {
     n = n_;
     W = W_;
@@ -268,7 +347,7 @@ void StateBatch::allocate(int n_, uint64_t W_, uint64_t ncb_, bool c64_, cudaStr
         else
             m.alloc(bytes, what);
     };
-    get(amps, (size_t(W) << n) * (c64 ? 8 : 16), "the statevector");
+    if (!amps.home) get(amps, (size_t(W) << n) * (c64 ? 8 : 16), "the statevector");
     get(cbits, size_t(W) * cwords * 8, "classical bits");
     get(seeds, size_t(W) * 8, "rng seeds");
     get(draws, size_t(W) * 8, "rng counters");
@@ -776,32 +855,32 @@ void Executor::prepare(const k::Batch& b) {
 void Executor::upload(cudaStream_t stream) {
     if (uploaded_) return;
     if (!pool_host_.empty()) {
-        pool_.alloc(pool_host_.size() * sizeof(double2), "gate matrices");
+        get(pool_, pool_host_.size() * sizeof(double2), stream, "gate matrices");
         cuda_check(cudaMemcpyAsync(pool_.p, pool_host_.data(), pool_host_.size() * sizeof(double2),
                                    cudaMemcpyHostToDevice, stream),
                    "upload gate matrices");
     }
     if (!tile_ops_host_.empty()) {
-        tile_ops_.alloc(tile_ops_host_.size() * sizeof(TileOp), "tile operations");
+        get(tile_ops_, tile_ops_host_.size() * sizeof(TileOp), stream, "tile operations");
         cuda_check(cudaMemcpyAsync(tile_ops_.p, tile_ops_host_.data(), tile_ops_host_.size() * sizeof(TileOp),
                                    cudaMemcpyHostToDevice, stream),
                    "upload tile operations");
     }
     if (!phase_words_host_.empty()) {
-        phase_words_.alloc(phase_words_host_.size() * sizeof(uint4), "tile phases");
+        get(phase_words_, phase_words_host_.size() * sizeof(uint4), stream, "tile phases");
         cuda_check(cudaMemcpyAsync(phase_words_.p, phase_words_host_.data(), phase_words_host_.size() * sizeof(uint4),
                                    cudaMemcpyHostToDevice, stream),
                    "upload tile phases");
     }
     if (!rot_words_host_.empty()) {
-        rot_words_.alloc(rot_words_host_.size() * sizeof(uint4), "rotation passes");
+        get(rot_words_, rot_words_host_.size() * sizeof(uint4), stream, "rotation passes");
         cuda_check(cudaMemcpyAsync(rot_words_.p, rot_words_host_.data(), rot_words_host_.size() * sizeof(uint4),
                                    cudaMemcpyHostToDevice, stream),
                    "upload rotation passes");
     }
     if (!fused_blocks_host_.empty()) {
-        fused_blocks_.alloc(fused_blocks_host_.size() * sizeof(FusedBlock), "fused block descriptors");
-        upool_.alloc(upool_host_.size() * sizeof(uint16_t), "fused block gate images");
+        get(fused_blocks_, fused_blocks_host_.size() * sizeof(FusedBlock), stream, "fused block descriptors");
+        get(upool_, upool_host_.size() * sizeof(uint16_t), stream, "fused block gate images");
         cuda_check(cudaMemcpyAsync(fused_blocks_.p, fused_blocks_host_.data(),
                                    fused_blocks_host_.size() * sizeof(FusedBlock), cudaMemcpyHostToDevice, stream),
                    "upload fused blocks");
@@ -851,8 +930,8 @@ void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, b
         if (s.fused >= 0) {
             const FusedPass& p = fused_[size_t(s.fused)];
             const size_t tiles = size_t(b.W) << (b.n - kFusedM);
-            norm_tiles_.ensure(tiles * 8, "fused tile norms");
-            norm_states_.ensure(size_t(b.W) * size_t(k::fused_norm_parts(b.n)) * 8, "fused state norms");
+            get(norm_tiles_, tiles * 8, b.stream, "fused tile norms");
+            get(norm_states_, size_t(b.W) * size_t(k::fused_norm_parts(b.n)) * 8, b.stream, "fused state norms");
             if (rec) rec->begin(kcFused, step_bytes(si, b));
             k::fused_pass(b, p, fused_blocks_.as<FusedBlock>(), upool_.as<uint16_t>(), b.err,
                           norm_pending ? norm_states_.as<double>() : nullptr, norm_tiles_.as<double>(),

@@ -26,10 +26,13 @@ void parallel_for(size_t count, const std::function<void(size_t)>& fn);
 
 // Owning device allocation.  Allocation failure is a MemoryError, as the
 // reference reports a failed statevector reservation (shots.rs:33-41).
+struct Device;
 struct DevMem {
     void* p = nullptr;
     size_t bytes = 0;
     cudaStream_t stream = nullptr;  // set: stream-ordered block from the engine's memory pool
+    int device = 0;                 // of a pool block
+    Device* home = nullptr;         // set: a block that goes back to its device's cache
     DevMem() = default;
     DevMem(const DevMem&) = delete;
     DevMem& operator=(const DevMem&) = delete;
@@ -39,6 +42,10 @@ struct DevMem {
     // block returns to the pool when released, in order on stream s, so the
     // next large buffer of the same size costs no driver mapping.
     void alloc_on(size_t b, cudaStream_t s, const char* what);
+    // A large buffer used on d's stream only: the one d keeps from an earlier
+    // owner when it has exactly this size, else a new allocation.  d must
+    // outlive it.
+    void alloc_cached(size_t b, Device& d, const char* what);
     void ensure(size_t b, const char* what) {
         if (b > bytes) alloc(b, what);
     }
@@ -58,6 +65,18 @@ struct Device {
     ~Device();
     void sync();
     void activate() const;
+    // One freed state buffer, kept for the next call of the same size on this
+    // stream (mapping gigabytes costs milliseconds, and cudaFree waits for the
+    // whole device).  Given back when another size replaces it, when an
+    // allocation on the device runs short, and with the Device.
+    void* take_block(size_t bytes);
+    void keep_block(void* p, size_t bytes);
+    void drop_block();
+
+  private:
+    std::mutex block_mu_;
+    void* block_ = nullptr;
+    size_t block_bytes_ = 0;
 };
 
 // W states of n qubits plus per-state classical bits and measurement scratch.
@@ -67,8 +86,11 @@ struct StateBatch {
     uint64_t W = 0, ncb = 0;
     int cwords = 1;
     bool c64 = false;
-    // With a stream, the statevector comes from the stream-ordered pool.
+    // With a stream, every buffer comes from the stream-ordered pool; with a
+    // device, the statevector comes from its cache and the rest from the pool
+    // on its stream.
     void allocate(int n, uint64_t W, uint64_t ncb, bool c64, cudaStream_t pool_stream = nullptr);
+    void allocate(int n, uint64_t W, uint64_t ncb, bool c64, Device& d);
     k::Batch view(cudaStream_t s, uint64_t W_active) const;
     size_t amp_bytes() const { return size_t(1) << n; }
 };
@@ -140,6 +162,9 @@ struct ExecConfig {
     // complex128 passes run as Pauli rotations (rotations.hpp) wherever every
     // operation of the pass has that form; the others in register phases.
     bool rotations = false;
+    // Gate images and scratch from the pool on the stream the executor runs
+    // on (which must outlive it): no device-wide wait when it goes.
+    bool pooled = false;
 };
 
 // How the fused plan of a segment was chosen: the portfolio's caps, the hand
@@ -238,6 +263,12 @@ class Executor {
     std::vector<int> widths_;
     std::vector<FusedPlanChoice> fused_choices_;
     void upload(cudaStream_t stream);
+    void get(DevMem& m, size_t bytes, cudaStream_t stream, const char* what) {
+        if (cfg_.pooled)
+            m.ensure_on(bytes, stream, what);
+        else
+            m.ensure(bytes, what);
+    }
     void lower(const Operation& op, std::vector<Condition>& conds);
     void lower_segment(const std::vector<Operation>& ops, size_t begin, size_t end);
     void add_tile_pass(TilePass&& p);

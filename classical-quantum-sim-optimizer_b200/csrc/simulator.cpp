@@ -145,6 +145,7 @@ ExecConfig exec_config(const Options& o, uint64_t n, bool force_per_gate, const 
     // The default complex128 passes are Pauli rotations; an explicit fusion
     // width asks for fused matrices of that width.
     c.rotations = !c.c64 && o.fusion_width == 0;
+    c.pooled = true;  // a simulator's executors run on its device's stream
     c.n = int(n);
     return c;
 }
@@ -431,7 +432,7 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
     cudaStream_t s = dev_->stream;
     StateBatch prefix;
     if (cache_prefix) {
-        prefix.allocate(int(n), 1, ncb, c64);
+        prefix.allocate(int(n), 1, ncb, c64, s);
         k::Batch pb = prefix.view(s, 1);
         reset_bookkeeping(prefix, 1, {seed}, s);
         Executor pre(ops, 0, prefix_end, exec_config(opt_, n));
@@ -439,7 +440,7 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
         pre.run(pb, nullptr, nullptr, true, pre.builds_basis());
     }
     StateBatch st;
-    st.allocate(int(n), workers, ncb, c64);
+    st.allocate(int(n), workers, ncb, c64, *dev_);
     Executor ex(ops, cache_prefix ? prefix_end : 0, ops.size(), exec_config(opt_, n));
     if (profile) out.shot_times.assign(shots, 0.0);
     std::vector<uint64_t> hbits(size_t(workers) * st.cwords);
@@ -495,7 +496,7 @@ std::unique_ptr<Result> Simulator::simulate(const char* json, size_t len) {
     auto res = std::make_unique<Result>();
     res->dev = dev_;
     res->n = n;
-    res->state.allocate(int(n), 1, ncb, opt_.precision == Precision::C64);
+    res->state.allocate(int(n), 1, ncb, opt_.precision == Precision::C64, *dev_);
     k::Batch b = res->state.view(s, 1);
     reset_bookkeeping(res->state, 1, {seed}, s);
     // Profiling times each reference operation, so it runs the per-gate form.
@@ -538,7 +539,7 @@ void Result::probabilities(const std::vector<uint64_t>& qubits, double* out) con
     dev->activate();
     const uint64_t m = uint64_t(1) << qubits.size();
     DevMem buf;
-    buf.alloc(m * 8, "probabilities");
+    buf.alloc_on(m * 8, dev->stream, "probabilities");
     k::Batch b = state.view(dev->stream, 1);
     probs_to(b, qubits, buf.as<double>());
     cuda_check(cudaMemcpyAsync(out, buf.p, m * 8, cudaMemcpyDeviceToHost, dev->stream), "read probabilities");
@@ -554,11 +555,11 @@ std::unordered_map<uint64_t, uint64_t> Result::counts(uint64_t shots, const std:
     cudaStream_t s = dev->stream;
     const uint64_t m = uint64_t(1) << qubits.size();
     DevMem cdf, tmp, idx;
-    cdf.alloc(m * 8, "the sampling table");
+    cdf.alloc_on(m * 8, s, "the sampling table");
     k::Batch b = state.view(s, 1);
     double total = build_sums(b, qubits, cdf.as<double>(), m, tmp);
     if (!std::isfinite(total) || total <= 0.0) fail(kRuntimeError, "Cannot sample a state with nonfinite or zero norm");
-    idx.alloc(shots * 8, "sampled outcomes");
+    idx.alloc_on(shots * 8, s, "sampled outcomes");
     k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), m, nullptr, total, true, seed, shots, false,
                    idx.as<uint64_t>());
     std::vector<uint64_t> h(shots);
@@ -573,8 +574,8 @@ double Result::fidelity(const double* other, uint64_t len) const {
     std::lock_guard<std::mutex> lk(dev->mu);
     dev->activate();
     DevMem o, part;
-    o.alloc(len * 16, "fidelity operand");
-    part.alloc(k::kDotBlocks * 16, "fidelity partial sums");
+    o.alloc_on(len * 16, dev->stream, "fidelity operand");
+    part.alloc_on(k::kDotBlocks * 16, dev->stream, "fidelity partial sums");
     cuda_check(cudaMemcpyAsync(o.p, other, len * 16, cudaMemcpyHostToDevice, dev->stream), "upload operand");
     k::Batch b = state.view(dev->stream, 1);
     int nb = k::dot_partials(b, o.as<double2>(), part.as<double2>());
@@ -597,8 +598,8 @@ void Result::amplitudes(const uint64_t* indices, uint64_t count, double* out) co
     std::lock_guard<std::mutex> lk(dev->mu);
     dev->activate();
     DevMem idx, buf;
-    idx.alloc(count * 8, "amplitude indices");
-    buf.alloc(count * 16, "amplitudes");
+    idx.alloc_on(count * 8, dev->stream, "amplitude indices");
+    buf.alloc_on(count * 16, dev->stream, "amplitudes");
     cuda_check(cudaMemcpyAsync(idx.p, indices, count * 8, cudaMemcpyHostToDevice, dev->stream), "upload indices");
     k::Batch b = state.view(dev->stream, 1);
     k::gather(b, idx.as<uint64_t>(), count, buf.as<double2>());
@@ -612,7 +613,7 @@ void Result::pauli_xz(uint64_t x, uint64_t z, double* re, double* im) const {
     std::lock_guard<std::mutex> lk(dev->mu);
     dev->activate();
     DevMem part;
-    part.alloc(k::kDotBlocks * 16, "expectation partial sums");
+    part.alloc_on(k::kDotBlocks * 16, dev->stream, "expectation partial sums");
     k::Batch b = state.view(dev->stream, 1);
     const int nb = k::pauli_partials(b, x, z, part.as<double2>());
     std::vector<double2> hp(static_cast<size_t>(nb));
