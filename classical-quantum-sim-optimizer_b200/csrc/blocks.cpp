@@ -160,7 +160,10 @@ void BlockContext::probabilities(const void* state, uint64_t n, const uint64_t* 
     }
     if (!qubits) fail(kValueError, "null qubit list");
     std::vector<int> q = qubit_list(n, qubits, kq, 40);
-    k::marginal(b, q, out);
+    DevMem scratch;  // returned to the pool in stream order
+    const size_t need = k::marginal_scratch(int(n), q);
+    if (need) scratch.alloc_on(need * 8, stream_, "marginal sums");
+    k::marginal(b, q, out, scratch.as<double>());
 }
 
 void BlockContext::running_sums(const void* state, uint64_t n, double* out) {

@@ -356,47 +356,105 @@ __global__ void k_norm2(const V* __restrict__ s, double* __restrict__ out, uint6
         out[g] = dev::norm2(s[g]);
 }
 
-struct QSel {
-    int k;
-    int q[64];
+// Marginal probabilities.  The state is read once, in index order: a CTA takes
+// chunks of 2^c amplitudes (c <= 12), each thread the 2^c / 256 elements t + 256 j
+// of a chunk, and adds the squared magnitudes of every chunk that only differs in
+// unselected high qubits into its own 16 sums.  The sums then meet in shared
+// memory, where those of one local output are added.  One CTA per value of the
+// selected high qubits and per part of the unselected ones; the parts' tables
+// are added by k_marginal_parts in order, so the result does not depend on
+// scheduling.
+constexpr int kMargBits = 12;  // local qubits of a chunk
+constexpr int kMargThreads = 256;
+
+struct MarginalPlan {
+    int c;                     // local qubits
+    int kl, kh;                // selected qubits below c, and from c up
+    int parts_bits;
+    uint64_t high_free;        // chunk-index bits of the unselected high qubits
+    uint8_t local_q[kMargBits], local_out[kMargBits];  // selected local qubit -> output bit (ascending)
+    uint8_t local_free[kMargBits];                     // unselected local qubits, ascending
+    uint8_t high_q[64], high_out[64];                  // selected high qubit (chunk-index bit) -> output bit
 };
 
-// Parallel bit deposit: the low bits of x go to the set bits of mask, in order.
-__device__ __forceinline__ uint64_t pdep(uint64_t x, uint64_t mask) {
-    uint64_t out = 0;
-    while (mask) {
-        uint64_t low = mask & (~mask + 1);
-        if (x & 1) out |= low;
-        x >>= 1;
-        mask ^= low;
-    }
-    return out;
+__device__ __forceinline__ uint64_t deposit_bits(uint64_t x, const uint8_t* to, int n) {
+    uint64_t r = 0;
+    for (int i = 0; i < n; i++) r |= ((x >> i) & 1) << to[i];
+    return r;
 }
 
-// out[j] = sum over the unselected bits r of |s[pdep(r, rest) | deposit(j)]|^2,
-// G threads per output summing r = lane, lane+G, ... then a fixed-order tree,
-// so the result does not depend on scheduling.
 template <typename V>
-__global__ void __launch_bounds__(256) k_marginal(const V* __restrict__ s, int n, QSel sel, uint64_t rest_mask,
-                                                 int G_bits, double* __restrict__ out, uint64_t nout) {
-    __shared__ double sm[256];
-    const int G = 1 << G_bits;
-    const int lane = threadIdx.x & (G - 1);
-    const uint64_t j = (uint64_t(blockIdx.x) * 256 + threadIdx.x) >> G_bits;
-    double acc = 0.0;
-    if (j < nout) {
-        uint64_t base = 0;
-        for (int t = 0; t < sel.k; t++) base |= ((j >> (sel.k - 1 - t)) & 1) << sel.q[t];
-        const uint64_t terms = uint64_t(1) << (n - sel.k);
-        for (uint64_t r = lane; r < terms; r += G) acc += dev::norm2(s[base | pdep(r, rest_mask)]);
+__global__ void __launch_bounds__(kMargThreads, 2)
+    k_marginal(const V* __restrict__ s, const __grid_constant__ MarginalPlan p, double* __restrict__ out,
+               uint64_t nout) {
+    constexpr int E = (1 << kMargBits) / kMargThreads;
+    __shared__ double sums[1 << kMargBits];
+    const uint32_t size = 1u << p.c;
+    const uint64_t part = blockIdx.x & ((uint64_t(1) << p.parts_bits) - 1);
+    const uint64_t h = blockIdx.x >> p.parts_bits;
+    const uint64_t fixed = deposit_bits(h, p.high_q, p.kh);
+    // Unselected high qubits: the part fixes the lowest of them, the loop runs over the others.
+    uint64_t mine = 0, loop = p.high_free;
+    for (int i = 0; i < p.parts_bits; i++) {
+        const uint64_t low = loop & (~loop + 1);
+        if ((part >> i) & 1) mine |= low;
+        loop ^= low;
     }
-    sm[threadIdx.x] = acc;
+    double acc[E];
+#pragma unroll
+    for (int j = 0; j < E; j++) acc[j] = 0.0;
+    uint64_t at = 0;
+    do {
+        const V* __restrict__ chunk = s + ((fixed | mine | at) << p.c);
+        V v[E];
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+            const uint32_t e = threadIdx.x + j * kMargThreads;
+            v[j] = e < size ? chunk[e] : dev::czero<V>();
+        }
+#pragma unroll
+        for (int j = 0; j < E; j++) acc[j] += dev::norm2(v[j]);
+        at = ((at | ~loop) + 1) & loop;
+    } while (at != 0);
+#pragma unroll
+    for (int j = 0; j < E; j++) {
+        const uint32_t e = threadIdx.x + j * kMargThreads;
+        if (e < size) sums[e] = acc[j];
+    }
     __syncthreads();
-    for (int w = G >> 1; w > 0; w >>= 1) {
-        if (lane < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-        __syncthreads();
+    // Local output x: the sum over the 2^(c - kl) elements with its selected
+    // bits, by G threads each and then by halves.
+    const int fb = p.c - p.kl;
+    const int gb = p.kl >= 8 ? 0 : (8 - p.kl < fb ? 8 - p.kl : fb);
+    const uint32_t G = 1u << gb, lane = threadIdx.x & (G - 1);
+    double* __restrict__ o = out + part * nout;
+    const uint64_t high_out = deposit_bits(h, p.high_out, p.kh);
+    const uint32_t step = kMargThreads >> gb;
+    for (uint32_t x0 = 0; x0 < (1u << p.kl); x0 += step) {
+        const uint32_t x = x0 + (threadIdx.x >> gb);
+        double sum = 0.0;
+        if (x < (1u << p.kl)) {
+            const uint32_t base = uint32_t(deposit_bits(x, p.local_q, p.kl));
+            for (uint32_t r = lane; r < (1u << fb); r += G)
+                sum += sums[base | uint32_t(deposit_bits(r, p.local_free, fb))];
+        }
+        for (uint32_t w = G >> 1; w >= 32; w >>= 1) {  // G > 32 only where one round covers every output
+            __syncthreads();
+            sums[threadIdx.x] = sum;
+            __syncthreads();
+            if (lane < w) sum += sums[threadIdx.x + w];
+        }
+        for (uint32_t w = G >= 32 ? 16 : G >> 1; w > 0; w >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, w);
+        if (lane == 0 && x < (1u << p.kl)) o[high_out | deposit_bits(x, p.local_out, p.kl)] = sum;
     }
-    if (lane == 0 && j < nout) out[j] = sm[threadIdx.x];
+}
+
+__global__ void k_marginal_parts(const double* __restrict__ parts, uint64_t nout, int count, double* __restrict__ out) {
+    const uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (j >= nout) return;
+    double sum = 0.0;
+    for (int i = 0; i < count; i++) sum += parts[uint64_t(i) * nout + j];
+    out[j] = sum;
 }
 
 constexpr int kScanItems = 8;
@@ -876,30 +934,58 @@ void norm2(const Batch& b, double* out) {
     check_launch("norm2");
 }
 
-void marginal(const Batch& b, const std::vector<int>& qubits, double* out) {
-    QSel sel{};
-    sel.k = int(qubits.size());
-    uint64_t sel_mask = 0;
-    for (int t = 0; t < sel.k; t++) {
-        sel.q[t] = qubits[t];
-        sel_mask |= uint64_t(1) << qubits[t];
+namespace {
+MarginalPlan marginal_plan(int n, const std::vector<int>& qubits) {
+    MarginalPlan p{};
+    p.c = std::min(n, kMargBits);
+    const int k = int(qubits.size());
+    std::vector<char> selected(size_t(n), 0);
+    for (int b = 0; b < k; b++) {  // output bit b
+        const int q = qubits[size_t(k - 1 - b)];
+        selected[size_t(q)] = 1;
+        if (q < p.c) {
+            p.local_q[p.kl] = uint8_t(q);
+            p.local_out[p.kl++] = uint8_t(b);
+        } else {
+            p.high_q[p.kh] = uint8_t(q - p.c);
+            p.high_out[p.kh++] = uint8_t(b);
+        }
     }
-    uint64_t full = b.n >= 64 ? ~uint64_t(0) : (uint64_t(1) << b.n) - 1;
-    uint64_t rest_mask = full & ~sel_mask;
-    int rest = b.n - sel.k;
-    uint64_t nout = uint64_t(1) << sel.k;
-    int G_bits = 0;
-    // About 2^20 threads in flight, at most 256 per output.
-    while (G_bits < 8 && G_bits < rest && (nout << (G_bits + 1)) <= (uint64_t(1) << 20)) G_bits++;
-    uint64_t threads = nout << G_bits;
-    unsigned grid = blocks_for(threads, 256);
+    int free = 0, high_free = 0;
+    for (int q = 0; q < n; q++) {
+        if (selected[size_t(q)]) continue;
+        if (q < p.c) {
+            p.local_free[free++] = uint8_t(q);
+        } else {
+            p.high_free |= uint64_t(1) << (q - p.c);
+            high_free++;
+        }
+    }
+    // About 8 CTAs to an SM, a part taking at least one chunk.
+    while (p.parts_bits < high_free && p.kh + p.parts_bits < 10) p.parts_bits++;
+    return p;
+}
+}  // namespace
+
+size_t marginal_scratch(int n, const std::vector<int>& qubits) {
+    const MarginalPlan p = marginal_plan(n, qubits);
+    return p.parts_bits ? size_t(1) << (p.parts_bits + int(qubits.size())) : 0;
+}
+
+void marginal(const Batch& b, const std::vector<int>& qubits, double* out, double* scratch) {
+    const MarginalPlan p = marginal_plan(b.n, qubits);
+    const uint64_t nout = uint64_t(1) << qubits.size();
+    const unsigned grid = blocks_for(uint64_t(1) << (p.kh + p.parts_bits), 1);
+    double* to = p.parts_bits ? scratch : out;
     if (b.c64)
-        k_marginal<float2><<<grid, 256, 0, b.stream>>>(static_cast<const float2*>(b.amps), b.n, sel, rest_mask, G_bits,
-                                                       out, nout);
+        k_marginal<float2><<<grid, kMargThreads, 0, b.stream>>>(static_cast<const float2*>(b.amps), p, to, nout);
     else
-        k_marginal<double2><<<grid, 256, 0, b.stream>>>(static_cast<const double2*>(b.amps), b.n, sel, rest_mask,
-                                                        G_bits, out, nout);
+        k_marginal<double2><<<grid, kMargThreads, 0, b.stream>>>(static_cast<const double2*>(b.amps), p, to, nout);
     check_launch("marginal");
+    if (p.parts_bits) {
+        k_marginal_parts<<<blocks_for(nout, 256), 256, 0, b.stream>>>(scratch, nout, 1 << p.parts_bits, out);
+        check_launch("marginal_parts");
+    }
 }
 
 size_t scan_tmp_size(uint64_t len) {

@@ -75,8 +75,10 @@ void broadcast(const Batch& b, const void* src);
 
 // |a_i|^2 into out (2^n doubles) for state 0.
 void norm2(const Batch& b, double* out);
-// Marginal probabilities over `qubits` (qubits[0] MSB) for state 0, 2^k doubles.
-void marginal(const Batch& b, const std::vector<int>& qubits, double* out);
+// Marginal probabilities over `qubits` (qubits[0] MSB) for state 0, 2^k doubles;
+// `scratch` holds marginal_scratch doubles (none: may be null).
+size_t marginal_scratch(int n, const std::vector<int>& qubits);
+void marginal(const Batch& b, const std::vector<int>& qubits, double* out, double* scratch);
 // In-place inclusive FP64 scan; `tmp` needs scan_tmp_size(len) doubles.
 size_t scan_tmp_size(uint64_t len);
 // Kernel launches scan (and scan_probs) makes for `len` entries.

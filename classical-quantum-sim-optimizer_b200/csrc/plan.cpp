@@ -137,7 +137,8 @@ double Plan::run(bool record) {
             k::scan_probs(bt, cdf_.as<double>(), tmp_.as<double>(), false);
         } else {
             std::vector<int> q(sample_qubits_.begin(), sample_qubits_.end());
-            k::marginal(bt, q, cdf_.as<double>());
+            marginal_.ensure_on(std::max<size_t>(1, k::marginal_scratch(int(n_), q)) * 8, s, "marginal sums");
+            k::marginal(bt, q, cdf_.as<double>(), marginal_.as<double>());
             k::scan_local(s, cdf_.as<double>(), clen, tmp_.as<double>());
         }
         k::take_total(s, cdf_.as<double>(), clen, tmp_.as<double>(), scalar_.as<double>(), st_.err.as<int>());

@@ -57,7 +57,7 @@ class Plan {
     std::vector<uint64_t> sample_qubits_;
     StateBatch st_;
     std::unique_ptr<Executor> ex_;
-    DevMem cdf_, tmp_, idx_, scalar_;
+    DevMem cdf_, tmp_, idx_, scalar_, marginal_;
     double ms_[kcNumClasses] = {}, bytes_[kcNumClasses] = {};
     uint64_t launches_[kcNumClasses] = {};
     double learned_ms_ = 0, greedy_ms_ = 0;

@@ -94,7 +94,10 @@ void probs_to(const k::Batch& b, const std::vector<uint64_t>& qubits, double* ou
     } else {
         std::vector<int> q;
         for (auto x : qubits) q.push_back(int(x));
-        k::marginal(b, q, out);
+        DevMem scratch;
+        const size_t need = k::marginal_scratch(b.n, q);
+        if (need) scratch.alloc_on(need * 8, b.stream, "marginal sums");
+        k::marginal(b, q, out, scratch.as<double>());
     }
 }
 
