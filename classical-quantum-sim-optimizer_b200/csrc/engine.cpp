@@ -901,7 +901,8 @@ void finish_tile_step(ProfileAcc* profile, cudaStream_t stream, std::chrono::ste
 }
 }  // namespace
 
-void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, bool normalize, bool from_basis) {
+void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, bool normalize, bool from_basis,
+                   bool discard) {
     upload(b.stream);
     std::vector<uint64_t> host_cbits;
     bool norm_pending = false;  // a fused pass left a norm the next fused pass divides out
@@ -980,6 +981,31 @@ void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, b
             if (rec) rec->end();
             finish_tile_step(profile, b.stream, t0);
             continue;
+        }
+        const bool plain_step = s.pass < 0 && s.rot < 0 && s.fused < 0;
+        if (plain_step && !profile && (s.type == Operation::Measure || s.type == Operation::Reset)) {
+            // Measurements in a row without conditions go as one run.
+            size_t end = si + 1;
+            if (s.type == Operation::Measure && s.cond.n == 0)
+                while (end < steps_.size() && end - si < size_t(k::measure_chain_max()) &&
+                       steps_[end].type == Operation::Measure && steps_[end].cond.n == 0 && steps_[end].pass < 0 &&
+                       steps_[end].rot < 0 && steps_[end].fused < 0)
+                    end++;
+            if (k::measure_chain_applies(b, int(end - si))) {
+                std::vector<int> qubits;
+                std::vector<int64_t> cbits;
+                for (size_t i = si; i < end; i++) {
+                    qubits.push_back(steps_[i].target);
+                    cbits.push_back(steps_[i].cbit);
+                }
+                // Branch sums read two states' worth; a kept state is read and written once more.
+                const bool keep = !(discard && end == steps_.size());
+                if (rec) rec->begin(kcMeasure, (keep ? 1.6 : 0.8) * step_bytes(si, b));
+                k::measure_chain(b, qubits, cbits, keep, s.type == Operation::Reset, s.cond);
+                if (rec) rec->end();
+                si = end - 1;
+                continue;
+            }
         }
         if (rec) {
             int cls = kcGate1q;

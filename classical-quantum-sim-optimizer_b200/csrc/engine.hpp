@@ -192,8 +192,9 @@ class Executor {
     // `from_basis`: every state of the batch is |0...0> on entry; a first step
     // that is a fused or a rotation pass then builds its input tiles itself
     // (the caller need not write the state first: builds_basis()).
+    // `discard`: the states are not read after the run (only classical bits are).
     void run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec = nullptr, bool normalize = true,
-             bool from_basis = false);
+             bool from_basis = false, bool discard = false);
     bool builds_basis() const { return !steps_.empty() && (steps_[0].fused >= 0 || steps_[0].rot >= 0); }
     // Uploads the matrix pools and sizes the scratch a run over batches like
     // `b` needs, so that later runs allocate nothing and copy nothing from the

@@ -328,6 +328,115 @@ __global__ void __launch_bounds__(kThreads) k_collapse(V* __restrict__ s, int n,
     }
 }
 
+// A run of measurements, one CTA per state.  Each outcome fixes a qubit, and the
+// next branch sums run over the amplitudes that agree with the outcomes so far,
+// so the sums read two states' worth in all and nothing is written until the
+// run ends: then the state is collapsed once (mode kChainKeep), reset (a run of
+// one, kChainReset) or left as it is when nothing follows that reads it
+// (kChainDiscard).  Separate measurements read and write 2.5 states each in
+// three launches.  States of up to 12 qubits keep their squared magnitudes in
+// shared memory.
+constexpr int kChainMax = 64;
+constexpr int kChainCached = 12;
+enum ChainMode : int { kChainDiscard = 0, kChainKeep = 1, kChainReset = 2 };
+
+struct MeasureList {
+    int count;
+    uint8_t q[kChainMax];
+    int64_t cbit[kChainMax];
+};
+
+__device__ __forceinline__ uint64_t deposit_mask(uint64_t x, uint64_t mask) {
+    uint64_t out = 0;
+    while (mask) {
+        const uint64_t low = mask & (~mask + 1);
+        if (x & 1) out |= low;
+        x >>= 1;
+        mask ^= low;
+    }
+    return out;
+}
+
+template <typename V>
+__global__ void k_measure_chain(V* __restrict__ s, int n, const __grid_constant__ MeasureList ml, int mode,
+                                CondList cond, const uint64_t* __restrict__ rng_seed, uint64_t* __restrict__ draws,
+                                uint64_t* __restrict__ cbits, int cwords, int* __restrict__ err) {
+    extern __shared__ double norms[];
+    __shared__ double branch;
+    __shared__ int result;
+    const uint64_t st = blockIdx.x;
+    if (cond.n && !dev::cond_ok(cond, cbits, cwords, st)) return;
+    V* __restrict__ a = s + (st << n);
+    const uint64_t len = uint64_t(1) << n;
+    const bool cached = n <= kChainCached;
+    if (cached) {
+        for (uint64_t i = threadIdx.x; i < len; i += blockDim.x) norms[i] = dev::norm2(a[i]);
+        __syncthreads();
+    }
+    uint64_t fixed = 0, value = 0;
+    uint64_t drawn = threadIdx.x == 0 ? draws[st] : 0;
+    for (int t = 0; t < ml.count; t++) {
+        const uint64_t bit = uint64_t(1) << ml.q[t];
+        double p0 = 0.0, p1 = 0.0;
+        if (!(fixed & bit)) {
+            const uint64_t free = (len - 1) ^ fixed;
+            const uint64_t count = uint64_t(1) << __popcll(free);
+            const uint64_t step = deposit_mask(blockDim.x, free);
+            uint64_t i = deposit_mask(threadIdx.x, free);
+            for (uint64_t k = threadIdx.x; k < count; k += blockDim.x) {
+                const double v = cached ? norms[i | value] : dev::norm2(a[i | value]);
+                if (i & bit)
+                    p1 += v;
+                else
+                    p0 += v;
+                i = ((i | ~free) + step) & free;
+            }
+            block_sum2(p0, p1);
+        }
+        if (threadIdx.x == 0) {
+            if (fixed & bit) {  // measured before in this run: its branch holds everything
+                p0 = value & bit ? 0.0 : branch;
+                p1 = value & bit ? branch : 0.0;
+            }
+            const double total = p0 + p1;
+            if (!(isfinite(total) && total > 0.0)) {
+                *err = 1;
+                result = -1;
+            } else {
+                const double r = dev::u64_to_unit(dev::chacha8_u64(rng_seed[st], drawn++));
+                const int o = r < p1 / total ? 1 : 0;
+                result = o;
+                branch = o ? p1 : p0;
+                const int64_t c = ml.cbit[t];
+                if (c >= 0) {
+                    uint64_t* w = cbits + st * uint64_t(cwords) + (uint64_t(c) >> 6);
+                    const uint64_t cb = uint64_t(1) << (uint64_t(c) & 63);
+                    *w = o ? (*w | cb) : (*w & ~cb);
+                }
+            }
+        }
+        __syncthreads();
+        const int o = result;
+        if (o < 0) break;
+        fixed |= bit;
+        if (o) value |= bit;
+        __syncthreads();  // `result` is read before the next round writes it
+    }
+    if (threadIdx.x == 0) draws[st] = drawn;
+    if (mode == kChainDiscard || fixed == 0) return;
+    const double sc = 1.0 / sqrt(branch);
+    if (mode == kChainReset) {
+        for (uint64_t j = threadIdx.x; j < len / 2; j += blockDim.x) {
+            const uint64_t i0 = (j & (fixed - 1)) | ((j & ~(fixed - 1)) << 1), i1 = i0 | fixed;
+            a[i0] = dev::cscale(a[value ? i1 : i0], sc);
+            a[i1] = dev::czero<V>();
+        }
+        return;
+    }
+    for (uint64_t i = threadIdx.x; i < len; i += blockDim.x)
+        a[i] = (i & fixed) == value ? dev::cscale(a[i], sc) : dev::czero<V>();
+}
+
 // ---------------------------------------------------------------------------
 // State initialisation
 // ---------------------------------------------------------------------------
@@ -882,6 +991,41 @@ void measure(const Batch& b, int qubit, int64_t cbit, bool reset, const CondList
         measure_t<float2>(b, qubit, cbit, reset, cond);
     else
         measure_t<double2>(b, qubit, cbit, reset, cond);
+}
+
+int measure_chain_max() { return kChainMax; }
+
+bool measure_chain_applies(const Batch& b, int count) {
+    // Microseconds of both forms, fitted on one B200: a CTA streams its state
+    // at about 60 GB/s, up to four a SM at a time; separate measurements take three
+    // launches and 2.5 passes at 5.5 TB/s.
+    const double bytes = double(uint64_t(1) << b.n) * (b.c64 ? 8.0 : 16.0);
+    const double rounds = std::ceil(double(b.W) / 592.0);
+    const double chain = 4.0 + 1.5 * count + rounds * 3.0 * bytes / 60e3;
+    const double separate = count * (12.0 + 2.5 * bytes * double(b.W) / 5.5e6);
+    return chain < separate && b.W <= 0x7fffffffULL;
+}
+
+void measure_chain(const Batch& b, const std::vector<int>& qubits, const std::vector<int64_t>& cbits, bool keep,
+                   bool reset, const dev::CondList& cond) {
+    if (qubits.empty() || qubits.size() > size_t(kChainMax) || (reset && qubits.size() != 1))
+        fail(kValueError, "a run of measurements holds 1 to 64 qubits");
+    MeasureList ml{};
+    ml.count = int(qubits.size());
+    for (size_t i = 0; i < qubits.size(); i++) {
+        ml.q[i] = uint8_t(qubits[i]);
+        ml.cbit[i] = cbits[i];
+    }
+    const int threads = 1 << std::min(9, std::max(5, b.n - 2));
+    const size_t smem = b.n <= kChainCached ? sizeof(double) << b.n : 0;
+    const int mode = reset ? kChainReset : keep ? kChainKeep : kChainDiscard;
+    if (b.c64)
+        k_measure_chain<float2><<<blocks_for(b.W, 1), threads, smem, b.stream>>>(
+            static_cast<float2*>(b.amps), b.n, ml, mode, cond, b.rng_seed, b.draws, b.cbits, b.cwords, b.err);
+    else
+        k_measure_chain<double2><<<blocks_for(b.W, 1), threads, smem, b.stream>>>(
+            static_cast<double2*>(b.amps), b.n, ml, mode, cond, b.rng_seed, b.draws, b.cbits, b.cwords, b.err);
+    check_launch("measure_chain");
 }
 
 void measure_draw(const Batch& b, int qubit, double draw, int* outcome) {

@@ -61,6 +61,15 @@ void dense(const Batch& b, const std::vector<int>& qubits, const double2* dmatri
 // sums, a ChaCha8 draw per state, collapse (engine.rs:367-426).  cbit < 0: no write.
 void measure(const Batch& b, int qubit, int64_t cbit, bool reset, const dev::CondList& cond);
 
+// A run of measurements (one CTA per state): the same outcomes and draws as
+// measure() one by one, with the state collapsed once at the end (`keep`) or
+// left as it is.  reset: a run of one that also returns its qubit to |0>.
+int measure_chain_max();
+// Whether the run is expected to take less time than measure() one by one.
+bool measure_chain_applies(const Batch& b, int count);
+void measure_chain(const Batch& b, const std::vector<int>& qubits, const std::vector<int64_t>& cbits, bool keep,
+                   bool reset, const dev::CondList& cond);
+
 // Measure one qubit of one state with a draw the caller supplies (uniform in
 // [0, 1)): branch sums, outcome = draw < p1 / (p0 + p1), collapse; the outcome
 // is returned to the host (the stream is synchronised).  engine.rs:367-426.

@@ -459,7 +459,7 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
         std::vector<uint64_t> seeds(Wr);
         for (uint64_t i = 0; i < Wr; i++) seeds[i] = seed + r0 + i;  // wrapping, shots.rs:224
         reset_bookkeeping(st, Wr, seeds, s);
-        ex.run(b, nullptr);
+        ex.run(b, nullptr, nullptr, true, false, /*discard=*/true);
         cuda_check(cudaMemcpyAsync(hbits.data(), st.cbits.p, size_t(Wr) * st.cwords * 8, cudaMemcpyDeviceToHost, s),
                    "read classical bits");
         check_err_flag(st, s);
