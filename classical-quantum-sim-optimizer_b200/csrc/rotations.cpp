@@ -15,7 +15,7 @@ constexpr long double kPiL = 3.14159265358979323846264338327950288L;
 // is then lost only where a factor is rounded for the kernel.
 using ld = long double;
 constexpr double kUnitaryTol = 1e-12;
-constexpr double kAngleTol = 2.3e-16;  // a quarter turn to the rounding of its angle
+constexpr double kAngleTol = 1.2e-16;  // no turn, or a quarter turn, to the rounding of the entries that give it
 constexpr int kMaxDiagQubits = 6;
 
 int parity64(uint64_t x) { return __builtin_parityll(x); }
@@ -35,14 +35,6 @@ struct Unsupported {};
 double norm2(cplx z) { return z.re * z.re + z.im * z.im; }
 ld arg(cplx z) { return std::atan2(ld(z.im), ld(z.re)); }
 ld modulus(cplx z) { return std::sqrt(ld(z.re) * z.re + ld(z.im) * z.im); }
-
-bool commute(const Item& x, const Item& y) {
-    if (!x.rot && !y.rot) return true;
-    int p = 0;
-    if (y.rot) p ^= parity64(x.mask & y.v);
-    if (x.rot) p ^= parity64(y.mask & x.v);
-    return p == 0;
-}
 
 // The gates of a pass as items, with the frame that relabels places.
 class Lowering {
@@ -101,7 +93,7 @@ class Lowering {
         const ld r = std::nearbyint(a / kPiL);
         a -= r * kPiL;
         if (std::fmod(std::fabs(r), 2.0L) == 1.0L) global += kPiL;
-        if (a == 0.0) return;
+        if (std::fabs(a) <= kAngleTol) return;
         if (std::fabs(std::fabs(a) - kPiL / 2) <= kAngleTol) {  // +-i Z^mask
             global += a > 0 ? kPiL / 2 : -kPiL / 2;
             sign ^= mask;
@@ -196,9 +188,8 @@ class Lowering {
                     mask ^= mask_[size_t(qubits[b])];
                     cons ^= cons_[size_t(qubits[b])];
                 }
-            // (phases that cancel leave the rounding of their sum)
             const ld a = phi[S] / ld(D);
-            if (std::fabs(a) > 1e-18L) phase(mask, cons, a);
+            if (a != 0.0) phase(mask, cons, a);
         }
     }
 
@@ -525,18 +516,25 @@ class Scheduler {
         const int W = int(std::min<size_t>(active_.size(), size_t(kWindow)));
         std::vector<const Item*> it(static_cast<size_t>(W));
         for (int i = 0; i < W; i++) it[size_t(i)] = &items_[size_t(active_[size_t(i)])];
-        std::vector<Bits> pred(static_cast<size_t>(W));
-        for (int j = 0; j < W; j++)
-            for (int i = 0; i < j; i++)
-                if (!commute(*it[size_t(i)], *it[size_t(j)])) pred[size_t(j)].set(i);
+        // Earlier items an item does not commute with (phases have no direction).
+        Bits pred[kWindow];
+        uint32_t dir[kWindow];
+        {
+            uint64_t mask[kWindow];
+            for (int j = 0; j < W; j++) {
+                dir[j] = it[size_t(j)]->v;
+                mask[j] = it[size_t(j)]->mask;
+                for (int i = 0; i < j; i++)
+                    pred[j].w[i >> 6] |= uint64_t(parity64((mask[i] & dir[j]) ^ (mask[j] & dir[i]))) << (i & 63);
+            }
+        }
         auto closure = [&](const Span& V, Bits& exec) {
             int rots = 0;
             exec = Bits{};
             for (int i = 0; i < W; i++) {
-                const Item& x = *it[size_t(i)];
-                if (!pred[size_t(i)].within(exec)) continue;
-                if (x.rot) {
-                    if (V.reduce(x.v)) continue;
+                if (!pred[i].within(exec)) continue;
+                if (dir[i]) {
+                    if (V.reduce(dir[i])) continue;
                     rots++;
                 }
                 exec.set(i);
@@ -552,7 +550,7 @@ class Scheduler {
             std::vector<uint32_t> cand;
             for (int i = 0; i < W && cand.size() < 8; i++) {
                 const Item& x = *it[size_t(i)];
-                if (!x.rot || exec.get(i) || !pred[size_t(i)].within(exec)) continue;
+                if (!x.rot || exec.get(i) || !pred[i].within(exec)) continue;
                 const uint32_t v = V.reduce(x.v);
                 if (v && std::find(cand.begin(), cand.end(), v) == cand.end()) cand.push_back(v);
             }
@@ -583,31 +581,33 @@ class Scheduler {
         // Order: rotations as far as they go, then the phases that hold the
         // next ones back, and so on.  `flush[f]` comes before the rotations of group f.
         std::vector<std::vector<int>> groups, flush;
-        Bits done;
+        Bits done, rot_bits;
+        for (int i = 0; i < W; i++)
+            if (dir[i]) rot_bits.set(i);
         while (true) {
             std::vector<int> g;
             for (int i = 0; i < W; i++)
-                if (it[size_t(i)]->rot && exec.get(i) && !done.get(i) && pred[size_t(i)].within(done)) {
+                if (it[size_t(i)]->rot && exec.get(i) && !done.get(i) && pred[i].within(done)) {
                     done.set(i);
                     g.push_back(i);
                 }
             groups.push_back(g);
-            std::vector<int> need;
+            Bits needed;
             for (int j = 0; j < W; j++) {
                 if (!it[size_t(j)]->rot || !exec.get(j) || done.get(j)) continue;
                 // Held back by phases only?
-                bool only = true;
-                for (int i = 0; i < j && only; i++)
-                    if (pred[size_t(j)].get(i) && !done.get(i) && it[size_t(i)]->rot) only = false;
-                if (!only) continue;
-                for (int i = 0; i < j; i++)
-                    if (pred[size_t(j)].get(i) && !done.get(i) && std::find(need.begin(), need.end(), i) == need.end())
-                        need.push_back(i);
+                Bits missing;
+                for (int w = 0; w < 2; w++) missing.w[w] = pred[j].w[w] & ~done.w[w];
+                if ((missing.w[0] & rot_bits.w[0]) || (missing.w[1] & rot_bits.w[1])) continue;
+                for (int w = 0; w < 2; w++) needed.w[w] |= missing.w[w];
             }
+            std::vector<int> need;
+            for (int i = 0; i < W; i++)
+                if (needed.get(i)) need.push_back(i);
             if (need.empty()) break;
             std::vector<int> ready;
             for (int i : need)
-                if (pred[size_t(i)].within(done)) ready.push_back(i);
+                if (pred[i].within(done)) ready.push_back(i);
             for (int i : ready) done.set(i);
             flush.push_back(ready);
         }
@@ -628,7 +628,7 @@ class Scheduler {
         std::vector<int> tail;
         if (last || std::all_of(groups.begin(), groups.end(), [](const std::vector<int>& g) { return g.empty(); }))
             for (int i = 0; i < W; i++)
-                if (!it[size_t(i)]->rot && !done.get(i) && pred[size_t(i)].within(done)) tail.push_back(i);
+                if (!it[size_t(i)]->rot && !done.get(i) && pred[i].within(done)) tail.push_back(i);
 
         // The slots' places: the complement of V in which the parities of up to
         // four of those phases vanish (their factors then depend on the
@@ -658,7 +658,7 @@ class Scheduler {
         for (int i : tail)
             if (!(it[size_t(i)]->mask & ~local)) take(it[size_t(i)]->mask);
         for (int i = 0; i < W; i++)
-            if (!it[size_t(i)]->rot && pred[size_t(i)].within(done) && !(it[size_t(i)]->mask & ~local))
+            if (!it[size_t(i)]->rot && pred[i].within(done) && !(it[size_t(i)]->mask & ~local))
                 take(it[size_t(i)]->mask);
         for (int b = 0; b < m_; b++) take(uint64_t(1) << b);
         // Place p shifted within its coset so that every M vanishes: solve
@@ -805,7 +805,7 @@ class Scheduler {
             for (int i : f) free_table = free_table || slots(it[size_t(i)]->mask) == 0;
             if (free_table)
                 for (int i = 0; i < W; i++)
-                    if (!it[size_t(i)]->rot && !done.get(i) && pred[size_t(i)].within(applied_) &&
+                    if (!it[size_t(i)]->rot && !done.get(i) && pred[i].within(applied_) &&
                         slots(it[size_t(i)]->mask) == 0 && std::find(f.begin(), f.end(), i) == f.end()) {
                         f.push_back(i);
                         done.set(i);
@@ -916,7 +916,7 @@ class Scheduler {
                     const uint64_t f = functional(low);
                     for (int j = 0; j < W && !in_place; j++)
                         in_place = !it[size_t(j)]->rot && !done.get(j) && it[size_t(j)]->mask == f &&
-                                   pred[size_t(j)].within(done);
+                                   pred[j].within(done);
                     for (size_t h = g; h < groups.size() && in_place; h++)
                         for (size_t hi = h == g ? gi + 1 : 0; hi < groups[h].size() && in_place; hi++)
                             in_place = !((direction(it[size_t(groups[h][hi])]->v) >> low) & 1);
@@ -977,7 +977,7 @@ class Scheduler {
             bool joined = false;
             for (int i = 0; i < W && !joined; i++) {
                 Item& x = items_[size_t(active_[size_t(i)])];
-                if (x.rot || applied_.get(i) || x.mask != f.mask || !pred[size_t(i)].within(applied_)) continue;
+                if (x.rot || applied_.get(i) || x.mask != f.mask || !pred[i].within(applied_)) continue;
                 x.b += f.b;
                 joined = true;
             }
