@@ -998,6 +998,40 @@ class Scheduler {
 
 }  // namespace
 
+namespace {
+
+// Whether an operation has a rotation form.
+bool rotation_form(const Operation& op) {
+    std::vector<uint64_t> q = op.touched();
+    std::sort(q.begin(), q.end());
+    auto local = [&](uint64_t x) { return uint64_t(std::lower_bound(q.begin(), q.end(), x) - q.begin()); };
+    Operation l = op;
+    l.target = local(op.target);
+    l.a = local(op.a);
+    l.b = local(op.b);
+    for (Control& c : l.controls) c.qubit = local(c.qubit);
+    for (uint64_t& x : l.qubits) x = local(x);
+    std::vector<int> tile;
+    for (size_t i = 0; i < q.size(); i++) tile.push_back(int(i));
+    try {
+        Lowering(tile, int(tile.size())).add(l);
+    } catch (const Unsupported&) {
+        return false;
+    }
+    return true;
+}
+
+}  // namespace
+
+bool rotation_targets_only(const std::vector<Operation>& ops, size_t begin, size_t end, int n, int m) {
+    m = std::min(m, n);
+    if (m < kRotMinTile || m > kRotMaxTile || n - m > kRotMaxOuter || n == m) return false;
+    bool wide = false;
+    for (size_t i = begin; i < end; i++) wide = wide || (ops[i].type == Operation::Diagonal && ops[i].qubits.size() > 1);
+    for (size_t i = begin; wide && i < end; i++) wide = rotation_form(ops[i]);
+    return wide;
+}
+
 bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<int>& tile_qubits, int n,
                          RotProgram& out) {
     const int m = int(tile_qubits.size());

@@ -94,10 +94,20 @@ inline uint32_t rot_swizzle(uint32_t p) {
     return p ^ (f & 7u);
 }
 
+// Whether ops[begin, end) are planned with the target qubits of a pass in its
+// tile only (TilePlanOptions::targets_only): all of them have a rotation form
+// (a pass that had to run in register phases would need every qubit) and some
+// are diagonal on several qubits.  Those reach out of the tile for a slot
+// phase each, and passes then hold far more of them (25-qubit QFT 9 -> 4
+// passes, 24-qubit ansatz 5 -> 4, both faster); with CX alone the phases lost
+// to slots outweigh the passes saved (27-qubit brickwork 13 -> 12, 3 % slower).
+bool rotation_targets_only(const std::vector<Operation>& ops, size_t begin, size_t end, int n, int m);
+
 // Plans the pass `ops` over `tile_qubits` (ascending) of an n-qubit state.
-// False when an operation has no such form (a dense matrix that is no Pauli
-// rotation, a matrix that is not unitary to 1e-12) or the tile is too small or
-// large.
+// Targets and swapped qubits are tile qubits; controls and diagonal qubits may
+// lie outside, where the tile's index gives their value.  False when an
+// operation has no such form (a dense matrix that is no Pauli rotation, a matrix
+// that is not unitary to 1e-12) or the tile is too small or large.
 bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<int>& tile_qubits, int n,
                          RotProgram& out);
 

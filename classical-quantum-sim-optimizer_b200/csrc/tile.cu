@@ -815,7 +815,8 @@ namespace {
 
 struct Dag {
     std::vector<std::vector<uint64_t>> qs;
-    std::vector<uint64_t> mask;                  // qubits of each op as a bit mask (n <= 64)
+    std::vector<uint64_t> mask;                  // qubits that must be tile qubits, as a bit mask (n <= 64)
+    std::vector<uint64_t> any;                   // all qubits of each op
     std::vector<std::vector<size_t>> per_qubit;  // op indices touching each qubit, in order
 };
 
@@ -842,8 +843,12 @@ size_t head_op(const Dag& g, const PlanState& s, size_t q) {
     return s.head[q] < g.per_qubit[q].size() ? g.per_qubit[q][s.head[q]] : SIZE_MAX;
 }
 
+// What a plan's coverage counts: an op that needs tile qubits far more than a
+// diagonal one that only rides along (targets_only).
+constexpr size_t kOpWeight = 64;
+
 // Absorbs every ready op inside T (bit mask) until nothing changes; appends
-// them to `taken` and returns how many.  Only an op at the head of one of its
+// them to `taken` and returns their weight.  Only an op at the head of one of its
 // qubits' lists can be ready, and taking an op moves only its own qubits'
 // heads, so a worklist of heads finds the whole closure.
 size_t closure(const Dag& g, PlanState& s, uint64_t T, std::vector<size_t>& taken, std::vector<size_t>& work) {
@@ -856,10 +861,10 @@ size_t closure(const Dag& g, PlanState& s, uint64_t T, std::vector<size_t>& take
     while (!work.empty()) {
         const size_t o = work.back();
         work.pop_back();
-        if (s.done[o] || (g.mask[o] & ~T) || !ready(g, s, o)) continue;
+        if (s.done[o] || (g.mask[o] & ~T) || !(g.any[o] & T) || !ready(g, s, o)) continue;
         take(g, s, o);
         taken.push_back(o);
-        count++;
+        count += g.mask[o] ? kOpWeight : 1;
         for (auto q : g.qs[o])
             if (head_op(g, s, q) != SIZE_MAX) work.push_back(head_op(g, s, q));
     }
@@ -918,7 +923,7 @@ size_t grow(const Dag& g, PlanState& s, size_t seed, const TileShape& sh, bool l
     const int m = sh.m, n = sh.n;
     const size_t first_open = s.first_open;
     taken.clear();
-    T = (sh.pinned >= 64 ? ~uint64_t(0) : (uint64_t(1) << sh.pinned) - 1) | g.mask[seed];
+    T = (sh.pinned >= 64 ? ~uint64_t(0) : (uint64_t(1) << sh.pinned) - 1) | (g.mask[seed] ? g.mask[seed] : g.any[seed]);
     if (n < 64) T &= (uint64_t(1) << n) - 1;
     int size = __builtin_popcountll(T);
     closure(g, s, T, taken, x.work);
@@ -930,17 +935,16 @@ size_t grow(const Dag& g, PlanState& s, size_t seed, const TileShape& sh, bool l
         }
         std::sort(x.cands.begin(), x.cands.end());
         x.cands.erase(std::unique(x.cands.begin(), x.cands.end()), x.cands.end());
-        size_t best = SIZE_MAX;
+        uint64_t best = 0;
         size_t best_gain = 0;
         int best_new = 1;
         x.tried.clear();  // new-qubit sets already scored
-        for (size_t o : x.cands) {
-            const uint64_t fresh = g.mask[o] & ~T;
+        auto score = [&](uint64_t fresh) {
             const int nw = __builtin_popcountll(fresh);
-            if (nw == 0 || size + nw > m) continue;
-            if (std::find(x.tried.begin(), x.tried.end(), fresh) != x.tried.end()) continue;
+            if (nw == 0 || size + nw > m) return;
+            if (std::find(x.tried.begin(), x.tried.end(), fresh) != x.tried.end()) return;
             x.tried.push_back(fresh);
-            if (sh.spread(T | fresh) > sh.max_spread) continue;
+            if (sh.spread(T | fresh) > sh.max_spread) return;
             size_t gain = 0;
             if (lookahead) {
                 const size_t fo = s.first_open;
@@ -951,14 +955,20 @@ size_t grow(const Dag& g, PlanState& s, size_t seed, const TileShape& sh, bool l
             }
             // gain / nw > best_gain / best_new, or equal with fewer new qubits
             const size_t lhs = gain * size_t(best_new), rhs = best_gain * size_t(nw);
-            if (best == SIZE_MAX || lhs > rhs || (lhs == rhs && nw < best_new)) {
-                best = o;
+            if (!best || lhs > rhs || (lhs == rhs && nw < best_new)) {
+                best = fresh;
                 best_gain = gain;
                 best_new = nw;
             }
+        };
+        for (size_t o : x.cands) {
+            score(g.mask[o] & ~T);
+            // A diagonal op that only has to touch the tile: by any one of its qubits.
+            if (!(g.any[o] & T))
+                for (uint64_t r = g.mask[o] ? 0 : g.any[o]; r; r &= r - 1) score(r & (~r + 1));
         }
-        if (best == SIZE_MAX) break;
-        T |= g.mask[best];
+        if (!best) break;
+        T |= best;
         size = __builtin_popcountll(T);
         closure(g, s, T, taken, x.work);
     }
@@ -966,7 +976,9 @@ size_t grow(const Dag& g, PlanState& s, size_t seed, const TileShape& sh, bool l
     s.first_open = first_open;
     // A depth limit keeps the first operations taken (a dependency-closed prefix).
     if (sh.max_ops && taken.size() > sh.max_ops) taken.resize(sh.max_ops);
-    return taken.size();
+    size_t weight = 0;
+    for (size_t o : taken) weight += g.mask[o] ? kOpWeight : 1;
+    return weight;
 }
 
 // One pass of a plan: its tile qubits (before padding) and the ops it takes.
@@ -1246,22 +1258,34 @@ std::vector<TilePass> plan_tiles(const std::vector<Operation>& ops, size_t begin
     std::vector<TilePass> passes;
     const size_t N = end - begin;
     if (N == 0) return passes;
-    // A pass holds every qubit of each of its operations.
+    auto needed = [&](const Operation& op) {
+        if (!opt.targets_only) return op.touched();
+        switch (op.type) {
+            case Operation::One:
+            case Operation::X: return std::vector<uint64_t>{op.target};
+            case Operation::Swap: return std::vector<uint64_t>{op.a, op.b};
+            case Operation::Diagonal: return std::vector<uint64_t>{};
+            default: return op.touched();
+        }
+    };
+    // A pass holds every qubit its operations need.
     int widest = 1;
-    for (size_t i = begin; i < end; i++) widest = std::max(widest, int(ops[i].touched().size()));
+    for (size_t i = begin; i < end; i++) widest = std::max(widest, int(needed(ops[i]).size()));
     const int pinned = std::min(std::max(opt.pinned_low, 0), n);
     const int m = std::min(std::max(opt.m, widest + pinned), n);
     if (n > 64) fail(kValueError, "tile passes take at most 64 qubits");
     Dag g;
     g.qs.resize(N);
     g.mask.assign(N, 0);
+    g.any.assign(N, 0);
     g.per_qubit.assign(n, {});
     for (size_t i = 0; i < N; i++) {
         g.qs[i] = ops[begin + i].touched();
         for (auto q : g.qs[i]) {
             g.per_qubit[q].push_back(i);
-            g.mask[i] |= uint64_t(1) << q;
+            g.any[i] |= uint64_t(1) << q;
         }
+        for (auto q : needed(ops[begin + i])) g.mask[i] |= uint64_t(1) << q;
     }
     const int beam = N > kPlanBeamMaxOps ? 1 : std::max(1, opt.beam);
     // A seed's own qubits are always allowed; the cap applies to the rest.

@@ -80,6 +80,11 @@ struct TilePlanOptions {
     // Shared-memory pass depth: at most this many operations per pass (0: no
     // limit).  Shallower passes cost more passes but less work per tile item.
     int max_pass_ops = 0;
+    // Only the qubits an operation moves amplitudes along (targets, swapped
+    // qubits, those of a dense matrix) must be tile qubits; controls and
+    // diagonal qubits may lie outside as long as one of the operation's qubits
+    // is in the tile (rotation passes, with keep_raw).
+    bool targets_only = false;
 };
 
 constexpr size_t kPlanBeamMaxOps = 50000;
