@@ -220,66 +220,89 @@ __global__ void k_first_amp(V* amps, const uint64_t* __restrict__ offs, int coun
     }
 }
 
-template <typename V>
-__global__ void k_arena_norm2(const V* __restrict__ amps, double* __restrict__ out, uint64_t len) {
-    for (uint64_t g = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < len; g += uint64_t(gridDim.x) * blockDim.x)
-        out[g] = dev::norm2(amps[g]);
-}
+// <Z0 Z1> per circuit: a CTA sums 2^kZzBits amplitudes, k_zz_total the CTAs of a
+// circuit in a fixed order (one CTA per circuit read a 20-qubit state in 2 ms).
+constexpr int kZzBits = 13;
 
-// <Z0 Z1> per circuit from its probabilities (one block per circuit, fixed-order tree).
-__global__ void k_zz(const double* __restrict__ probs, const uint64_t* __restrict__ offs, int count,
-                     double* __restrict__ out) {
-    __shared__ double sm[256];
-    const int c = blockIdx.x;
-    const uint64_t b = offs[c], e = offs[count + c];
+template <typename V>
+__global__ void __launch_bounds__(256) k_zz_parts(const V* __restrict__ amps, const uint64_t* __restrict__ offs, int count,
+                                                  const uint64_t* __restrict__ parts_at, double* __restrict__ parts) {
+    __shared__ double sm[8];
+    // The circuit of this CTA: the last one whose parts start at or before it.
+    int lo = 0, hi = count;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) / 2;
+        if (parts_at[mid] <= blockIdx.x)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    const uint64_t b = offs[lo], len = offs[count + lo] - b;
+    const uint64_t first = (blockIdx.x - parts_at[lo]) << kZzBits;
+    const uint64_t end = first + (uint64_t(1) << kZzBits) < len ? first + (uint64_t(1) << kZzBits) : len;
     double acc = 0.0;
-    for (uint64_t i = threadIdx.x; i < e - b; i += blockDim.x) {
-        double p = probs[b + i];
+#pragma unroll 8
+    for (uint64_t i = first + threadIdx.x; i < end; i += 256) {
+        const double p = dev::norm2(amps[b + i]);
         acc += ((i ^ (i >> 1)) & 1) ? -p : p;
     }
-    sm[threadIdx.x] = acc;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) acc += sm[w];
+        parts[blockIdx.x] = acc;
     }
-    if (threadIdx.x == 0) out[c] = sm[0];
 }
 
-// base/total of each circuit's segment of the global inclusive scan.
-__global__ void k_seg_totals(const double* __restrict__ scan, const uint64_t* __restrict__ offs, int count,
-                             double* __restrict__ base_total, int* __restrict__ err) {
+__global__ void k_zz_total(const double* __restrict__ parts, const uint64_t* __restrict__ parts_at, int count,
+                           double* __restrict__ out) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= count) return;
+    double acc = 0.0;
+    for (uint64_t i = parts_at[c]; i < parts_at[c + 1]; i++) acc += parts[i];
+    out[c] = acc;
+}
+
+// Entry i of the arena's running sums: its tile's sum plus the tiles before.
+__device__ __forceinline__ double running_sum(const double* __restrict__ x, const double* __restrict__ tiles,
+                                              uint64_t i) {
+    double v = x[i];
+    if (i >= uint64_t(k::kScanTileEntries)) v = v + tiles[i / uint64_t(k::kScanTileEntries) - 1];
+    return v;
+}
+
+// base/total of each circuit's segment of the arena's running sums.
+__global__ void k_seg_totals(const double* __restrict__ scan, const double* __restrict__ tiles,
+                             const uint64_t* __restrict__ offs, int count, double* __restrict__ base_total,
+                             int* __restrict__ err) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= count) return;
     uint64_t b = offs[c], e = offs[count + c];
-    double base = b > 0 ? scan[b - 1] : 0.0;
-    double tot = scan[e - 1] - base;
+    double base = b > 0 ? running_sum(scan, tiles, b - 1) : 0.0;
+    double tot = running_sum(scan, tiles, e - 1) - base;
     if (!(isfinite(tot) && tot > 0.0)) atomicExch(err, 1);
     base_total[2 * c] = base;
     base_total[2 * c + 1] = tot;
 }
 
-__global__ void k_seg_normalize(double* __restrict__ cdf, const uint64_t* __restrict__ offs, int count,
-                                const double* __restrict__ base_total) {
-    int c = blockIdx.y;
-    uint64_t b = offs[c], e = offs[count + c];
-    double base = base_total[2 * c], tot = base_total[2 * c + 1];
-    for (uint64_t i = b + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < e; i += uint64_t(gridDim.x) * blockDim.x)
-        cdf[i] = (i == e - 1) ? 1.0 : (cdf[i] - base) / tot;
-}
-
-__global__ void k_seg_sample(const double* __restrict__ cdf, const uint64_t* __restrict__ offs, int count,
+// Draws each shot by binary search; a probed entry is normalised as it is read
+// (the last one of a circuit is 1), so no pass over the table does it.
+__global__ void k_seg_sample(const double* __restrict__ scan, const double* __restrict__ tiles,
+                             const uint64_t* __restrict__ offs, int count, const double* __restrict__ base_total,
                              const uint64_t* __restrict__ seeds, uint64_t shots, uint64_t* __restrict__ out) {
     uint64_t g = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (g >= uint64_t(count) * shots) return;
     int c = int(g / shots);
     uint64_t t = g % shots;
     uint64_t b = offs[c], e = offs[count + c];
+    const double base = base_total[2 * c], tot = base_total[2 * c + 1];
     double draw = dev::u64_to_unit(dev::chacha8_u64(seeds[c] + t, 0));
     uint64_t lo = b, hi = e;
     while (lo < hi) {
         uint64_t mid = lo + (hi - lo) / 2;
-        if (cdf[mid] <= draw)
+        const double v = mid == e - 1 ? 1.0 : (running_sum(scan, tiles, mid) - base) / tot;
+        if (v <= draw)
             lo = mid + 1;
         else
             hi = mid;
@@ -426,6 +449,14 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
                "upload");
     cuda_check(cudaMemcpyAsync(circ_off_.p, offs.data(), offs.size() * 8, cudaMemcpyHostToDevice, s), "upload");
     cuda_check(cudaMemcpyAsync(seeds_.p, seeds.data(), seeds.size() * 8, cudaMemcpyHostToDevice, s), "upload");
+    std::vector<uint64_t> zz_at(1, 0);
+    for (const Circ& c : circuits_)
+        zz_at.push_back(zz_at.back() + (((uint64_t(1) << c.n) + (uint64_t(1) << kZzBits) - 1) >> kZzBits));
+    zz_parts_ = zz_at.back();
+    if (zz_parts_ > 0x7fffffffULL) fail(kMemoryError, "batch too large");
+    zz_at_.alloc(zz_at.size() * 8, "expectation parts");
+    zz_sums_.alloc(std::max<uint64_t>(1, zz_parts_) * 8, "expectation parts");
+    cuda_check(cudaMemcpyAsync(zz_at_.p, zz_at.data(), zz_at.size() * 8, cudaMemcpyHostToDevice, s), "upload");
     // Fused circuits: executors prepared (pools uploaded, scratch sized) so that
     // runs allocate nothing and can be captured; longest first onto the least
     // loaded side stream.
@@ -589,21 +620,22 @@ void BatchRun::enqueue() {
                                                               err_.as<int>());
     }
     for (cudaEvent_t e : join_) cuda_check(cudaStreamWaitEvent(s, e, 0), "join");
-    const unsigned sgrid = unsigned(std::min<uint64_t>((total_amps_ + 255) / 256, 148 * 32));
     if (c64_)
-        k_arena_norm2<float2><<<sgrid, 256, 0, s>>>(amps_.as<float2>(), probs_.as<double>(), total_amps_);
+        k_zz_parts<float2><<<unsigned(zz_parts_), 256, 0, s>>>(amps_.as<float2>(), offs, count, zz_at_.as<uint64_t>(),
+                                                               zz_sums_.as<double>());
     else
-        k_arena_norm2<double2><<<sgrid, 256, 0, s>>>(amps_.as<double2>(), probs_.as<double>(), total_amps_);
-    k_zz<<<count, 256, 0, s>>>(probs_.as<double>(), offs, count, zz_part_.as<double>());
+        k_zz_parts<double2><<<unsigned(zz_parts_), 256, 0, s>>>(amps_.as<double2>(), offs, count,
+                                                                zz_at_.as<uint64_t>(), zz_sums_.as<double>());
+    k_zz_total<<<(count + 127) / 128, 128, 0, s>>>(zz_sums_.as<double>(), zz_at_.as<uint64_t>(), count,
+                                                   zz_part_.as<double>());
     double* tmp = tmp_.as<double>();
     double* base_total = tmp + k::scan_tmp_size(total_amps_);
-    k::scan(s, probs_.as<double>(), total_amps_, tmp);
-    k_seg_totals<<<(count + 127) / 128, 128, 0, s>>>(probs_.as<double>(), offs, count, base_total, err_.as<int>());
-    k_seg_normalize<<<dim3(64, count), 256, 0, s>>>(probs_.as<double>(), offs, count, base_total);
+    k::scan_states(s, c64_, amps_.p, total_amps_, probs_.as<double>(), tmp);
+    k_seg_totals<<<(count + 127) / 128, 128, 0, s>>>(probs_.as<double>(), tmp, offs, count, base_total, err_.as<int>());
     if (shots_ > 0) {
         const uint64_t th = uint64_t(count) * shots_;
-        k_seg_sample<<<unsigned((th + 127) / 128), 128, 0, s>>>(probs_.as<double>(), offs, count, seeds_.as<uint64_t>(),
-                                                                shots_, samples_.as<uint64_t>());
+        k_seg_sample<<<unsigned((th + 127) / 128), 128, 0, s>>>(probs_.as<double>(), tmp, offs, count, base_total,
+                                                                seeds_.as<uint64_t>(), shots_, samples_.as<uint64_t>());
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) fail(kCudaError, std::string("batch launch: ") + cudaGetErrorString(e));

@@ -88,10 +88,10 @@ class BatchRun {
     std::vector<PassRec> pass_recs_;
     std::vector<TileOp> ops_host_;
     std::vector<double2> pool_host_;
-    uint64_t total_items_ = 0, total_amps_ = 0;
+    uint64_t total_items_ = 0, total_amps_ = 0, zz_parts_ = 0;
     int max_m_ = 0;
     DevMem amps_, recs_, ops_, pool_, done_, head_, err_, probs_, tmp_, circ_off_, circ_of_tile_, samples_, zz_part_,
-        seeds_;
+        zz_at_, zz_sums_, seeds_;
     cudaGraphExec_t graph_ = nullptr;
     std::vector<cudaStream_t> side_;
     std::vector<cudaEvent_t> join_;

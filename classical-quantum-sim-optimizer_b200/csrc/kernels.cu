@@ -568,6 +568,7 @@ __global__ void k_marginal_parts(const double* __restrict__ parts, uint64_t nout
 
 constexpr int kScanItems = 8;
 constexpr int kScanTile = 256 * kScanItems;
+static_assert(kScanTile == kScanTileEntries, "the tile that callers index by");
 
 // Tile-local inclusive scan of `in` into x (V = double: in == x, in place;
 // V = float2 / double2: the squared magnitudes of a state, as k_norm2 computes
@@ -1179,6 +1180,16 @@ void scan_local(cudaStream_t s, double* x, uint64_t len, double* tmp) {
     uint64_t nb = (len + kScanTile - 1) / kScanTile;
     k_scan_tiles<double><<<blocks_for(nb, 1), 256, 0, s>>>(x, x, len, tmp);
     check_launch("scan_tiles");
+    if (nb > 1) scan(s, tmp, nb, tmp + nb);
+}
+
+void scan_states(cudaStream_t s, bool c64, const void* amps, uint64_t len, double* x, double* tmp) {
+    const uint64_t nb = (len + kScanTile - 1) / kScanTile;
+    if (c64)
+        k_scan_tiles<float2><<<blocks_for(nb, 1), 256, 0, s>>>(static_cast<const float2*>(amps), x, len, tmp);
+    else
+        k_scan_tiles<double2><<<blocks_for(nb, 1), 256, 0, s>>>(static_cast<const double2*>(amps), x, len, tmp);
+    check_launch("scan_states");
     if (nb > 1) scan(s, tmp, nb, tmp + nb);
 }
 

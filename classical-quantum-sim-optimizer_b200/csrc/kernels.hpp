@@ -117,6 +117,9 @@ void scan_probs(const Batch& b, double* x, double* tmp, bool add_tiles = true);
 // the inclusive sums of whole tiles (entry i of the full scan is x[i] +
 // tmp[i / 2048 - 1] for i >= 2048).
 void scan_local(cudaStream_t s, double* x, uint64_t len, double* tmp);
+constexpr int kScanTileEntries = 2048;
+// scan_local of the squared magnitudes of `len` amplitudes (any number).
+void scan_states(cudaStream_t s, bool c64, const void* amps, uint64_t len, double* x, double* tmp);
 uint64_t scan_tile_of(uint64_t i);
 // *scalar = entry len-1 of the (two-level when tiles) sums; *err = 1 when it is
 // not finite and positive.
