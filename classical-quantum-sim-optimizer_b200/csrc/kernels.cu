@@ -383,7 +383,27 @@ __global__ void k_measure_chain(V* __restrict__ s, int n, const __grid_constant_
             const uint64_t count = uint64_t(1) << __popcll(free);
             const uint64_t step = deposit_mask(blockDim.x, free);
             uint64_t i = deposit_mask(threadIdx.x, free);
-            for (uint64_t k = threadIdx.x; k < count; k += blockDim.x) {
+            uint64_t k = threadIdx.x;
+            // Four loads in flight: a CTA alone has to keep its state's reads going.
+            for (; !cached && k + 3 * uint64_t(blockDim.x) < count; k += 4 * uint64_t(blockDim.x)) {
+                V v[4];
+                uint64_t at[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    at[u] = i;
+                    v[u] = a[i | value];
+                    i = ((i | ~free) + step) & free;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const double x = dev::norm2(v[u]);
+                    if (at[u] & bit)
+                        p1 += x;
+                    else
+                        p0 += x;
+                }
+            }
+            for (; k < count; k += blockDim.x) {
                 const double v = cached ? norms[i | value] : dev::norm2(a[i | value]);
                 if (i & bit)
                     p1 += v;
@@ -433,8 +453,19 @@ __global__ void k_measure_chain(V* __restrict__ s, int n, const __grid_constant_
         }
         return;
     }
-    for (uint64_t i = threadIdx.x; i < len; i += blockDim.x)
-        a[i] = (i & fixed) == value ? dev::cscale(a[i], sc) : dev::czero<V>();
+    for (uint64_t i = threadIdx.x; i < len; i += 4 * uint64_t(blockDim.x)) {
+        V v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint64_t at = i + u * uint64_t(blockDim.x);
+            v[u] = at < len && (at & fixed) == value ? a[at] : dev::czero<V>();
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint64_t at = i + u * uint64_t(blockDim.x);
+            if (at < len) a[at] = (at & fixed) == value ? dev::cscale(v[u], sc) : dev::czero<V>();
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -433,18 +433,27 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
     std::lock_guard<std::mutex> lk(dev_->mu);
     dev_->activate();
     cudaStream_t s = dev_->stream;
+    // The executors are kept with the circuit's cached plan (the device lock
+    // above serialises their use), or built for this call.
+    ShotPlan own;
+    ShotPlan& sp = shot_plan ? *shot_plan : own;
     StateBatch prefix;
     if (cache_prefix) {
         prefix.allocate(int(n), 1, ncb, c64, s);
         k::Batch pb = prefix.view(s, 1);
         reset_bookkeeping(prefix, 1, {seed}, s);
-        Executor pre(ops, 0, prefix_end, exec_config(opt_, n));
-        if (!pre.builds_basis()) k::init_basis(pb);
-        pre.run(pb, nullptr, nullptr, true, pre.builds_basis());
+        if (!sp.prefix) sp.prefix = std::make_unique<Executor>(ops, 0, prefix_end, exec_config(opt_, n));
+        if (!sp.prefix->builds_basis()) k::init_basis(pb);
+        sp.prefix->run(pb, nullptr, nullptr, true, sp.prefix->builds_basis());
     }
     StateBatch st;
     st.allocate(int(n), workers, ncb, c64, *dev_);
-    Executor ex(ops, cache_prefix ? prefix_end : 0, ops.size(), exec_config(opt_, n));
+    const size_t begin = cache_prefix ? prefix_end : 0;
+    if (!sp.rest || sp.rest_begin != begin) {
+        sp.rest = std::make_unique<Executor>(ops, begin, ops.size(), exec_config(opt_, n));
+        sp.rest_begin = begin;
+    }
+    Executor& ex = *sp.rest;
     if (profile) out.shot_times.assign(shots, 0.0);
     std::vector<uint64_t> hbits(size_t(workers) * st.cwords);
     std::vector<uint8_t> cb(ncb);

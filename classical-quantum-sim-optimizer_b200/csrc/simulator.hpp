@@ -98,15 +98,17 @@ class Result {
 };
 
 // A circuit text this simulator ran through simulate_shots: its compiled
-// operations and, once a terminal-sampling call has planned it, the executor
-// of its unitary prefix (passes, fused blocks and gate images on the device).
+// operations and, once a call has planned them, the executors of its unitary
+// prefix and of the operations a trajectory runs (passes, fused blocks and gate
+// images on the device).
 // A call with the byte-identical text reuses both, skipping parse, validation,
 // compilation and planning, which give the same result for the same text.
 struct ShotPlan {
     std::string json;
     std::vector<Operation> ops;
     uint64_t n = 0, ncb = 0;
-    std::unique_ptr<Executor> prefix;
+    std::unique_ptr<Executor> prefix, rest;
+    size_t rest_begin = 0;
 };
 
 // Device buffers of terminal sampling, kept by a simulator between calls:
