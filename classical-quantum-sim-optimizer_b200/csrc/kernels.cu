@@ -1137,8 +1137,9 @@ MarginalPlan marginal_plan(int n, const std::vector<int>& qubits) {
             high_free++;
         }
     }
-    // About 8 CTAs to an SM, a part taking at least one chunk.
-    while (p.parts_bits < high_free && p.kh + p.parts_bits < 10) p.parts_bits++;
+    // About 8 CTAs to an SM, a part taking at least one chunk; up to four chunks
+    // take less time in one CTA than a second launch.
+    while (high_free > 2 && p.parts_bits < high_free && p.kh + p.parts_bits < 10) p.parts_bits++;
     return p;
 }
 }  // namespace

@@ -33,8 +33,29 @@ struct Item {
 struct Unsupported {};
 
 double norm2(cplx z) { return z.re * z.re + z.im * z.im; }
-ld arg(cplx z) { return std::atan2(ld(z.im), ld(z.re)); }
+ld arg(cplx z) {
+    if (z.im == 0.0) return z.re < 0 ? kPiL : 0.0L;
+    return std::atan2(ld(z.im), ld(z.re));
+}
 ld modulus(cplx z) { return std::sqrt(ld(z.re) * z.re + ld(z.im) * z.im); }
+
+bool unitary(const Mat2& u) {
+    const double dev[] = {std::fabs(norm2(u[0][0]) + norm2(u[1][0]) - 1.0),
+                          std::fabs(norm2(u[0][1]) + norm2(u[1][1]) - 1.0),
+                          std::fabs(u[0][0].re * u[0][1].re + u[0][0].im * u[0][1].im + u[1][0].re * u[1][1].re +
+                                    u[1][0].im * u[1][1].im),
+                          std::fabs(u[0][0].re * u[0][1].im - u[0][0].im * u[0][1].re + u[1][0].re * u[1][1].im -
+                                    u[1][0].im * u[1][1].re)};
+    for (double d : dev)
+        if (!(d <= kUnitaryTol)) return false;
+    return true;
+}
+
+bool unit_moduli(const std::vector<cplx>& values) {
+    for (cplx d : values)
+        if (!(std::fabs(norm2(d) - 1.0) <= kUnitaryTol)) return false;
+    return true;
+}
 
 // The gates of a pass as items, with the frame that relabels places.
 class Lowering {
@@ -215,13 +236,7 @@ class Lowering {
     void one(uint64_t target, const Mat2& u, const std::vector<Control>& controls) {
         // u = e^{i alpha} RZ(beta) RY(theta) RZ(gamma)
         const ld c = modulus(u[0][0]), s = modulus(u[1][0]);
-        const double dev[] = {std::fabs(double(c * c + s * s - 1.0L)), std::fabs(norm2(u[0][1]) + norm2(u[1][1]) - 1.0),
-                              std::fabs(u[0][0].re * u[0][1].re + u[0][0].im * u[0][1].im + u[1][0].re * u[1][1].re +
-                                        u[1][0].im * u[1][1].im),
-                              std::fabs(u[0][0].re * u[0][1].im - u[0][0].im * u[0][1].re + u[1][0].re * u[1][1].im -
-                                        u[1][0].im * u[1][1].re)};
-        for (double d : dev)
-            if (!(d <= kUnitaryTol)) throw Unsupported{};
+        if (!unitary(u)) throw Unsupported{};
         // Arguments of u00, u10 and u11; the fourth entry's follows from
         // unitarity, so the smaller pair gives one argument only.
         ld A, B, D;
@@ -319,11 +334,9 @@ class Lowering {
     }
 
     void diagonal(const Operation& op) {
+        if (!unit_moduli(op.values)) throw Unsupported{};
         std::vector<ld> phi;
-        for (cplx d : op.values) {
-            if (!(std::fabs(norm2(d) - 1.0) <= kUnitaryTol)) throw Unsupported{};
-            phi.push_back(arg(d));
-        }
+        for (cplx d : op.values) phi.push_back(arg(d));
         phases(op.qubits, phi);
     }
 
@@ -394,6 +407,9 @@ struct Span {
 
 constexpr ld kMaxOwed = 200.0L;  // rotations may leave amplitudes e^200 too large before a table
 constexpr int kWindow = 128;  // items a phase chooses among
+// Below this many qubits half of them: planning then takes a third less time,
+// where it is most of a call, for at most 3 % longer programs (either way).
+constexpr int kWideQubits = 20;
 struct Bits {
     uint64_t w[2] = {0, 0};
     void set(int i) { w[i >> 6] |= uint64_t(1) << (i & 63); }
@@ -409,33 +425,47 @@ uint4 word(double a, double b) {
     return u;
 }
 
-// S e^{ia} as doubles.  Entries recur (a CZ's are e^{+-i pi/4}), so the rounding
+// A factor as doubles.  Entries recur (a CZ's are e^{+-i pi/4}), so the rounding
 // of their modulus would add up: of the nearest pairs the one closest in modulus.
 // `off` gains the logarithm of the modulus, and the angle, by which it misses.
-uint4 factor_word(ld S, ld a, ld off[2]) {
-    const ld re = S * std::cos(a), im = S * std::sin(a);
+struct Factor {
+    ld re = 1.0L, im = 0.0L;
+    void times(const Factor& f) {
+        const ld r = re * f.re - im * f.im;
+        im = re * f.im + im * f.re;
+        re = r;
+    }
+};
+
+Factor factor(ld b, ld a) {
+    const ld g = b == 0.0L ? 1.0L : std::exp(b);
+    return a == 0.0L ? Factor{g, 0.0L} : Factor{g * std::cos(a), g * std::sin(a)};
+}
+
+uint4 factor_word(const Factor& f, ld off[2]) {
+    const ld re = f.re, im = f.im, S2 = re * re + im * im;
     const double x = double(re), y = double(im);
     double best[2] = {x, y};
-    ld miss = std::fabs(ld(x) * x + ld(y) * y - S * S);
+    ld miss = std::fabs(ld(x) * x + ld(y) * y - S2);
     const double tries[4][2] = {{std::nextafter(x, 4.0 * x), y}, {std::nextafter(x, 0.0), y},
                                 {x, std::nextafter(y, 4.0 * y)}, {x, std::nextafter(y, 0.0)}};
     for (const auto& t : tries) {
-        const ld m = std::fabs(ld(t[0]) * t[0] + ld(t[1]) * t[1] - S * S);
+        const ld m = std::fabs(ld(t[0]) * t[0] + ld(t[1]) * t[1] - S2);
         if (m < miss) {
             miss = m;
             best[0] = t[0];
             best[1] = t[1];
         }
     }
-    off[0] += ((best[0] - re) * re + (best[1] - im) * im) / (S * S);
-    off[1] += ((best[1] - im) * re - (best[0] - re) * im) / (S * S);
+    off[0] += ((best[0] - re) * re + (best[1] - im) * im) / S2;
+    off[1] += ((best[1] - im) * re - (best[0] - re) * im) / S2;
     return word(best[0], best[1]);
 }
 
 class Scheduler {
   public:
-    Scheduler(std::vector<Item> items, int m, Lowering& lw, RotProgram& out)
-        : items_(std::move(items)), m_(m), lw_(lw), out_(out) {}
+    Scheduler(std::vector<Item> items, int m, int n, Lowering& lw, RotProgram& out)
+        : items_(std::move(items)), m_(m), window_(n < kWideQubits ? kWindow / 2 : kWindow), lw_(lw), out_(out) {}
 
     void run() {
         for (size_t i = 0; i < items_.size(); i++)
@@ -473,7 +503,7 @@ class Scheduler {
 
   private:
     std::vector<Item> items_;
-    int m_;
+    int m_, window_;
     Lowering& lw_;
     RotProgram& out_;
     std::vector<int> active_;  // items not applied yet, in order
@@ -513,67 +543,69 @@ class Scheduler {
     }
 
     void one_phase(uint4 head[3]) {
-        const int W = int(std::min<size_t>(active_.size(), size_t(kWindow)));
+        const int W = int(std::min<size_t>(active_.size(), size_t(window_)));
         std::vector<const Item*> it(static_cast<size_t>(W));
         for (int i = 0; i < W; i++) it[size_t(i)] = &items_[size_t(active_[size_t(i)])];
         // Earlier items an item does not commute with (phases have no direction).
         Bits pred[kWindow];
         uint32_t dir[kWindow];
         {
-            uint64_t mask[kWindow];
+            uint32_t mask[kWindow];  // directions are tile-local
             for (int j = 0; j < W; j++) {
                 dir[j] = it[size_t(j)]->v;
-                mask[j] = it[size_t(j)]->mask;
+                mask[j] = uint32_t(it[size_t(j)]->mask);
                 for (int i = 0; i < j; i++)
-                    pred[j].w[i >> 6] |= uint64_t(parity64((mask[i] & dir[j]) ^ (mask[j] & dir[i]))) << (i & 63);
+                    pred[j].w[i >> 6] |= uint64_t(__builtin_parity((mask[i] & dir[j]) ^ (mask[j] & dir[i]))) << (i & 63);
             }
         }
-        auto closure = [&](const Span& V, Bits& exec) {
+        // Directions modulo V: a rotation can run when its own is 0, or the one
+        // direction `more` that V is tried with.
+        Span V;
+        uint32_t red[kWindow];
+        auto reduce = [&] {
+            for (int i = 0; i < W; i++) red[i] = dir[i] ? V.reduce(dir[i]) : 0;
+        };
+        auto closure = [&](uint32_t more, Bits& exec) {
             int rots = 0;
             exec = Bits{};
             for (int i = 0; i < W; i++) {
-                if (!pred[i].within(exec)) continue;
-                if (dir[i]) {
-                    if (V.reduce(dir[i])) continue;
-                    rots++;
-                }
+                if ((red[i] && red[i] != more) || !pred[i].within(exec)) continue;
+                rots += dir[i] ? 1 : 0;
                 exec.set(i);
             }
             return rots;
         };
         // Directions one at a time: the one that lets the most rotations in,
         // among those of the first rotations that only lack their direction.
-        Span V;
         Bits exec;
-        closure(V, exec);
+        reduce();
+        closure(0, exec);
         while (V.dim < kRotRegBits) {
-            std::vector<uint32_t> cand;
-            for (int i = 0; i < W && cand.size() < 8; i++) {
-                const Item& x = *it[size_t(i)];
-                if (!x.rot || exec.get(i) || !pred[i].within(exec)) continue;
-                const uint32_t v = V.reduce(x.v);
-                if (v && std::find(cand.begin(), cand.end(), v) == cand.end()) cand.push_back(v);
-            }
-            if (cand.empty()) break;
+            uint32_t cand[8];
+            int count = 0;
+            for (int i = 0; i < W && count < 8; i++)
+                if (red[i] && !exec.get(i) && pred[i].within(exec) && std::find(cand, cand + count, red[i]) == cand + count)
+                    cand[count++] = red[i];
+            if (count == 0) break;
             int best = -1;
-            Span bestV;
+            uint32_t bestv = 0;
             Bits bestE;
-            for (uint32_t v : cand) {
-                Span T = V;
-                T.add(v);
+            for (int k = 0; k < count; k++) {
                 Bits e;
-                const int r = closure(T, e);
+                const int r = closure(cand[k], e);
                 if (r > best) {
                     best = r;
-                    bestV = T;
+                    bestv = cand[k];
                     bestE = e;
                 }
             }
-            V = bestV;
+            V.add(bestv);
             exec = bestE;
+            reduce();
         }
         for (int b = m_ - 1; b >= 0 && V.dim < kRotRegBits; b--) V.add(1u << b);
-        closure(V, exec);
+        reduce();
+        closure(0, exec);
         bool last = int(active_.size()) == W;
         for (int i = 0; i < W && last; i++)
             if (it[size_t(i)]->rot && !exec.get(i)) last = false;
@@ -709,22 +741,22 @@ class Scheduler {
             };
             std::vector<uint32_t> unit;
             for (int b = 0; b < m_; b++) unit.push_back(project(1u << b));
-            std::vector<uint32_t> pool = unit;
-            for (int i = 0; i < m_; i++)
-                for (int j = 0; j < i; j++) pool.push_back(unit[size_t(i)] ^ unit[size_t(j)]);
             uint32_t banks[3] = {}, nb = 0;
-            for (uint32_t p : pool) {
-                if (nb == 3 || int(U.size()) == m_ - kRotRegBits) break;
+            auto lane = [&](uint32_t p) {
+                if (nb == 3 || int(U.size()) == m_ - kRotRegBits) return;
                 uint32_t l = rot_swizzle(p) & 7u;
                 for (uint32_t i = 0; i < nb; i++)
                     if (l & (1u << (31 - __builtin_clz(banks[i])))) l ^= banks[i];
-                if (!p || !l || !independent(p, true)) continue;
+                if (!p || !l || !independent(p, true)) return;
                 const uint32_t top = 1u << (31 - __builtin_clz(l));
                 for (uint32_t i = 0; i < nb; i++)
                     if (banks[i] & top) banks[i] ^= l;
                 banks[nb++] = l;
                 U.push_back(p);
-            }
+            };
+            for (uint32_t p : unit) lane(p);
+            for (int i = 0; i < m_ && nb < 3; i++)
+                for (int j = 0; j < i; j++) lane(unit[size_t(i)] ^ unit[size_t(j)]);
             for (uint32_t p : unit)
                 if (int(U.size()) < m_ - kRotRegBits && p && independent(p, true)) U.push_back(p);
         }
@@ -738,31 +770,37 @@ class Scheduler {
             for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) s |= uint32_t(__builtin_parity(r & v)) << v;
             return s;
         };
+        uint32_t combined[kRotEntries] = {};  // the places of the register entries
+        for (uint32_t d = 1; d < uint32_t(kRotEntries); d++)
+            combined[d] = combined[d & (d - 1)] ^ basis[__builtin_ctz(d)];
         auto direction = [&](uint32_t v) {  // v on the basis
-            uint32_t d = 0, best = 0;
-            for (d = 1; d < uint32_t(kRotEntries); d++) {
-                uint32_t x = 0;
-                for (int j = 0; j < kRotRegBits; j++)
-                    if ((d >> j) & 1) x ^= basis[j];
-                if (x == v) best = d;
-            }
-            return best;
+            uint32_t d = 1;
+            while (d < uint32_t(kRotEntries) && combined[d] != v) d++;
+            return d & uint32_t(kRotEntries - 1);
         };
 
         // Emission.  pend[j]: logarithm of the factor still owed by the entries
         // with register bit j clear (the others owe its negative).
         ld pend[kRotRegBits] = {};
-        auto emit_table = [&](const ld A[kRotEntries], ld B[kRotEntries], ld G) {
+        // A table: the phases `f` (none needs a slot parity), what the entries and
+        // the state are owed, and the angle G.
+        auto emit_table = [&](const std::vector<int>& f, ld G) {
             Part part;
             part.place = 5;
             part.data = uint32_t(tables_.size());
             parts_.push_back(part);
+            Factor T[kRotEntries];
+            T[0] = factor(uniform_, std::remainder(G, 2 * kPiL));
+            for (int v = 1; v < kRotEntries; v++) T[v] = T[0];
+            auto spread = [&](uint32_t r, ld b, ld a) {  // e^{b + ia}, inverted by the parity of r
+                const Factor plus = factor(b, a), minus = b == 0.0L ? Factor{plus.re, -plus.im} : factor(-b, -a);
+                for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) T[v].times(__builtin_parity(r & v) ? minus : plus);
+            };
+            for (int j = 0; j < kRotRegBits; j++)
+                if (pend[j] != 0.0L) spread(1u << j, pend[j], 0.0L);
+            for (int i : f) spread(on_V(it[size_t(i)]->mask), it[size_t(i)]->b, it[size_t(i)]->a);
             ld off[2] = {};
-            for (int v = 0; v < kRotEntries; v++) {
-                B[v] += uniform_;
-                for (int j = 0; j < kRotRegBits; j++) B[v] += (v >> j) & 1 ? -pend[j] : pend[j];
-                tables_.push_back(factor_word(std::exp(B[v]), std::remainder(A[v] + G, 2 * kPiL), off));
-            }
+            for (const Factor& t : T) tables_.push_back(factor_word(t, off));
             for (ld& p : pend) p = 0.0;
             // What the table misses on average is owed to the next ones.
             uniform_ = -off[0] / kRotEntries;
@@ -811,7 +849,7 @@ class Scheduler {
                         done.set(i);
                     }
             std::vector<std::pair<uint32_t, std::vector<int>>> by;  // register parity -> phases
-            ld A[kRotEntries] = {}, B[kRotEntries] = {};
+            std::vector<int> here;  // of the table
             bool table = false;
             for (int i : f) {
                 const Item& x = *it[size_t(i)];
@@ -820,11 +858,7 @@ class Scheduler {
                 const uint32_t r = on_V(x.mask);
                 if (slots(x.mask) == 0) {
                     table = true;
-                    for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) {
-                        const bool neg = __builtin_parity(r & v);
-                        A[v] += neg ? -x.a : x.a;
-                        B[v] += neg ? -x.b : x.b;
-                    }
+                    here.push_back(i);
                     continue;
                 }
                 auto b = std::find_if(by.begin(), by.end(), [&](auto& e) { return e.first == r; });
@@ -842,7 +876,7 @@ class Scheduler {
                 for (ld p : pend) table = table || p != 0.0;
                 table = table || uniform_ != 0.0;
             }
-            if (table) emit_table(A, B, G);
+            if (table) emit_table(here, G);
             for (auto& b : by) {
                 const std::vector<int>& terms = b.second;
                 auto part_of = [&](uint32_t kind, const std::vector<int>& t) {
@@ -867,7 +901,7 @@ class Scheduler {
                 if (!angles.empty()) {
                     part_of(kRotSlots, angles);
                     ld off[2] = {};
-                    for (int i : angles) tables_.push_back(factor_word(1.0L, it[size_t(i)]->a, off));
+                    for (int i : angles) tables_.push_back(factor_word(factor(0.0L, it[size_t(i)]->a), off));
                     uniform_ -= off[0];
                     out_.slot_phases++;
                     fma_ += 6.0 + 6.0 * double(angles.size()) / kRotEntries;
@@ -937,8 +971,7 @@ class Scheduler {
                 } else {
                     for (int j = 0; j < kRotRegBits; j++)
                         if (((d >> j) & 1) && pend[j] != 0.0) {
-                            ld A[kRotEntries] = {}, B[kRotEntries] = {};
-                            emit_table(A, B, 0.0);
+                            emit_table({}, 0.0);
                             break;
                         }
                     pend[low] -= lost;
@@ -952,8 +985,7 @@ class Scheduler {
         }
         if (last || !tail.empty()) emit_flush(tail, last);
         if (!last && uniform_ < -kMaxOwed) {  // a circuit without phases: keep the amplitudes in range
-            ld A[kRotEntries] = {}, B[kRotEntries] = {};
-            emit_table(A, B, 0.0);
+            emit_table({}, 0.0);
         }
         // Factors still owed become phases of the register bits' parities (the
         // coordinate functionals), for later phases of the pass.
@@ -1002,6 +1034,13 @@ namespace {
 
 // Whether an operation has a rotation form.
 bool rotation_form(const Operation& op) {
+    switch (op.type) {
+        case Operation::One: return op.controls.size() < size_t(kMaxDiagQubits) && unitary(op.m);
+        case Operation::X: return op.controls.size() < size_t(kMaxDiagQubits);
+        case Operation::Swap: return op.controls.size() + 1 < size_t(kMaxDiagQubits);
+        case Operation::Diagonal: return op.qubits.size() <= size_t(kMaxDiagQubits) && unit_moduli(op.values);
+        default: break;
+    }
     std::vector<uint64_t> q = op.touched();
     std::sort(q.begin(), q.end());
     auto local = [&](uint64_t x) { return uint64_t(std::lower_bound(q.begin(), q.end(), x) - q.begin()); };
@@ -1044,7 +1083,7 @@ bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<in
     }
     out = RotProgram{};
     out.m = m;
-    Scheduler s(lw.items, m, lw, out);
+    Scheduler s(lw.items, m, n, lw, out);
     s.run();
     // Place of tile index e: sum over q of (e_q ^ const_q ^ outer part) v_q.
     uint32_t c = 0;

@@ -101,11 +101,21 @@ void probs_to(const k::Batch& b, const std::vector<uint64_t>& qubits, double* ou
     }
 }
 
+// What build_sums leaves on the device for the sampler and the host: the total
+// (the last entry of the full running sums) and whether it can be sampled from.
+struct SumTotal {
+    double total;
+    int bad;  // not finite and positive
+    int pad;
+};
+constexpr size_t kTotalBytes = sizeof(SumTotal);
+
 // Two-level running sums of state 0's probabilities over `qubits` on the
 // device (sums within 2048-entry tiles in cdf, inclusive sums of whole tiles in
-// tmp; the full register in descending order reads the state directly);
-// returns the total, the last entry of the full running sums.
-double build_sums(const k::Batch& b, const std::vector<uint64_t>& qubits, double* cdf, uint64_t len, DevMem& tmp) {
+// tmp; the full register in descending order reads the state directly), and
+// their total in `total`.  Nothing waits: the sampler reads the total there.
+void build_sums(const k::Batch& b, const std::vector<uint64_t>& qubits, double* cdf, uint64_t len, DevMem& tmp,
+                SumTotal* total) {
     cudaStream_t s = b.stream;
     tmp.ensure_on(k::scan_tmp_size(len) * 8, s, "scan scratch");
     if (is_full_descending(qubits, uint64_t(b.n))) {
@@ -114,12 +124,8 @@ double build_sums(const k::Batch& b, const std::vector<uint64_t>& qubits, double
         probs_to(b, qubits, cdf);
         k::scan_local(s, cdf, len, tmp.as<double>());
     }
-    double last = 0, offset = 0;
-    const uint64_t t = k::scan_tile_of(len - 1);
-    cuda_check(cudaMemcpyAsync(&last, cdf + (len - 1), 8, cudaMemcpyDeviceToHost, s), "read total");
-    if (t > 0) cuda_check(cudaMemcpyAsync(&offset, tmp.as<double>() + (t - 1), 8, cudaMemcpyDeviceToHost, s), "read total");
-    cuda_check(cudaStreamSynchronize(s), "stream synchronize");
-    return t > 0 ? last + offset : last;
+    cuda_check(cudaMemsetAsync(total, 0, kTotalBytes, s), "clear total");
+    k::take_total(s, cdf, len, tmp.as<double>(), &total->total, &total->bad);
 }
 
 std::string json_double(double v) {
@@ -283,7 +289,6 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
             std::lock_guard<std::mutex> lk(dev_->mu);
             dev_->activate();
             cudaStream_t s = dev_->stream;
-            uint64_t kept_seed = seed;
             clk::time_point mark = clk::now();
             auto phase = [&](int i) {
                 const clk::time_point now = clk::now();
@@ -297,7 +302,8 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
                 if (!st.amps.p || st.n != int(n) || st.W != 1 || st.ncb != ncb || st.c64 != c64)
                     st.allocate(int(n), 1, ncb, c64, s);
                 k::Batch b = st.view(s, 1);
-                reset_bookkeeping(st, 1, {kept_seed}, s);
+                // A unitary prefix reads no classical bits and draws nothing.
+                cuda_check(cudaMemsetAsync(st.err.p, 0, 16, s), "clear error flag");
                 phase(kPhState);
                 DevMem& cdf = ws_->table;
                 DevMem& tmp = ws_->scratch;
@@ -306,7 +312,9 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
                 if (cdf.bytes != clen * 8) cdf.alloc_on(clen * 8, s, "the sampling table");
                 const uint64_t tmp_bytes = std::max<uint64_t>(k::scan_tmp_size(clen) * 8, 16);
                 if (tmp.bytes != tmp_bytes) tmp.alloc_on(tmp_bytes, s, "scan scratch");
-                if (idx.bytes != shots * 8) idx.alloc_on(shots * 8, s, "sampled outcomes");
+                // The outcomes, and behind them the total: one copy brings both.
+                if (idx.bytes != shots * 8 + kTotalBytes) idx.alloc_on(shots * 8 + kTotalBytes, s, "sampled outcomes");
+                SumTotal* total_dev = reinterpret_cast<SumTotal*>(idx.as<uint64_t>() + shots);
                 phase(kPhTable);
                 // The prefix's executor: kept with the circuit's cached plan (the
                 // device lock above serialises its use), or built for this call.
@@ -334,17 +342,22 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
                 ex->run(b, nullptr, nullptr, /*normalize=*/false, /*from_basis=*/built);  // the sampler divides by the total
                 cuda_check(cudaEventRecord(ev[1], s), "cudaEventRecord");
                 phase(kPhRun);
-                double total = build_sums(b, qubits, cdf.as<double>(), clen, tmp);
-                if (!std::isfinite(total) || total <= 0.0) fail(kMemoryError, "Invalid state normalization when sampling");
+                build_sums(b, qubits, cdf.as<double>(), clen, tmp, total_dev);
+                k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), clen, &total_dev->total, 0.0, false, seed, shots,
+                               true, idx.as<uint64_t>());
+                cuda_check(cudaEventSynchronize(ev[1]), "cudaEventSynchronize");
                 phase(kPhSums);
+                std::vector<uint64_t> h(shots + kTotalBytes / 8);
+                cuda_check(cudaMemcpyAsync(h.data(), idx.p, shots * 8 + kTotalBytes, cudaMemcpyDeviceToHost, s),
+                           "read samples");
+                cuda_check(cudaStreamSynchronize(s), "stream synchronize");
+                SumTotal total;
+                std::memcpy(&total, h.data() + shots, kTotalBytes);
+                h.resize(shots);
+                if (total.bad) fail(kMemoryError, "Invalid state normalization when sampling");
                 float prefix_ms = 0.f;
                 if (cudaEventElapsedTime(&prefix_ms, ev[0], ev[1]) == cudaSuccess)
                     set_phase(kPhPrefixDevice, double(prefix_ms) * 1e-3);
-                k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), clen, nullptr, total, false, seed, shots, true,
-                               idx.as<uint64_t>());
-                std::vector<uint64_t> h(shots);
-                cuda_check(cudaMemcpyAsync(h.data(), idx.p, shots * 8, cudaMemcpyDeviceToHost, s), "read samples");
-                cuda_check(cudaStreamSynchronize(s), "stream synchronize");
                 phase(kPhSample);
                 sort_outcomes(h);
                 if (ncb <= 64) {
@@ -568,15 +581,19 @@ std::unordered_map<uint64_t, uint64_t> Result::counts(uint64_t shots, const std:
     const uint64_t m = uint64_t(1) << qubits.size();
     DevMem cdf, tmp, idx;
     cdf.alloc_on(m * 8, s, "the sampling table");
+    idx.alloc_on(shots * 8 + kTotalBytes, s, "sampled outcomes");
+    SumTotal* total_dev = reinterpret_cast<SumTotal*>(idx.as<uint64_t>() + shots);
     k::Batch b = state.view(s, 1);
-    double total = build_sums(b, qubits, cdf.as<double>(), m, tmp);
-    if (!std::isfinite(total) || total <= 0.0) fail(kRuntimeError, "Cannot sample a state with nonfinite or zero norm");
-    idx.alloc_on(shots * 8, s, "sampled outcomes");
-    k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), m, nullptr, total, true, seed, shots, false,
+    build_sums(b, qubits, cdf.as<double>(), m, tmp, total_dev);
+    k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), m, &total_dev->total, 0.0, true, seed, shots, false,
                    idx.as<uint64_t>());
-    std::vector<uint64_t> h(shots);
-    cuda_check(cudaMemcpyAsync(h.data(), idx.p, shots * 8, cudaMemcpyDeviceToHost, s), "read samples");
+    std::vector<uint64_t> h(shots + kTotalBytes / 8);
+    cuda_check(cudaMemcpyAsync(h.data(), idx.p, shots * 8 + kTotalBytes, cudaMemcpyDeviceToHost, s), "read samples");
     dev->sync();
+    SumTotal total;
+    std::memcpy(&total, h.data() + shots, kTotalBytes);
+    h.resize(shots);
+    if (total.bad) fail(kRuntimeError, "Cannot sample a state with nonfinite or zero norm");
     for (uint64_t v : h) res[v]++;
     return res;
 }
