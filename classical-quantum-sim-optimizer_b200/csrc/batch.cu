@@ -13,8 +13,20 @@ namespace dq {
 namespace {
 
 constexpr int kBatchThreads = 256;
-// Side streams the fused circuits of a batch run on.
-constexpr size_t kSideStreams = 16;
+constexpr size_t kMaxTileBytes = size_t(1) << 17;  // 14 tile qubits of complex64, 13 of complex128
+// Side streams the fused circuits spread over.  A circuit's passes follow one
+// another, so with 16 streams a batch of 64 waited on four circuits in a row
+// (64 circuits of 12-20 qubits 1.19 ms, of 12-15 qubits 0.44 ms; with 64 streams
+// 0.97 and 0.21 ms; 256 circuits of 12-22 qubits 11.7 and 11.5 ms).
+constexpr size_t kSideStreams = 64;
+// Tile groups a CTA of a fused pass takes at least, for circuits of at least
+// kShareQuads groups in a batch of at least kFullQuads: there the passes of
+// other circuits fill the device and a CTA's set-up is worth sharing (256
+// circuits of 12-22 qubits 11.5 ms at 1, 10.6 at 3, 10.9 at 4); where they do
+// not, fewer CTAs only take longer (12 circuits of 12-20 qubits 0.31 ms at 1,
+// 0.60 at 3).
+constexpr int kShare = 3;
+constexpr uint64_t kShareQuads = 32, kFullQuads = 148 * 8;
 // Spin limit of one dependency wait: 2^24 polls of >= 256 ns, several seconds.
 constexpr uint64_t kMaxSpins = uint64_t(1) << 24;
 
@@ -348,7 +360,8 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
         // Sampling runs over the full register; measured qubits are read from the sampled index.
         for (auto& kv : mapping) c.cbit_map.emplace_back(kv.first, kv.second);
         c.tile_m = tuning.tile_m > 0 ? tuning.tile_m : (c64_ ? 13 : 12);
-        c.fuse = tuning.fuse > 0 ? tuning.fuse : 2;
+        // Unless a shape is asked for, complex128 circuits run rotation passes.
+        c.fuse = tuning.fuse > 0 ? tuning.fuse : !c64_ && tuning.tile_m <= 0 && tuning.depth == 0 ? kTuneRotations : 2;
         c.depth = tuning.depth;
         auto tuned = tuning.per_n.find(c.n);
         if (tuning.tile_m <= 0 && tuning.fuse <= 0 && tuned != tuning.per_n.end()) {
@@ -356,6 +369,7 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
             c.fuse = tuned->second.fuse;
             c.depth = tuned->second.depth;
         }
+        if (c.fuse == 5 && !c64_) c.fuse = kTuneRotations;
         std::vector<TilePass> passes;
         if (c.fuse == 5 && c64_ && c.n >= uint64_t(kFusedM)) {
             // Tensor-core fused passes, run by an executor of their own on a side stream.
@@ -365,8 +379,16 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
             cfg.c64 = true;
             cfg.n = int(c.n);
             c.fused = std::make_unique<Executor>(ops, 0, prefix, cfg);
+        } else if (c.fuse == kTuneRotations && !c64_ && c.n >= uint64_t(kRotMinTile)) {
+            // Rotation passes, run the same way.
+            ExecConfig cfg;
+            cfg.tiled = true;
+            cfg.rotations = true;
+            cfg.n = int(c.n);
+            c.fused = std::make_unique<Executor>(ops, 0, prefix, cfg);
         } else {
-            if (c.fuse == 5) c.fuse = 2;  // no tensor-core form below 12 qubits or in complex128
+            // No tensor-core form below 12 qubits or in complex128, no rotation form in complex64.
+            if (c.fuse == 5 || c.fuse == kTuneRotations) c.fuse = 2;
             TilePlanOptions po;
             po.m = c.tile_m;
             po.fuse = std::min(c.fuse, kTileMaxDense);
@@ -464,7 +486,8 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
     for (size_t ci = 0; ci < circuits_.size(); ci++)
         if (circuits_[ci].fused) order.push_back(ci);
     auto cost = [&](size_t ci) {
-        return double(uint64_t(1) << circuits_[ci].n) * double(circuits_[ci].fused->fused_blocks() + 3);
+        const Executor& ex = *circuits_[ci].fused;
+        return double(uint64_t(1) << circuits_[ci].n) * double((c64_ ? ex.fused_blocks() : ex.tile_ops()) + 3);
     };
     std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return cost(a) > cost(b); });
     if (!order.empty()) {
@@ -482,19 +505,25 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
             cuda_check(cudaEventCreateWithFlags(&join_[j], cudaEventDisableTiming), "cudaEventCreate");
         }
         cuda_check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
+        for (size_t ci : order) {
+            const uint64_t n = circuits_[ci].n;
+            fused_quads_ += n > uint64_t(kFusedM) ? uint64_t(1) << (n - kFusedM) >> 2 : 1;
+        }
         for (size_t ci : order) circuits_[ci].fused->prepare(circuit_view(circuits_[ci], s));
     }
-    const size_t smem = (S << max_m_);
+    // The largest tile's shared memory, whatever this batch needs: the limit
+    // belongs to the kernel, which batches of other shapes also launch.
     // Largest carveout: the occupancy query that sizes the persistent grid must
     // match what the launch gets, since every CTA has to be resident at once.
+    const int most = int(kMaxTileBytes);
     if (c64_) {
-        cuda_check(cudaFuncSetAttribute(k_batch<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
+        cuda_check(cudaFuncSetAttribute(k_batch<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most),
                    "smem attribute");
         cuda_check(cudaFuncSetAttribute(k_batch<float2>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         int(cudaSharedmemCarveoutMaxShared)),
                    "carveout attribute");
     } else {
-        cuda_check(cudaFuncSetAttribute(k_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
+        cuda_check(cudaFuncSetAttribute(k_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most),
                    "smem attribute");
         cuda_check(cudaFuncSetAttribute(k_batch<double2>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         int(cudaSharedmemCarveoutMaxShared)),
@@ -524,6 +553,8 @@ k::Batch BatchRun::circuit_view(const Circ& c, cudaStream_t s) const {
     b.n = int(c.n);
     b.W = 1;
     b.err = err_.as<int>();
+    const uint64_t quads = c.n > uint64_t(kFusedM) ? uint64_t(1) << (c.n - kFusedM) >> 2 : 1;
+    if (fused_quads_ >= kFullQuads && quads >= kShareQuads) b.fused_quads = kShare;
     return b;
 }
 
@@ -536,7 +567,7 @@ size_t BatchRun::passes() const {
 
 size_t BatchRun::fused_circuits() const {
     size_t total = 0;
-    for (const Circ& c : circuits_) total += c.fused ? 1 : 0;
+    for (const Circ& c : circuits_) total += c.fused && c64_ ? 1 : 0;
     return total;
 }
 
@@ -569,7 +600,7 @@ void BatchRun::work(double* bytes, double* tensor_flops, double* cuda_core_flops
         c.fused->arith_flops(b, &cc, &tc);
         cf += cc;
         tf += tc;
-        by += double(c.fused->passes()) * 2.0 * 8.0 * double(uint64_t(1) << c.n);
+        by += double(c.fused->passes()) * 2.0 * (c64_ ? 8.0 : 16.0) * double(uint64_t(1) << c.n);
     }
     *bytes = by;
     *tensor_flops = tf;
@@ -763,10 +794,14 @@ TuneResult autotune_tile(Simulator& sim, const std::string& json, bool c64) {
         const double ms = time_shape(best.tile_m, best.fuse, depth);
         if (ms < best.ms) best = {best.tile_m, best.fuse, depth, ms};
     }
-    // ... and the tensor-core fused passes (complex64, 12 qubits or more).
+    // ... and the tensor-core fused passes (complex64, 12 qubits or more) or the
+    // rotation passes (complex128).
     if (c64 && n >= uint64_t(kFusedM)) {
         const double ms = time_shape(kFusedM, 5, 0);
         if (ms < best.ms) best = {kFusedM, 5, 0, ms};
+    } else if (!c64 && n >= uint64_t(kRotMinTile)) {
+        const double ms = time_shape(12, kTuneRotations, 0);
+        if (ms < best.ms) best = {12, kTuneRotations, 0, ms};
     }
     std::lock_guard<std::mutex> lk(mu);
     cache[{n, c64 ? 1 : 0}] = best;

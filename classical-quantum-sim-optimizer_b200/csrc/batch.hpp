@@ -25,9 +25,11 @@
 namespace dq {
 
 // How the circuits of one qubit count run.  fuse 5 (complex64, >= 12 qubits):
-// tensor-core fused passes; otherwise CUDA-core tile passes of tile_m qubits
+// tensor-core fused passes; kTuneRotations (complex128, >= 5 qubits): rotation
+// passes; otherwise CUDA-core tile passes of tile_m qubits
 // with operations fused to `fuse` qubits and at most `depth` operations per
 // shared-memory pass (0: no limit).
+constexpr int kTuneRotations = 6;
 struct BatchShape {
     int tile_m = 0, fuse = 0, depth = 0;
 };
@@ -78,7 +80,7 @@ class BatchRun {
         std::vector<uint64_t> sample_qubits;                  // descending
         bool full_register = true;
         int tile_m = 12, fuse = 2, depth = 0;
-        std::unique_ptr<Executor> fused;  // tensor-core passes on a side stream
+        std::unique_ptr<Executor> fused;  // tensor-core or rotation passes on a side stream
         int stream = 0;                   // its side stream
     };
     std::shared_ptr<Device> dev_;
@@ -88,7 +90,7 @@ class BatchRun {
     std::vector<PassRec> pass_recs_;
     std::vector<TileOp> ops_host_;
     std::vector<double2> pool_host_;
-    uint64_t total_items_ = 0, total_amps_ = 0, zz_parts_ = 0;
+    uint64_t total_items_ = 0, total_amps_ = 0, zz_parts_ = 0, fused_quads_ = 0;
     int max_m_ = 0;
     DevMem amps_, recs_, ops_, pool_, done_, head_, err_, probs_, tmp_, circ_off_, circ_of_tile_, samples_, zz_part_,
         zz_at_, zz_sums_, seeds_;

@@ -825,7 +825,8 @@ void fused_pass(const Batch& b, const FusedPass& p, const FusedBlock* blocks_dev
     fused_configure();
     // One CTA per SM, persistent over groups of kGroups tiles.
     const uint64_t total = b.W << (b.n - kFusedM);
-    const uint64_t grid = std::min<uint64_t>((total + kGroups - 1) / kGroups, uint64_t(sm_count()));
+    const uint64_t quads = (total + kGroups - 1) / kGroups, each = uint64_t(std::max(1, b.fused_quads));
+    const uint64_t grid = std::min<uint64_t>((quads + each - 1) / each, uint64_t(sm_count()));
     k_fused<<<unsigned(grid), kThreads, kSmemBytes, b.stream>>>(static_cast<float2*>(b.amps), b.n, fq, tile_map,
                                                                blocks_dev + p.first_block, p.nblocks, upool_dev, total,
                                                                err, in_norm, fused_norm_parts(b.n), tile_norm);

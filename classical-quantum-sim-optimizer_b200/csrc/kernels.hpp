@@ -32,6 +32,10 @@ struct Batch {
     double* scale = nullptr;       // 1/sqrt(p) of the last outcome
     double* partial = nullptr;     // W * kMaxChunks * 2 branch sums
     int* err = nullptr;            // set to 1 on a nonfinite or zero norm
+    // Fused passes: tile groups a CTA takes at least.  1 spreads a pass over the
+    // device; more where passes of other states fill it (a CTA's set-up is then
+    // shared).
+    int fused_quads = 1;
 };
 
 constexpr int kMaxChunks = 1024;
