@@ -211,7 +211,53 @@ __device__ __forceinline__ uint32_t swz(uint32_t e) {
     return e ^ (f & 7u);
 }
 
-// Persistent over tiles.  A CTA holds `1 << pack` tiles of 2^m amplitudes at
+// One phase of a tile: this thread's 16 amplitudes through the steps.
+template <class W>
+__device__ __forceinline__ void rotation_phase(double2* tile, const W& words, int ph, uint32_t slot, uint32_t index) {
+                const uint4 h0 = words(3 * ph), h1 = words(3 * ph + 1), h2 = words(3 * ph + 2);
+                const uint32_t ub[9] = {h1.x & 0xFFFFu, h1.x >> 16, h1.y & 0xFFFFu, h1.y >> 16, h1.z & 0xFFFFu,
+                                        h1.z >> 16,     h1.w & 0xFFFFu, h1.w >> 16, h2.x & 0xFFFFu};
+                uint32_t place = 0;
+    #pragma unroll
+                for (int b = 0; b < 9; b++) place ^= (slot >> b) & 1u ? ub[b] : 0u;
+                const uint32_t vb[4] = {h0.z & 0xFFFFu, h0.z >> 16, h0.w & 0xFFFFu, h0.w >> 16};
+                uint32_t vv[E];
+    #pragma unroll
+                for (int v = 0; v < E; v++)
+                    vv[v] = (v & 1 ? vb[0] : 0u) ^ (v & 2 ? vb[1] : 0u) ^ (v & 4 ? vb[2] : 0u) ^ (v & 8 ? vb[3] : 0u);
+                double2 a[E];
+    #pragma unroll
+                for (int v = 0; v < E; v++) a[v] = tile[place ^ vv[v]];
+                RotStream<W> rots(words, h2.y, index);
+                uint4 next = words(h0.x);
+                for (uint32_t o = 1; o <= h0.y; o++) {
+                    const uint4 st = next;
+                    next = words(h0.x + o);
+                    apply_step(a, words, st, index, rots);
+                }
+    #pragma unroll
+                for (int v = 0; v < E; v++) tile[place ^ vv[v]] = a[v];
+}
+
+// The last sweep: out of the frame, with its signs, to the state.
+__device__ __forceinline__ void store_tile(const double2* tile, double2* __restrict__ gp, const RotPass& p, int rest,
+                                           uint64_t outer, uint32_t slot, uint32_t place) {
+                uint32_t c = p.out_const ^ place;
+                uint32_t sg = uint32_t(p.sign_const) ^ odd(p.sign_outer & uint32_t(outer)) ^ odd(p.sign_local & slot);
+                if (p.outer_moves)
+                    for (int j = 0; j < rest; j++)
+                        if ((outer >> j) & 1) c ^= p.out_outer[j];
+    #pragma unroll
+                for (int k = 0; k < E; k++) {
+                    double2 x = tile[c ^ p.reg_out[k]];
+                    const int flip = int((sg ^ (uint32_t(p.reg_sign) >> k)) << 31);
+                    x.x = __hiloint2double(__double2hiint(x.x) ^ flip, __double2loint(x.x));
+                    x.y = __hiloint2double(__double2hiint(x.y) ^ flip, __double2loint(x.y));
+                    gp[p.reg_off[k]] = x;
+                }
+}
+
+// Few or small tiles.  Persistent; a CTA holds `1 << pack` tiles of 2^m amplitudes at
 // a time, 2^(m-4) threads each.
 template <class W>
 __device__ __forceinline__ void rotation_body(double2* __restrict__ s, int n, const RotPass& p, int pack,
@@ -263,46 +309,10 @@ __device__ __forceinline__ void rotation_body(double2* __restrict__ s, int n, co
         __syncthreads();
         const uint32_t index = slot | uint32_t(outer) << kRotSlotBits;
         for (int ph = 0; ph < p.nphases; ph++) {
-            const uint4 h0 = words(3 * ph), h1 = words(3 * ph + 1), h2 = words(3 * ph + 2);
-            const uint32_t ub[9] = {h1.x & 0xFFFFu, h1.x >> 16, h1.y & 0xFFFFu, h1.y >> 16, h1.z & 0xFFFFu,
-                                    h1.z >> 16,     h1.w & 0xFFFFu, h1.w >> 16, h2.x & 0xFFFFu};
-            uint32_t place = 0;
-#pragma unroll
-            for (int b = 0; b < 9; b++) place ^= (slot >> b) & 1u ? ub[b] : 0u;
-            const uint32_t vb[4] = {h0.z & 0xFFFFu, h0.z >> 16, h0.w & 0xFFFFu, h0.w >> 16};
-            uint32_t vv[E];
-#pragma unroll
-            for (int v = 0; v < E; v++)
-                vv[v] = (v & 1 ? vb[0] : 0u) ^ (v & 2 ? vb[1] : 0u) ^ (v & 4 ? vb[2] : 0u) ^ (v & 8 ? vb[3] : 0u);
-            double2 a[E];
-#pragma unroll
-            for (int v = 0; v < E; v++) a[v] = tile[place ^ vv[v]];
-            RotStream<W> rots(words, h2.y, index);
-            uint4 next = words(h0.x);
-            for (uint32_t o = 1; o <= h0.y; o++) {
-                const uint4 st = next;
-                next = words(h0.x + o);
-                apply_step(a, words, st, index, rots);
-            }
-#pragma unroll
-            for (int v = 0; v < E; v++) tile[place ^ vv[v]] = a[v];
+            rotation_phase(tile, words, ph, slot, index);
             __syncthreads();
         }
-        if (live) {
-            uint32_t c = p.out_const ^ slot_out[slot];
-            uint32_t sg = uint32_t(p.sign_const) ^ odd(p.sign_outer & uint32_t(outer)) ^ odd(p.sign_local & slot);
-            if (p.outer_moves)
-                for (int j = 0; j < rest; j++)
-                    if ((outer >> j) & 1) c ^= p.out_outer[j];
-#pragma unroll
-            for (int k = 0; k < E; k++) {
-                double2 x = tile[c ^ p.reg_out[k]];
-                const int flip = int((sg ^ (uint32_t(p.reg_sign) >> k)) << 31);
-                x.x = __hiloint2double(__double2hiint(x.x) ^ flip, __double2loint(x.x));
-                x.y = __hiloint2double(__double2hiint(x.y) ^ flip, __double2loint(x.y));
-                gp[p.reg_off[k]] = x;
-            }
-        }
+        if (live) store_tile(tile, gp, p, rest, outer, slot, slot_out[slot]);
         __syncthreads();
     }
 }
@@ -331,6 +341,137 @@ __global__ void __launch_bounds__(kRotThreads, 1)
     rotation_body(s, n, p, pack, total_tiles, basis, DevWords{w, w + p.data});
 }
 
+constexpr int kTeamTile = 12;      // qubits of a team's tile
+constexpr int kTeamThreads = 256;  // one thread per 16 amplitudes
+constexpr int kTeamBuffers = 3;
+// Tiles to an SM from which the teams are used.  With few, the rounds are what
+// counts and the teams start behind (one B200, 20 layers of brickwork: 512 tiles,
+// 3.5 to an SM, 0.738 ms against 0.755 in teams; 1,024 tiles 1.386 against 1.376).
+constexpr uint64_t kTeamTiles = 6;
+
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Two teams of 256 threads take a CTA's tiles in turn, from three buffers.
+// Tile j lies in buffer j % 3 and is worked on by team j % 2; the other team
+// fetches it, when it has stored tile j - 3, and says so (barrier 3 + j % 3)
+// while it works on tile j - 1, so that neither team waits for memory and each
+// starts its tile in the middle of the other's.  Two CTAs of one tile each left an SM
+// with half its warps while a tile was fetched: 27-qubit brickwork of 40 layers 97.0 -> 91.5 ms,
+// 25-qubit QFT 2.70 -> 2.60, 24-qubit ansatz of 8 layers 2.17 -> 2.05.  (With
+// an mbarrier for a tile's arrival the teams drift together: 97.0 ms.)
+template <class W>
+__device__ __forceinline__ void team_body(double2* __restrict__ s, int n, const RotPass& p, uint64_t total_tiles, int basis,
+                                          const W& words) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int m = kTeamTile;
+    double2* all = reinterpret_cast<double2*>(smem_raw);
+    uint64_t* slot_off = reinterpret_cast<uint64_t*>(all + (size_t(kTeamBuffers) << m));
+    uint16_t* slot_out = reinterpret_cast<uint16_t*>(slot_off + kTeamThreads);
+    uint16_t* outer_bit = slot_out + kTeamThreads;
+    const uint32_t slot = threadIdx.x & (kTeamThreads - 1);
+    // (the shuffle tells the compiler that a warp's threads agree; without it the
+    // program's words leave the uniform registers: 105 ms for the 91.5 above)
+    const int team = __shfl_sync(~0u, int(threadIdx.x / kTeamThreads), 0);
+    const int rest = n - m;
+    if (team == 0) {
+        uint64_t off = 0;
+        uint32_t pl = 0;
+        for (int b = 0; b < m - kRotRegBits; b++)
+            if ((slot >> b) & 1u) {
+                off |= uint64_t(1) << p.q[b];
+                pl ^= p.out_dir[b];
+            }
+        slot_off[slot] = off;
+        slot_out[slot] = uint16_t(pl);
+    } else if (slot < 32) {
+        int bit = int(slot);
+        for (int b = 0; b < m; b++) bit += int(p.q[b]) <= bit;
+        outer_bit[slot] = uint16_t(bit);
+    }
+    __syncthreads();  // (the steps' data too)
+    const int tiles = int((total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    auto outer_of = [&](int j) { return (blockIdx.x + uint64_t(j) * gridDim.x) & ((uint64_t(1) << rest) - 1); };
+    auto state_of = [&](int j) {
+        const uint64_t t = blockIdx.x + uint64_t(j) * gridDim.x;
+        const uint32_t lane = threadIdx.x & 31u;
+        const uint64_t mine = ((t >> lane) & 1u & uint32_t(int(lane) < rest)) << outer_bit[lane];
+        const uint64_t at = uint64_t(__reduce_or_sync(~0u, uint32_t(mine >> 32))) << 32 | __reduce_or_sync(~0u, uint32_t(mine));
+        return s + (((t >> rest) << n) | at | slot_off[slot]);
+    };
+    auto fetch = [&](int j, int buffer) {
+        double2* tile = all + (size_t(buffer) << m);
+        const uint32_t in_place = swz(slot);
+        const double2* gp = state_of(j);
+        const bool one = outer_of(j) == 0 && slot == 0;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            double2* to = &tile[in_place ^ p.reg_in[k]];
+            if (basis)
+                *to = make_double2(one && k == 0 ? 1.0 : 0.0, 0.0);
+            else
+                __pipeline_memcpy_async(to, gp + p.reg_off[k], sizeof(double2));
+        }
+        __pipeline_commit();
+    };
+    if (team < tiles) fetch(team, team);
+    if (team == 1 && tiles > 2) fetch(2, 2);
+    // Told after the second phase (the first of two): after the first, the teller
+    // waits for its own fetch (92.6 ms for the 91.5 above); in the middle, the
+    // other team waits for the teller (95.7).
+    const int tell = min(1, (p.nphases - 1) / 2);
+    int buffer = team;
+    // Both teams take the same number of turns (uniform control flow); the
+    // second's last one may be idle: its buffer's old tile, not stored.
+    for (int i = 0; i < (tiles + 1) / 2; i++) {
+        const int j = 2 * i + team;
+        if (i == 0) {
+            if (team == 1 && tiles > 2)
+                __pipeline_wait_prior(1);
+            else
+                __pipeline_wait_prior(0);
+            bar_sync(1 + team, kTeamThreads);
+        } else if (j < tiles) {
+            bar_sync(3 + buffer, 2 * kTeamThreads);
+        }
+        double2* tile = all + (size_t(buffer) << m);
+        const uint32_t index = slot | uint32_t(outer_of(j)) << kRotSlotBits;
+        for (int ph = 0; ph < p.nphases; ph++) {
+            rotation_phase(tile, words, ph, slot, index);
+            if (ph == tell && j >= 1 && j + 1 < tiles) {
+                __pipeline_wait_prior(0);
+                __threadfence_block();
+                bar_arrive(3 + (buffer == kTeamBuffers - 1 ? 0 : buffer + 1), 2 * kTeamThreads);
+            }
+            bar_sync(1 + team, kTeamThreads);
+        }
+        if (j < tiles) store_tile(tile, state_of(j), p, rest, outer_of(j), slot, slot_out[slot]);
+        if (j + 3 < tiles) {
+            bar_sync(1 + team, kTeamThreads);
+            fetch(j + 3, buffer);
+        }
+        buffer = buffer == 0 ? kTeamBuffers - 1 : buffer - 1;  // (j + 2) % 3
+    }
+}
+
+__host__ __device__ constexpr size_t team_tile_smem() {
+    return (sizeof(double2) * kTeamBuffers << kTeamTile) + kTeamThreads * (sizeof(uint64_t) + sizeof(uint16_t)) +
+           32 * sizeof(uint16_t);
+}
+
+__global__ void __launch_bounds__(2 * kTeamThreads, 1)
+    k_rotations_team(double2* __restrict__ s, int n, uint64_t total_tiles, int basis, const __grid_constant__ RotPass p,
+                     const __grid_constant__ RotWords w) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint4* table = reinterpret_cast<uint4*>(smem_raw + team_tile_smem());
+    for (int i = threadIdx.x; i < p.ndata; i += blockDim.x) table[i] = w.w[p.data + i];
+    team_body(s, n, p, total_tiles, basis, ArgWords{&w, table});
+}
+
 // CTAs of the kernel that are resident at once on the current device, asked of
 // the runtime when the shape differs from this thread's last launch.
 template <typename Kernel>
@@ -346,7 +487,10 @@ uint64_t resident_ctas(Kernel kernel, int threads, size_t smem) {
     cudaGetDevice(&dev);
     const void* id = reinterpret_cast<const void*>(kernel);
     if (last.kernel == id && last.dev == dev && last.threads == threads && last.smem >= smem) return last.ctas;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    // The limit is the device's, not this launch's: it holds for every thread's launches of the kernel.
+    int most = 0;
+    cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, int(cudaSharedmemCarveoutMaxShared));
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -397,9 +541,16 @@ void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const Ro
     if (as_argument) {
         static thread_local RotWords args;
         std::memcpy(args.w, r.words.data(), r.words.size() * sizeof(uint4));
-        k_rotations_arg<<<unsigned(std::min(ctas, resident_ctas(k_rotations_arg, threads, smem))), unsigned(threads), smem,
-                          b.stream>>>(
-            static_cast<double2*>(b.amps), b.n, pack, total, basis ? 1 : 0, p, args);
+        const size_t team_smem = team_tile_smem() + size_t(p.ndata) * sizeof(uint4);
+        const bool teams = r.m == kTeamTile && r.nphases > 0;
+        const uint64_t sms = teams ? resident_ctas(k_rotations_team, 2 * kTeamThreads, team_smem) : 0;
+        if (teams && total >= kTeamTiles * sms) {
+            k_rotations_team<<<unsigned(sms), 2 * kTeamThreads, team_smem, b.stream>>>(static_cast<double2*>(b.amps), b.n, total, basis ? 1 : 0, p, args);
+        } else {
+            k_rotations_arg<<<unsigned(std::min(ctas, resident_ctas(k_rotations_arg, threads, smem))), unsigned(threads), smem,
+                              b.stream>>>(
+                static_cast<double2*>(b.amps), b.n, pack, total, basis ? 1 : 0, p, args);
+        }
     } else {
         if (!words_dev) fail(kValueError, "rotation pass without its device words");
         k_rotations_dev<<<unsigned(std::min(ctas, resident_ctas(k_rotations_dev, threads, smem))), unsigned(threads), smem,

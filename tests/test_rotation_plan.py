@@ -204,3 +204,21 @@ def test_rotation_passes_in_trajectories(n):
     c = Circuit(n, ins + [inst("measure", qubit=q, cbit=q) for q in range(n)], n)
     got = dqsim.StatevectorSimulator(seed=3).simulate_shots(c, shots=67)
     assert got == o.OracleSimulator(seed=3).simulate_shots(c, shots=67)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["one_phase", "brickwork", "qft"])
+def test_rotation_passes_with_many_tiles_to_an_sm(kind):
+    """1,024 tiles of 12 qubits (six or seven to an SM of 148): two teams of a CTA in turn, ends with one and with both."""
+    n = 22
+    c = {"one_phase": lambda: Circuit(n, [inst("ry", qubit=q, theta=0.1 + q) for q in range(4)]),
+         "brickwork": lambda: brickwork(n, 4, seed=5, measure=False), "qft": lambda: qft(n, seed=3)}[kind]()
+    assert np.max(np.abs(dqsim.StatevectorSimulator(seed=1).simulate(c).statevector - oracle_state(c))) <= 1e-12
+
+
+@pytest.mark.gpu
+def test_trajectories_with_many_tiles_to_an_sm():
+    ins = workloads.benchmark_layers(13, 2) + [inst("measure", qubit=0, cbit=0)] + workloads.benchmark_layers(13, 2)
+    c = Circuit(13, ins + [inst("measure", qubit=q, cbit=q) for q in range(13)], 13)
+    got = dqsim.StatevectorSimulator(seed=3).simulate_shots(c, shots=451)  # 902 tiles
+    assert got == o.OracleSimulator(seed=3).simulate_shots(c, shots=451)
