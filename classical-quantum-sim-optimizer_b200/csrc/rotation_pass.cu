@@ -18,6 +18,7 @@ constexpr int E = kRotEntries;
 struct RotPass {
     int m, nphases;
     int data, ndata;  // words of the steps' data
+    int tell;
     uint8_t q[kRotMaxTile];  // tile qubits, ascending
     uint16_t out_dir[kRotMaxTile];
     uint16_t out_outer[kRotMaxOuter];
@@ -364,6 +365,10 @@ __device__ __forceinline__ void bar_arrive(int id, int threads) {
 // with half its warps while a tile was fetched: 27-qubit brickwork of 40 layers 97.0 -> 91.5 ms,
 // 25-qubit QFT 2.70 -> 2.60, 24-qubit ansatz of 8 layers 2.17 -> 2.05.  (With
 // an mbarrier for a tile's arrival the teams drift together: 97.0 ms.)
+// Phase `tell` is the second of the pass (the first of two): after the first, the
+// teller waits for its own fetch (92.6 ms for the 91.5), in the pass's middle the
+// other team for the teller (95.7).  Past the middle the teams would take turns
+// for good: passes with most of their work in the first phase run without teams.
 template <class W>
 __device__ __forceinline__ void team_body(double2* __restrict__ s, int n, const RotPass& p, uint64_t total_tiles, int basis,
                                           const W& words) {
@@ -420,10 +425,6 @@ __device__ __forceinline__ void team_body(double2* __restrict__ s, int n, const 
     };
     if (team < tiles) fetch(team, team);
     if (team == 1 && tiles > 2) fetch(2, 2);
-    // Told after the second phase (the first of two): after the first, the teller
-    // waits for its own fetch (92.6 ms for the 91.5 above); in the middle, the
-    // other team waits for the teller (95.7).
-    const int tell = min(1, (p.nphases - 1) / 2);
     int buffer = team;
     // Both teams take the same number of turns (uniform control flow); the
     // second's last one may be idle: its buffer's old tile, not stored.
@@ -442,7 +443,7 @@ __device__ __forceinline__ void team_body(double2* __restrict__ s, int n, const 
         const uint32_t index = slot | uint32_t(outer_of(j)) << kRotSlotBits;
         for (int ph = 0; ph < p.nphases; ph++) {
             rotation_phase(tile, words, ph, slot, index);
-            if (ph == tell && j >= 1 && j + 1 < tiles) {
+            if (ph == p.tell && j >= 1 && j + 1 < tiles) {
                 __pipeline_wait_prior(0);
                 __threadfence_block();
                 bar_arrive(3 + (buffer == kTeamBuffers - 1 ? 0 : buffer + 1), 2 * kTeamThreads);
@@ -507,6 +508,7 @@ void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const Ro
     RotPass p{};
     p.m = r.m;
     p.nphases = r.nphases;
+    p.tell = r.tell;
     for (int i = 0; i < r.m; i++) {
         p.q[i] = uint8_t(tile_qubits[size_t(i)]);
         p.out_dir[i] = r.out_dir[i];
@@ -542,7 +544,7 @@ void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const Ro
         static thread_local RotWords args;
         std::memcpy(args.w, r.words.data(), r.words.size() * sizeof(uint4));
         const size_t team_smem = team_tile_smem() + size_t(p.ndata) * sizeof(uint4);
-        const bool teams = r.m == kTeamTile && r.nphases > 0;
+        const bool teams = r.m == kTeamTile && r.tell >= 0;
         const uint64_t sms = teams ? resident_ctas(k_rotations_team, 2 * kTeamThreads, team_smem) : 0;
         if (teams && total >= kTeamTiles * sms) {
             k_rotations_team<<<unsigned(sms), 2 * kTeamThreads, team_smem, b.stream>>>(static_cast<double2*>(b.amps), b.n, total, basis ? 1 : 0, p, args);

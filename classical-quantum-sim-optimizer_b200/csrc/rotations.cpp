@@ -499,9 +499,26 @@ class Scheduler {
         // The kernel fetches a step and a rotation ahead.
         out_.words.insert(out_.words.end(), 2, make_uint4(0, 0, 0, 0));
         out_.nphases = int(phases.size());
+        std::vector<double> upto;  // the work up to each phase's end
+        for (const Ph& p : phases) upto.push_back((upto.empty() ? 0.0 : upto.back()) + phase_work(p.steps));
+        const double half = phases.empty() ? 0.0 : 0.55 * (upto.back() + 3000.0);  // (the rest: stores and fetches)
+        out_.tell = std::min(1, int(phases.size() - 1) / 2);
+        while (out_.tell >= 0 && upto[size_t(out_.tell)] > half) out_.tell--;
     }
 
   private:
+    // SM cycles of a 12-qubit tile's phase, as measured step by step.
+    static double phase_work(const std::vector<uint4>& steps) {
+        const double rotation[4] = {0, 135, 300, 340};
+        double cycles = 1100;
+        for (const uint4& s : steps) {
+            cycles += 75 + (s.x & 0xF00u ? 300 : 0) + (s.x & kRotTable ? 300 : 0);
+            for (int j = 0; j < 4; j++) cycles += rotation[(s.x >> (2 * j)) & 3u];
+            if (s.x & (kRotSlots | kRotSlotModuli)) cycles += 370 + 73.0 * double(s.w & 0xFFFFu);
+        }
+        return cycles;
+    }
+
     std::vector<Item> items_;
     int m_, window_;
     Lowering& lw_;

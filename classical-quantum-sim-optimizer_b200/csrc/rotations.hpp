@@ -74,6 +74,7 @@ struct RotProgram {
     int nphases = 0;
     std::vector<uint4> words;
     int data = 0;                    // first word of the steps' data
+    int tell = -1;                   // phase after which a team's fetch counts as done (rotation_pass.cu); -1: no teams
     // Where the last sweep finds the amplitude of tile index e: XOR of
     // out_dir[q] over e's set bits, out_outer[j] over the set bits of the
     // tile's index, and out_const (all swizzled).
