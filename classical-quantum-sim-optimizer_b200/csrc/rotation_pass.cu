@@ -43,12 +43,15 @@ struct ArgWords {
     const uint4* table;
     __device__ __forceinline__ uint4 operator()(uint32_t i) const { return a->w[i]; }
     __device__ __forceinline__ uint4 data(uint32_t i) const { return table[i]; }
+    // (as doubles: taken apart from a uint4, each factor cost two register moves, a quarter of a table's instructions)
+    __device__ __forceinline__ double2 factor(uint32_t i) const { return reinterpret_cast<const double2*>(table)[i]; }
 };
 struct DevWords {
     const uint4* __restrict__ w;
     const uint4* __restrict__ table;
     __device__ __forceinline__ uint4 operator()(uint32_t i) const { return __ldg(w + i); }
     __device__ __forceinline__ uint4 data(uint32_t i) const { return __ldg(table + i); }
+    __device__ __forceinline__ double2 factor(uint32_t i) const { return __ldg(reinterpret_cast<const double2*>(table) + i); }
 };
 
 __device__ __forceinline__ double lo_hi(uint32_t lo, uint32_t hi) { return __hiloint2double(int(hi), int(lo)); }
@@ -56,6 +59,14 @@ __device__ __forceinline__ double2 pair_of(uint4 u) { return make_double2(lo_hi(
 
 __device__ __forceinline__ double2 cmul_fma(double2 a, double2 b) {
     return make_double2(fma(-a.y, b.y, a.x * b.x), fma(a.y, b.x, a.x * b.y));
+}
+
+// a <- a b in place: one temporary.
+__device__ __forceinline__ void cmul_in_place(double2& a, double2 b) {
+    const double t = a.y * b.y;
+    a.y *= b.x;
+    a.y = fma(a.x, b.y, a.y);
+    a.x = fma(a.x, b.x, -t);
 }
 
 // x <- x - s t y, y <- y + s w x (kRotKept: y <- w y + s t x; kRotImag: x - i s t y, y - i s w x) on the pairs of
@@ -173,7 +184,7 @@ __device__ __forceinline__ void apply_step(double2 (&a)[E], const W& words, uint
     }
     if (s.x & kRotTable) {
 #pragma unroll
-        for (int v = 0; v < E; v++) a[v] = cmul_fma(a[v], pair_of(words.data(s.y + v)));
+        for (int v = 0; v < E; v++) cmul_in_place(a[v], words.factor(s.y + v));
     }
     if (s.x & kRotSlots) {
         const uint32_t n = s.w & 0xFFFFu, data = s.z + ((n + 3) >> 2);
@@ -186,7 +197,7 @@ __device__ __forceinline__ void apply_step(double2 (&a)[E], const W& words, uint
 #pragma unroll
         for (int v = 0; v < E; v++) {
             const int hi = __double2hiint(z.y) ^ int((s.w << (15 - v)) & 0x80000000u);
-            a[v] = cmul_fma(a[v], make_double2(z.x, __hiloint2double(hi, __double2loint(z.y))));
+            cmul_in_place(a[v], make_double2(z.x, __hiloint2double(hi, __double2loint(z.y))));
         }
     }
     if (s.x & kRotSlotModuli) {
