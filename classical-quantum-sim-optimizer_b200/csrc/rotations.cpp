@@ -484,6 +484,7 @@ class Scheduler {
             pack(p.steps, p.rots);
             phases.push_back(std::move(p));
         } while (!active_.empty());
+        if (phases.size() == 1 && phases[0].steps.empty()) phases.clear();  // relabellings only
         size_t step_at = phases.size() * 3, rot_at = step_at;
         for (const Ph& p : phases) rot_at += p.steps.size();
         out_.words.clear();
@@ -505,7 +506,7 @@ class Scheduler {
         std::vector<double> upto;  // the work up to each phase's end
         for (const Ph& p : phases) upto.push_back((upto.empty() ? 0.0 : upto.back()) + phase_work(p.steps));
         const double half = phases.empty() ? 0.0 : 0.55 * (upto.back() + 3000.0);  // (the rest: stores and fetches)
-        out_.tell = std::min(1, int(phases.size() - 1) / 2);
+        out_.tell = phases.empty() ? -1 : std::min(1, int(phases.size() - 1) / 2);
         while (out_.tell >= 0 && upto[size_t(out_.tell)] > half) out_.tell--;
     }
 

@@ -222,3 +222,28 @@ def test_trajectories_with_many_tiles_to_an_sm():
     c = Circuit(13, ins + [inst("measure", qubit=q, cbit=q) for q in range(13)], 13)
     got = dqsim.StatevectorSimulator(seed=3).simulate_shots(c, shots=451)  # 902 tiles
     assert got == o.OracleSimulator(seed=3).simulate_shots(c, shots=451)
+
+
+def moved(n, tile, how):
+    """Distinct amplitudes, then relabellings only."""
+    ins = [inst("u3", qubit=q, theta=0.3 + q, phi=0.1 * q, lam=0.7) for q in range(n)]
+    if how == "cx":
+        return Circuit(n, ins + [inst("cx", control=q, target=(q + d) % n) for d in (5, 3, 2) for q in range(n)])
+    ins += [inst("swap", a=q, b=n - 1 - q) for q in range(n // 2)]
+    if how == "swaps_x_z":
+        ins += [inst("x", qubit=q) for q in (1, n - 2, n // 2)] + [inst("z", qubit=q) for q in (2, n - 3)]
+    ins += [inst("swap", a=q, b=q + n // 2) for q in range(n // 2)]
+    ins += [inst("swap", a=q, b=n - 2 - q) for q in range(1, n // 2 - 1)]
+    return Circuit(n, ins)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["swaps", "swaps_x_z", "cx"])
+@pytest.mark.parametrize("n,tile", [(9, 5), (13, 5), (14, 8)])
+def test_passes_that_only_move_amplitudes(n, tile, how):
+    """Swap networks trade places where they are, other permutations go through tiles; tiles with and without qubit 0."""
+    c = moved(n, tile, how)
+    passes = _core.rotation_plan_dump(c.model_dump_json(), tile)["passes"]
+    assert any(p["phases"] == 0 for p in passes)
+    got = dqsim.StatevectorSimulator(seed=1, tile_qubits=tile).simulate(c).statevector
+    assert np.max(np.abs(got - oracle_state(c))) <= 1e-13
