@@ -969,6 +969,7 @@ int dq_rotation_plan_dump(const char* json, size_t len, int tile_qubits, char** 
         o.beam = kPlanBeam;
         o.keep_raw = true;
         o.targets_only = rotation_targets_only(ops, 0, ops.size(), int(n), tile_qubits);
+        o.pinned_low = rotation_pinned_low(ops, 0, ops.size(), int(n), tile_qubits);
         std::vector<double2> pool;
         auto passes = plan_tiles(ops, 0, ops.size(), int(n), o, &pool);
         std::string s = "{\"n\":" + std::to_string(n) + ",\"passes\":[";

@@ -617,6 +617,7 @@ void Executor::lower_segment(const std::vector<Operation>& ops, size_t begin, si
     const bool rotations = cfg_.rotations && !cfg_.c64 && !cfg_.model;
     o.keep_raw = rotations;
     o.targets_only = rotations && rotation_targets_only(ops, begin, end, cfg_.n, cfg_.tile_m);
+    if (rotations) o.pinned_low = rotation_pinned_low(ops, begin, end, cfg_.n, cfg_.tile_m);
     std::vector<TilePass> ps = plan_tiles(ops, begin, end, cfg_.n, o, &pool_host_);
     if (!rotations) {
         for (auto& p : ps) add_tile_pass(std::move(p));

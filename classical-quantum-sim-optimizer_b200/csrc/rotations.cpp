@@ -413,6 +413,7 @@ constexpr int kWindow = 128;  // items a phase chooses among
 // Below this many qubits half of them: planning then takes a third less time,
 // where it is most of a call, for at most 3 % longer programs (either way).
 constexpr int kWideQubits = 20;
+constexpr int kPinnedLow = 2, kPinnedQubits = 20, kPinnedTile = 12;
 struct Bits {
     uint64_t w[2] = {0, 0};
     void set(int i) { w[i >> 6] |= uint64_t(1) << (i & 63); }
@@ -1090,6 +1091,13 @@ bool rotation_targets_only(const std::vector<Operation>& ops, size_t begin, size
     for (size_t i = begin; i < end; i++) wide = wide || (ops[i].type == Operation::Diagonal && ops[i].qubits.size() > 1);
     for (size_t i = begin; wide && i < end; i++) wide = rotation_form(ops[i]);
     return wide;
+}
+
+int rotation_pinned_low(const std::vector<Operation>& ops, size_t begin, size_t end, int n, int m) {
+    if (n < kPinnedQubits || m < kPinnedTile) return 0;
+    for (size_t i = begin; i < end; i++)
+        if (!rotation_form(ops[i]) || int(ops[i].touched().size()) + kPinnedLow > m) return 0;
+    return kPinnedLow;
 }
 
 bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<int>& tile_qubits, int n,

@@ -104,6 +104,17 @@ inline uint32_t rot_swizzle(uint32_t p) {
 // to slots outweigh the passes saved (27-qubit brickwork 13 -> 12, 3 % slower).
 bool rotation_targets_only(const std::vector<Operation>& ops, size_t begin, size_t end, int n, int m);
 
+// Lowest qubits that every tile of ops[begin, end) holds
+// (TilePlanOptions::pinned_low).  A tile without them is fetched and stored 16
+// bytes at a time, half a sector and an L1 lookup each: some 8,000 cycles on the
+// 35,000 to 45,000 of a pass.  Two give up a sixth of a tile's qubits for runs of 64
+// bytes.  20 to 26 qubits, brickwork, QFT, ansatz and layers: 13 % faster at 24 qubits,
+// 7 to 10 % at the others (one pinned qubit 5 to 9 %, three 2 to 9 %); 27-qubit
+// brickwork 89.0 -> 84.8 ms, 25-qubit QFT 2.39 -> 2.12, 28-qubit ansatz 22.5 -> 17.2.  Below 20 qubits a pass is one
+// wave of tiles and their number counts: 18 qubits 7 % slower.  None
+// where an operation has no rotation form or touches more than the tile has left.
+int rotation_pinned_low(const std::vector<Operation>& ops, size_t begin, size_t end, int n, int m);
+
 // Plans the pass `ops` over `tile_qubits` (ascending) of an n-qubit state.
 // Targets and swapped qubits are tile qubits; controls and diagonal qubits may
 // lie outside, where the tile's index gives their value.  False when an

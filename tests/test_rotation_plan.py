@@ -247,3 +247,11 @@ def test_passes_that_only_move_amplitudes(n, tile, how):
     assert any(p["phases"] == 0 for p in passes)
     got = dqsim.StatevectorSimulator(seed=1, tile_qubits=tile).simulate(c).statevector
     assert np.max(np.abs(got - oracle_state(c))) <= 1e-13
+
+
+@pytest.mark.parametrize("n,tile,low", [(19, 12, 0), (20, 12, 2), (20, 11, 0), (21, 13, 2)])
+def test_tiles_of_wide_registers_hold_the_low_qubits(n, tile, low):
+    ins = [inst("ry", qubit=q, theta=0.1 + q) for q in range(n)] + [inst("cx", control=q, target=(q + 7) % n) for q in range(n)]
+    passes = _core.rotation_plan_dump(Circuit(n, ins).model_dump_json(), tile)["passes"]
+    assert all(p["ok"] and len(p["qubits"]) == tile for p in passes)
+    assert all(set(range(low)) <= set(p["qubits"]) for p in passes)
