@@ -485,6 +485,7 @@ __global__ void __launch_bounds__(2 * kTeamThreads, 1)
 }
 
 constexpr int kSwapThreads = 256, kSwapEach = 8;
+constexpr uint64_t kSwapStates = uint64_t(1) << 19;  // amplitudes, 8 MB
 
 // A permutation of the state: amplitude x becomes -+ the one at y = const ^ the XOR of to[b] over x's bits.
 struct StateMap {
@@ -492,13 +493,13 @@ struct StateMap {
     int sign_const;
 };
 
-// Passes of relabellings that are their own inverse (swap networks), over tiles
-// without qubit 0: pairs (x, y) change places where they are.  Bound by HBM.
-// A tile kernel moves 16 bytes at a time here, half a sector, from rows a tile's
-// lowest qubit apart; this one moves whole rows: the last 12 swapped qubits of a
-// 25-qubit QFT, 6 to 11 and 13 to 18, 0.43 -> 0.24 ms (4.5 TB/s), the QFT
-// 2.58 -> 2.39 ms.  Tiles with qubit 0 (rows of whole sectors) and other
-// permutations go through a tile kernel.
+// Passes of relabellings that are their own inverse (swap networks) and leave
+// qubit 0 in place: pairs (x, y) change places where they are.  Bound by HBM or L2.
+// A tile kernel without qubit 0 moves 16 bytes at a time, half a sector; this one
+// moves whole rows (25-qubit QFT without pinned qubits: last pass 0.43 -> 0.24 ms).
+// With qubit 0 in the tile it is the faster one while the state stays in L2
+// (QFT of 16 qubits 0.076 -> 0.069 ms; 13 and 19 qubits equal); from 22 qubits on the
+// tile kernel reads its rows in better order (25 qubits 2.12 ms against 2.28).
 __global__ void __launch_bounds__(kSwapThreads) k_swap_places(double2* __restrict__ s, int n, uint64_t states,
                                                               const __grid_constant__ StateMap map) {
     constexpr uint64_t chunk = uint64_t(kSwapThreads) * kSwapEach;
@@ -610,7 +611,8 @@ uint64_t resident_ctas(Kernel kernel, int threads, size_t smem) {
 void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const RotProgram& r, const uint4* words_dev,
                    bool basis) {
     if (b.c64) fail(kValueError, "rotation passes run on complex128 states");
-    if (StateMap map; r.nphases == 0 && !basis && tile_qubits[0] > 0 && own_inverse(r, tile_qubits, b.n, map)) {
+    const bool swaps = r.nphases == 0 && !basis && (tile_qubits[0] > 0 || (b.W << b.n) <= kSwapStates);
+    if (StateMap map; swaps && own_inverse(r, tile_qubits, b.n, map) && map.to[0] == 1) {
         const uint64_t chunks = ((uint64_t(1) << b.n) + kSwapThreads * kSwapEach - 1) / (kSwapThreads * kSwapEach) * b.W;
         k_swap_places<<<unsigned(std::min(chunks, resident_ctas(k_swap_places, kSwapThreads, 0))), kSwapThreads, 0, b.stream>>>(
             static_cast<double2*>(b.amps), b.n, b.W, map);
