@@ -847,8 +847,9 @@ void Executor::lower(const Operation& op, std::vector<Condition>& conds) {
 
 void Executor::prepare(const k::Batch& b) {
     if (!fused_.empty()) {
-        norm_tiles_.ensure((size_t(b.W) << (b.n - kFusedM)) * 8, "fused tile norms");
-        norm_states_.ensure(size_t(b.W) * size_t(k::fused_norm_parts(b.n)) * 8, "fused state norms");
+        norm_tiles_.ensure((size_t(b.W) << (b.n - kFusedM)) * (k::fused_norm_direct(b.n) ? 16 : 8), "fused tile norms");
+        if (!k::fused_norm_direct(b.n))
+            norm_states_.ensure(size_t(b.W) * size_t(k::fused_norm_parts(b.n)) * 8, "fused state norms");
         k::fused_configure();
     }
     upload(b.stream);
@@ -907,6 +908,7 @@ void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, b
                    bool discard) {
     upload(b.stream);
     std::vector<uint64_t> host_cbits;
+    bool norm_half = false;
     bool norm_pending = false;  // a fused pass left a norm the next fused pass divides out
     for (size_t si = 0; si < steps_.size(); si++) {
         const Step& s = steps_[si];
@@ -933,27 +935,33 @@ void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, b
         if (s.fused >= 0) {
             const FusedPass& p = fused_[size_t(s.fused)];
             const size_t tiles = size_t(b.W) << (b.n - kFusedM);
-            get(norm_tiles_, tiles * 8, b.stream, "fused tile norms");
-            get(norm_states_, size_t(b.W) * size_t(k::fused_norm_parts(b.n)) * 8, b.stream, "fused state norms");
+            const bool direct = k::fused_norm_direct(b.n);
+            get(norm_tiles_, tiles * (direct ? 16 : 8), b.stream, "fused tile norms");
+            if (!direct)
+                get(norm_states_, size_t(b.W) * size_t(k::fused_norm_parts(b.n)) * 8, b.stream, "fused state norms");
+            // This pass's tile norms; the last pass's are its input (the two halves in turn).
+            if (direct) norm_half = !norm_half;
+            double* tile_norms = norm_tiles_.as<double>() + (norm_half ? tiles : 0);
+            const double* in_norms = direct ? norm_tiles_.as<double>() + (norm_half ? 0 : tiles) : norm_states_.as<double>();
             if (rec) rec->begin(kcFused, step_bytes(si, b));
             k::fused_pass(b, p, fused_blocks_.as<FusedBlock>(), upool_.as<uint16_t>(), b.err,
-                          norm_pending ? norm_states_.as<double>() : nullptr, norm_tiles_.as<double>(),
-                          from_basis && si == 0);
+                          norm_pending ? in_norms : nullptr, tile_norms, from_basis && si == 0);
             if (rec) rec->end();
             const bool last_fused = si + 1 == steps_.size() || steps_[si + 1].fused < 0;
             if (normalize || si + 1 != steps_.size()) {
                 // Tile norms read (8 B per tile); the final rescale reads and writes the state.
-                if (rec)
+                const int launches = (direct ? 0 : 1) + (last_fused ? 1 : 0);
+                if (rec && launches)
                     rec->begin(kcNorm,
                                double(tiles) * 8.0 + (last_fused ? 2.0 * double(size_t(b.W) << b.n) * 8.0 : 0.0),
-                               last_fused ? 2 : 1);
-                k::fused_state_norm(b, norm_tiles_.as<double>(), norm_states_.as<double>());
+                               launches);
+                if (!direct) k::fused_state_norm(b, tile_norms, norm_states_.as<double>());
                 norm_pending = true;
                 if (last_fused) {
-                    k::fused_renormalize(b, norm_states_.as<double>());
+                    k::fused_renormalize(b, direct ? tile_norms : norm_states_.as<double>());
                     norm_pending = false;
                 }
-                if (rec) rec->end();
+                if (rec && launches) rec->end();
             }
             if (profile) {
                 cuda_check(cudaStreamSynchronize(b.stream), "stream synchronize");

@@ -248,6 +248,15 @@ __device__ __forceinline__ void put_split2(unsigned char* x, uint32_t off, uint6
     *reinterpret_cast<__half2*>(x + kPartBytes + off) = __floats2half2_rn(__uint_as_float(lr), __uint_as_float(li));
 }
 
+// Sum of `count` numbers by a whole warp, in a fixed order; every lane gets it.
+__device__ __forceinline__ double sum_parts(const double* __restrict__ parts, int count) {
+    if (count == 1) return parts[0];
+    double sum = 0.0;
+    for (int p = int(threadIdx.x & 31u); p < count; p += 32) sum += parts[p];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(~0u, sum, o);
+    return sum;
+}
+
 // Global position of the first amplitude of tile t (its local index 0).
 __device__ __forceinline__ uint64_t tile_base(uint64_t t, int n, const FusedQubits& fq) {
     const int rest = n - kFusedM;
@@ -406,9 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // state's norm is the fixed-order sum of its partial sums.
         if (in_norm && (base >> n) != scale_state) {
             scale_state = base >> n;
-            double nrm = 0.0;
-            for (int p = 0; p < norm_parts; p++) nrm += in_norm[scale_state * uint64_t(norm_parts) + uint64_t(p)];
-            scale = 1.0 / sqrt(nrm);
+            scale = 1.0 / sqrt(sum_parts(in_norm + scale_state * uint64_t(norm_parts), norm_parts));
         }
         const float fs = float(scale * double(kScale));
         const uint64_t fs2 = pack2(__float_as_uint(fs), __float_as_uint(fs));
@@ -668,7 +675,11 @@ int sm_count() {
 // Tile norms per partial: block (state st, part p) sums tiles
 // [p * kNormChunk, (p + 1) * kNormChunk) of state st in a fixed order, so the
 // state's norm (the sum of its parts in order) is the same on every run.
-constexpr uint64_t kNormChunk = 2048;
+// Up to kNormDirect tiles the next pass sums the tile norms itself: the sum's kernel
+// was 3 of the 28 us of a small circuit's pass and near half of a batch's launches (14-qubit
+// ansatz 0.068 -> 0.060 ms, 18 qubits 0.111 -> 0.099, 64 circuits of 12 to 15
+// qubits 0.156 -> 0.140; 256 of 12 to 22 qubits, which fill the device, 12.05 -> 12.2).
+constexpr uint64_t kNormChunk = 2048, kNormDirect = 64;
 __global__ void k_state_norm(const double* __restrict__ tile_norm, uint64_t tiles_per_state, int parts,
                              double* __restrict__ norm) {
     __shared__ double sm[256];
@@ -693,9 +704,7 @@ __global__ void k_scale_states(float2* __restrict__ s, int n, uint64_t items, co
     for (uint64_t g = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < items; g += uint64_t(gridDim.x) * blockDim.x) {
         if ((g >> n) != cur) {
             cur = g >> n;
-            double nrm = 0.0;
-            for (int p = 0; p < parts; p++) nrm += norm[cur * uint64_t(parts) + uint64_t(p)];
-            sc = 1.0 / sqrt(nrm);
+            sc = 1.0 / sqrt(sum_parts(norm + cur * uint64_t(parts), parts));  // (a warp's items belong to one state)
         }
         float2 v = s[g];
         s[g] = make_float2(float(double(v.x) * sc), float(double(v.y) * sc));
@@ -706,9 +715,11 @@ __global__ void k_scale_states(float2* __restrict__ s, int n, uint64_t items, co
 
 size_t fused_smem_bytes() { return kSmemBytes; }
 
+bool fused_norm_direct(int n) { return (uint64_t(1) << (n - kFusedM)) <= kNormDirect; }
+
 int fused_norm_parts(int n) {
     const uint64_t tiles = uint64_t(1) << (n - kFusedM);
-    return int((tiles + kNormChunk - 1) / kNormChunk);
+    return int(fused_norm_direct(n) ? tiles : (tiles + kNormChunk - 1) / kNormChunk);
 }
 
 void fused_state_norm(const Batch& b, const double* tile_norm, double* norm) {

@@ -270,8 +270,11 @@ namespace k {
 void fused_pass(const Batch& b, const FusedPass& p, const FusedBlock* blocks_dev, const uint16_t* upool_dev,
                 int* err_dev, const double* in_norm, double* tile_norm, bool basis = false);
 // Partial sums of each state's tile norms, fused_norm_parts(n) per state in
-// a fixed order (state st's norm is the in-order sum of norm[st*parts ..]).
+// a fixed order (state st's norm is the sum of norm[st*parts ..]).  Where
+// fused_norm_direct(n), the tile norms themselves are the parts and the next
+// pass, which writes its own elsewhere, or fused_renormalize takes them as they are.
 int fused_norm_parts(int n);
+bool fused_norm_direct(int n);
 void fused_state_norm(const Batch& b, const double* tile_norm, double* norm);
 // Divides every state by the square root of its norm, summed from the partial
 // sums fused_state_norm left (FP64 scale).
