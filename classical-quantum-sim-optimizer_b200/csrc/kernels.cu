@@ -335,7 +335,9 @@ __global__ void __launch_bounds__(kThreads) k_collapse(V* __restrict__ s, int n,
 // one, kChainReset) or left as it is when nothing follows that reads it
 // (kChainDiscard).  Separate measurements read and write 2.5 states each in
 // three launches.  States of up to 12 qubits keep their squared magnitudes in
-// shared memory.
+// shared memory.  Bound by L2 and HBM; 300 states of 15 qubits (157 MB): 89 us a
+// run of one, 168 us one of all 15 qubits with the histogram's bits; the 15-qubit dynamic
+// circuit of three rounds 3.7 -> 2.65 ms with it.
 constexpr int kChainMax = 64;
 constexpr int kChainCached = 12;
 enum ChainMode : int { kChainDiscard = 0, kChainKeep = 1, kChainReset = 2 };
@@ -503,7 +505,8 @@ __global__ void k_norm2(const V* __restrict__ s, double* __restrict__ out, uint6
 // memory, where those of one local output are added.  One CTA per value of the
 // selected high qubits and per part of the unselected ones; the parts' tables
 // are added by k_marginal_parts in order, so the result does not depend on
-// scheduling.
+// scheduling.  Bound by HBM: 1.28 ms at 30 qubits of complex64 (6.7 TB/s), 88 us at 25
+// of complex128 (6.1 TB/s); with one atomic add per amplitude it took 42 ms at 30 qubits.
 constexpr int kMargBits = 12;  // local qubits of a chunk
 constexpr int kMargThreads = 256;
 

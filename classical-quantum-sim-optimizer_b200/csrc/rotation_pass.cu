@@ -226,47 +226,47 @@ __device__ __forceinline__ uint32_t swz(uint32_t e) {
 // One phase of a tile: this thread's 16 amplitudes through the steps.
 template <class W>
 __device__ __forceinline__ void rotation_phase(double2* tile, const W& words, int ph, uint32_t slot, uint32_t index) {
-                const uint4 h0 = words(3 * ph), h1 = words(3 * ph + 1), h2 = words(3 * ph + 2);
-                const uint32_t ub[9] = {h1.x & 0xFFFFu, h1.x >> 16, h1.y & 0xFFFFu, h1.y >> 16, h1.z & 0xFFFFu,
-                                        h1.z >> 16,     h1.w & 0xFFFFu, h1.w >> 16, h2.x & 0xFFFFu};
-                uint32_t place = 0;
-    #pragma unroll
-                for (int b = 0; b < 9; b++) place ^= (slot >> b) & 1u ? ub[b] : 0u;
-                const uint32_t vb[4] = {h0.z & 0xFFFFu, h0.z >> 16, h0.w & 0xFFFFu, h0.w >> 16};
-                uint32_t vv[E];
-    #pragma unroll
-                for (int v = 0; v < E; v++)
-                    vv[v] = (v & 1 ? vb[0] : 0u) ^ (v & 2 ? vb[1] : 0u) ^ (v & 4 ? vb[2] : 0u) ^ (v & 8 ? vb[3] : 0u);
-                double2 a[E];
-    #pragma unroll
-                for (int v = 0; v < E; v++) a[v] = tile[place ^ vv[v]];
-                RotStream<W> rots(words, h2.y, index);
-                uint4 next = words(h0.x);
-                for (uint32_t o = 1; o <= h0.y; o++) {
-                    const uint4 st = next;
-                    next = words(h0.x + o);
-                    apply_step(a, words, st, index, rots);
-                }
-    #pragma unroll
-                for (int v = 0; v < E; v++) tile[place ^ vv[v]] = a[v];
+    const uint4 h0 = words(3 * ph), h1 = words(3 * ph + 1), h2 = words(3 * ph + 2);
+    const uint32_t ub[9] = {h1.x & 0xFFFFu, h1.x >> 16, h1.y & 0xFFFFu, h1.y >> 16, h1.z & 0xFFFFu,
+                            h1.z >> 16,     h1.w & 0xFFFFu, h1.w >> 16, h2.x & 0xFFFFu};
+    uint32_t place = 0;
+#pragma unroll
+    for (int b = 0; b < 9; b++) place ^= (slot >> b) & 1u ? ub[b] : 0u;
+    const uint32_t vb[4] = {h0.z & 0xFFFFu, h0.z >> 16, h0.w & 0xFFFFu, h0.w >> 16};
+    uint32_t vv[E];
+#pragma unroll
+    for (int v = 0; v < E; v++)
+        vv[v] = (v & 1 ? vb[0] : 0u) ^ (v & 2 ? vb[1] : 0u) ^ (v & 4 ? vb[2] : 0u) ^ (v & 8 ? vb[3] : 0u);
+    double2 a[E];
+#pragma unroll
+    for (int v = 0; v < E; v++) a[v] = tile[place ^ vv[v]];
+    RotStream<W> rots(words, h2.y, index);
+    uint4 next = words(h0.x);
+    for (uint32_t o = 1; o <= h0.y; o++) {
+        const uint4 st = next;
+        next = words(h0.x + o);
+        apply_step(a, words, st, index, rots);
+    }
+#pragma unroll
+    for (int v = 0; v < E; v++) tile[place ^ vv[v]] = a[v];
 }
 
 // The last sweep: out of the frame, with its signs, to the state.
 __device__ __forceinline__ void store_tile(const double2* tile, double2* __restrict__ gp, const RotPass& p, int rest,
                                            uint64_t outer, uint32_t slot, uint32_t place) {
-                uint32_t c = p.out_const ^ place;
-                uint32_t sg = uint32_t(p.sign_const) ^ odd(p.sign_outer & uint32_t(outer)) ^ odd(p.sign_local & slot);
-                if (p.outer_moves)
-                    for (int j = 0; j < rest; j++)
-                        if ((outer >> j) & 1) c ^= p.out_outer[j];
-    #pragma unroll
-                for (int k = 0; k < E; k++) {
-                    double2 x = tile[c ^ p.reg_out[k]];
-                    const int flip = int((sg ^ (uint32_t(p.reg_sign) >> k)) << 31);
-                    x.x = __hiloint2double(__double2hiint(x.x) ^ flip, __double2loint(x.x));
-                    x.y = __hiloint2double(__double2hiint(x.y) ^ flip, __double2loint(x.y));
-                    gp[p.reg_off[k]] = x;
-                }
+    uint32_t c = p.out_const ^ place;
+    uint32_t sg = uint32_t(p.sign_const) ^ odd(p.sign_outer & uint32_t(outer)) ^ odd(p.sign_local & slot);
+    if (p.outer_moves)
+        for (int j = 0; j < rest; j++)
+            if ((outer >> j) & 1) c ^= p.out_outer[j];
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        double2 x = tile[c ^ p.reg_out[k]];
+        const int flip = int((sg ^ (uint32_t(p.reg_sign) >> k)) << 31);
+        x.x = __hiloint2double(__double2hiint(x.x) ^ flip, __double2loint(x.x));
+        x.y = __hiloint2double(__double2hiint(x.y) ^ flip, __double2loint(x.y));
+        gp[p.reg_off[k]] = x;
+    }
 }
 
 // Few or small tiles.  Persistent; a CTA holds `1 << pack` tiles of 2^m amplitudes at
@@ -438,7 +438,8 @@ __device__ __forceinline__ void team_body(double2* __restrict__ s, int n, const 
     if (team == 1 && tiles > 2) fetch(2, 2);
     int buffer = team;
     // Both teams take the same number of turns (uniform control flow); the
-    // second's last one may be idle: its buffer's old tile, not stored.
+    // second's last one may be idle and touches no buffer: the other team may
+    // still be at work there.
     for (int i = 0; i < (tiles + 1) / 2; i++) {
         const int j = 2 * i + team;
         if (i == 0) {
@@ -452,7 +453,8 @@ __device__ __forceinline__ void team_body(double2* __restrict__ s, int n, const 
         }
         double2* tile = all + (size_t(buffer) << m);
         const uint32_t index = slot | uint32_t(outer_of(j)) << kRotSlotBits;
-        for (int ph = 0; ph < p.nphases; ph++) {
+        const int phases = j < tiles ? p.nphases : 0;
+        for (int ph = 0; ph < phases; ph++) {
             rotation_phase(tile, words, ph, slot, index);
             if (ph == p.tell && j >= 1 && j + 1 < tiles) {
                 __pipeline_wait_prior(0);
