@@ -498,13 +498,7 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
             circuits_[ci].stream = int(j);
             load[j] += cost(ci);
         }
-        side_.resize(nside, nullptr);
-        join_.resize(nside, nullptr);
-        for (size_t j = 0; j < nside; j++) {
-            cuda_check(cudaStreamCreateWithFlags(&side_[j], cudaStreamNonBlocking), "cudaStreamCreate");
-            cuda_check(cudaEventCreateWithFlags(&join_[j], cudaEventDisableTiming), "cudaEventCreate");
-        }
-        cuda_check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
+        sides_ = nside;
         for (size_t ci : order) {
             const uint64_t n = circuits_[ci].n;
             fused_quads_ += n > uint64_t(kFusedM) ? uint64_t(1) << (n - kFusedM) >> 2 : 1;
@@ -607,7 +601,36 @@ void BatchRun::work(double* bytes, double* tensor_flops, double* cuda_core_flops
     *cuda_core_flops = cf;
 }
 
-void BatchRun::enqueue() {
+void BatchRun::open_side_streams() {
+    if (sides_ == 0 || !side_.empty()) return;
+    side_.resize(sides_, nullptr);
+    join_.resize(sides_, nullptr);
+    for (size_t j = 0; j < sides_; j++) {
+        cuda_check(cudaStreamCreateWithFlags(&side_[j], cudaStreamNonBlocking), "cudaStreamCreate");
+        cuda_check(cudaEventCreateWithFlags(&join_[j], cudaEventDisableTiming), "cudaEventCreate");
+    }
+    cuda_check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
+}
+
+// While it is captured, the side streams are chains of graph nodes: the main
+// stream continues from a chain's last node, so none has to be created (64 streams
+// take milliseconds to create and to destroy).
+struct Chains {
+    cudaStream_t s;
+    std::vector<cudaGraphNode_t> at() const {
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t* nodes = nullptr;
+        size_t count = 0;
+        cuda_check(cudaStreamGetCaptureInfo_v2(s, &status, nullptr, nullptr, &nodes, &count), "capture info");
+        return std::vector<cudaGraphNode_t>(nodes, nodes + count);
+    }
+    void go(std::vector<cudaGraphNode_t>& nodes) const {
+        cuda_check(cudaStreamUpdateCaptureDependencies(s, nodes.data(), nodes.size(), cudaStreamSetCaptureDependencies),
+                   "capture dependencies");
+    }
+};
+
+void BatchRun::enqueue(bool capturing) {
     cudaStream_t s = dev_->stream;
     const size_t S = c64_ ? 8 : 16;
     const int count = int(circuits_.size());
@@ -620,8 +643,21 @@ void BatchRun::enqueue() {
         k_first_amp<float2><<<(count + 127) / 128, 128, 0, s>>>(amps_.as<float2>(), offs, count);
     else
         k_first_amp<double2><<<(count + 127) / 128, 128, 0, s>>>(amps_.as<double2>(), offs, count);
-    if (!side_.empty()) {
+    const Chains chains{s};
+    std::vector<std::vector<cudaGraphNode_t>> tails;
+    if (sides_ > 0 && capturing) {
+        std::vector<cudaGraphNode_t> fork = chains.at();
+        tails.assign(sides_, fork);
+        for (const Circ& c : circuits_) {
+            if (!c.fused) continue;
+            chains.go(tails[size_t(c.stream)]);
+            c.fused->run(circuit_view(c, s), nullptr);
+            tails[size_t(c.stream)] = chains.at();
+        }
+        chains.go(fork);
+    } else if (sides_ > 0) {
         // Fused circuits on the side streams, beside the persistent kernel.
+        open_side_streams();
         cuda_check(cudaEventRecord(fork_, s), "fork");
         for (cudaStream_t st : side_) cuda_check(cudaStreamWaitEvent(st, fork_, 0), "fork");
         for (const Circ& c : circuits_)
@@ -650,7 +686,13 @@ void BatchRun::enqueue() {
                                                               head_.as<unsigned long long>(), total_items_,
                                                               err_.as<int>());
     }
-    for (cudaEvent_t e : join_) cuda_check(cudaStreamWaitEvent(s, e, 0), "join");
+    if (capturing && sides_ > 0) {
+        std::vector<cudaGraphNode_t> all = chains.at();
+        for (const auto& t : tails) all.insert(all.end(), t.begin(), t.end());
+        chains.go(all);
+    } else if (sides_ > 0) {
+        for (cudaEvent_t e : join_) cuda_check(cudaStreamWaitEvent(s, e, 0), "join");
+    }
     if (c64_)
         k_zz_parts<float2><<<unsigned(zz_parts_), 256, 0, s>>>(amps_.as<float2>(), offs, count, zz_at_.as<uint64_t>(),
                                                                zz_sums_.as<double>());
@@ -680,7 +722,7 @@ double BatchRun::run(bool use_graph) {
         cudaGraph_t g;
         cuda_check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
         try {
-            enqueue();
+            enqueue(true);
         } catch (...) {
             cudaStreamEndCapture(s, &g);
             throw;
@@ -696,7 +738,7 @@ double BatchRun::run(bool use_graph) {
     if (use_graph)
         cuda_check(cudaGraphLaunch(graph_, s), "graph launch");
     else
-        enqueue();
+        enqueue(false);
     cuda_check(cudaEventRecord(b, s), "event");
     cuda_check(cudaEventSynchronize(b), "event sync");
     float ms = 0;

@@ -95,11 +95,13 @@ class BatchRun {
     DevMem amps_, recs_, ops_, pool_, done_, head_, err_, probs_, tmp_, circ_off_, circ_of_tile_, samples_, zz_part_,
         zz_at_, zz_sums_, seeds_;
     cudaGraphExec_t graph_ = nullptr;
+    size_t sides_ = 0;  // side streams the fused circuits are spread over
     std::vector<cudaStream_t> side_;
     std::vector<cudaEvent_t> join_;
     cudaEvent_t fork_ = nullptr;
     double tile_bytes_ = 0, tile_flops_ = 0;
-    void enqueue();
+    void enqueue(bool capturing);
+    void open_side_streams();
     k::Batch circuit_view(const Circ& c, cudaStream_t s) const;
 };
 
