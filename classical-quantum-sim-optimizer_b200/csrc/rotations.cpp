@@ -987,15 +987,17 @@ class Scheduler {
                 part.mask = slots(x.mask);
                 part.t = x.t;
                 part.u = double(ld(x.t) / (1.0L + ld(x.t) * x.t));
+                // Entries that owe different factors must not mix, whatever the kind: those
+                // without the factor i are in place without the look-ahead above.
+                for (int j = 0; j < kRotRegBits; j++)
+                    if (((d >> j) & 1) && pend[j] != 0.0) {
+                        emit_table({}, 0.0);
+                        break;
+                    }
                 if (part.kind == kRotKept) {
                     part.u = double(1.0L + ld(x.t) * x.t);
                     uniform_ -= lost;
                 } else {
-                    for (int j = 0; j < kRotRegBits; j++)
-                        if (((d >> j) & 1) && pend[j] != 0.0) {
-                            emit_table({}, 0.0);
-                            break;
-                        }
                     pend[low] -= lost;
                 }
                 parts_.push_back(part);

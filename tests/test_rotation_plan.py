@@ -12,7 +12,7 @@ import struct
 import numpy as np
 import pytest
 
-from helpers import Circuit, brickwork, hea, inst, qft, random_circuit
+from helpers import GATES, Circuit, brickwork, hea, inst, qft, random_circuit
 from oracle import oracle as o
 
 import dqsim
@@ -255,3 +255,119 @@ def test_tiles_of_wide_registers_hold_the_low_qubits(n, tile, low):
     passes = _core.rotation_plan_dump(Circuit(n, ins).model_dump_json(), tile)["passes"]
     assert all(p["ok"] and len(p["qubits"]) == tile for p in passes)
     assert all(set(range(low)) <= set(p["qubits"]) for p in passes)
+
+
+# What random circuits below draw from: every gate with a rotation form (no dense matrices but RXX).
+FORMS = [g for g in GATES if g[0] not in ("rccx", "rc3x")]
+SPECIAL = [0.0, np.pi, -np.pi, np.pi / 2, -np.pi / 2, np.pi / 4, 2 * np.pi, 1.0, -0.3]
+
+
+def form_circuit(seed, n, gates, names=None):
+    """Gates with a rotation form on random qubits; a third of the angles are multiples of pi/4 or the like."""
+    rng = np.random.default_rng(seed)
+    forms = [g for g in FORMS if len(g[1]) <= n and (names is None or g[0] in names)]
+    ins = []
+    for _ in range(gates):
+        kind, qubits, params = forms[int(rng.integers(len(forms)))]
+        fields = dict(zip(qubits, rng.choice(n, size=len(qubits), replace=False).tolist()))
+        for p in params:
+            fields[p] = float(rng.choice(SPECIAL) if rng.random() < 1 / 3 else rng.uniform(-np.pi, np.pi))
+        ins.append(inst(kind, **fields))
+    return Circuit(n, ins)
+
+
+def mixed_layers(n, depth, seed, kinds, two):
+    """Layers of one-qubit gates (kinds[layer % len] everywhere, or drawn from a tuple of them) and bricks of `two`."""
+    rng = np.random.default_rng(seed)
+    ins = []
+    for layer in range(depth):
+        for q in range(n):
+            kind = kinds[layer % len(kinds)]
+            kind = kind if isinstance(kind, str) else str(rng.choice(kind))
+            params = next(g[2] for g in GATES if g[0] == kind)
+            ins.append(inst(kind, qubit=q, **{p: float(rng.uniform(-np.pi, np.pi)) for p in params}))
+        for a in range(layer % 2, n - 1, 2):
+            ins.append(inst("rxx", a=a, b=a + 1, theta=float(rng.uniform(-np.pi, np.pi))) if two == "rxx" else
+                       inst(two, control=a, target=a + 1))
+    return Circuit(n, ins)
+
+
+def replay_error(c, tile):
+    plan = _core.rotation_plan_dump(c.model_dump_json(), tile)
+    assert all(p["ok"] for p in plan["passes"])
+    return np.max(np.abs(replay(plan) - oracle_state(c))), plan
+
+
+def kinds_by_phase(plan):
+    """Per phase of every pass, the kinds of its rotations."""
+    for p in plan["passes"]:
+        words = np.array(p["words"], dtype=np.uint32).reshape(-1, 4).tolist()
+        for ph in range(p["phases"]):
+            first, steps = words[3 * ph][:2]
+            found = set()
+            for w in words[first:first + steps]:
+                found |= {((w[0] >> (2 * j)) & 3) - 1 for j in range(4) if (w[0] >> (2 * j)) & 3}
+                if (w[0] >> 8) & 15:
+                    found.add((w[0] >> 12) & 3)
+            yield found
+
+
+# Layers in which rotations without the factor i (RX, SX, RXX) meet those with it.
+MIXED = [(("rx", "ry"), "cx"), (("rx", "ry"), "cz"), ((("sx", "t", "h"),), "cx"), ((("sx", "t", "h"),), "cz"),
+         ((("rx", "h"),), "cx"), ((("rx", "h"),), "cz"), ((("sx", "u3"),), "cx"), ((("sx", "u3"),), "cz"),
+         (("ry",), "rxx"), ((("rx", "ry"),), "rxx")]
+
+
+@pytest.mark.parametrize("kinds,two", MIXED, ids=str)
+def test_layers_of_rotations_with_and_without_the_factor_i(kinds, two):
+    for n, depth in ((5, 2), (6, 3), (7, 8), (8, 5), (9, 6), (10, 12)):
+        c = mixed_layers(n, depth, n, kinds, two)
+        for tile in {5, n}:
+            assert replay_error(c, tile)[0] <= 1e-13, (n, depth, tile)
+
+
+@pytest.mark.parametrize("kinds,two", [(("rx", "ry"), "cx"), ((("sx", "t", "h"),), "cx"), (("ry",), "rxx")], ids=str)
+def test_those_layers_hold_phases_of_both_kinds(kinds, two):
+    """Kept rotations and rotations without the factor i in one phase, so that the replay above covers it."""
+    plan = replay_error(mixed_layers(10, 12, 10, kinds, two), 10)[1]
+    assert any({KEPT, IMAG} <= found for found in kinds_by_phase(plan))
+
+
+@pytest.mark.parametrize("instructions", [
+    [inst("sx", qubit=4), inst("cx", control=3, target=4), inst("h", qubit=4), inst("cx", control=3, target=4),
+     inst("sx", qubit=4)],
+    [inst("rx", qubit=4, theta=1.1), inst("cx", control=3, target=4), inst("ry", qubit=4, theta=1.2),
+     inst("cx", control=3, target=4), inst("rx", qubit=4, theta=0.7)],
+    [inst("rx", qubit=2, theta=1.0), inst("rxx", a=3, b=0, theta=0.8), inst("rxx", a=4, b=2, theta=0.8),
+     inst("h", qubit=2), inst("h", qubit=4)]])
+def test_few_gates_that_owe_different_factors(instructions):
+    assert replay_error(Circuit(5, instructions), 5)[0] <= 1e-15
+
+
+@pytest.mark.parametrize("n", [5, 6, 7, 8, 9])
+def test_random_circuits_of_every_gate_with_a_rotation_form(n):
+    for seed in range(30):
+        for gates, names in ((60, None), (25, ("h", "x", "sx", "t", "rx", "ry", "rz", "u3", "cx", "cz", "rxx", "rzz"))):
+            c = form_circuit(1000 * n + seed, n, gates, names)
+            for tile in {5, min(n, 6 + seed % 3)}:
+                assert replay_error(c, tile)[0] <= 1e-13, (seed, gates, tile)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kinds,two", [(("rx", "ry"), "cx"), ((("sx", "t", "h"),), "cz"), (("ry",), "rxx")], ids=str)
+def test_mixed_rotations_on_the_device(kinds, two):
+    """The default complex128 form as a state, as shots and in a batch."""
+    sizes = [(5, 4), (8, 6), (13, 5), (15, 3)]
+    plain = [mixed_layers(n, depth, n, kinds, two) for n, depth in sizes]
+    measured = [Circuit(n, c.data["instructions"] + [inst("measure", qubit=q, cbit=q) for q in range(n)], n)
+                for (n, _), c in zip(sizes, plain)]
+    batch = _core.BatchedCircuits(dqsim.StatevectorSimulator(seed=3), measured, shots=200)
+    batch.run()
+    for i, (n, _) in enumerate(sizes):
+        want = oracle_state(plain[i])
+        assert np.max(np.abs(dqsim.StatevectorSimulator(seed=1).simulate(plain[i]).statevector - want)) <= 1e-12
+        assert np.max(np.abs(batch.statevector(i, n) - want)) <= 1e-12
+        seed = (3 + i * _core.BATCH_SEED_STRIDE) % (1 << 64)
+        counts = o.OracleSimulator(seed=seed).simulate_shots(measured[i], shots=200)
+        assert dqsim.StatevectorSimulator(seed=seed).simulate_shots(measured[i], shots=200) == counts
+        assert batch.counts(i) == counts
