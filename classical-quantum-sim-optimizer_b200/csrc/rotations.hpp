@@ -119,7 +119,7 @@ int rotation_pinned_low(const std::vector<Operation>& ops, size_t begin, size_t 
 // Targets and swapped qubits are tile qubits; controls and diagonal qubits may
 // lie outside, where the tile's index gives their value.  False when an
 // operation has no such form (a dense matrix that is no Pauli rotation, a matrix
-// that is not unitary to 1e-12) or the tile is too small or large.
+// further from a unitary one than its entries' rounding) or the tile is too small or large.
 bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<int>& tile_qubits, int n,
                          RotProgram& out);
 

@@ -371,3 +371,56 @@ def test_mixed_rotations_on_the_device(kinds, two):
         counts = o.OracleSimulator(seed=seed).simulate_shots(measured[i], shots=200)
         assert dqsim.StatevectorSimulator(seed=seed).simulate_shots(measured[i], shots=200) == counts
         assert batch.counts(i) == counts
+
+
+def product_of_entries(c):
+    """The gates' double entries applied in long double."""
+    n = c.data["qregs"]["q"]["size"]
+    r = 0.7071067811865476
+    psi = np.zeros(1 << n, dtype=np.clongdouble)
+    psi[0] = 1
+    for op in c.data["instructions"]:
+        if op["kind"] in ("cx", "cz"):
+            i = np.arange(1 << n)
+            held = ((i >> op["control"]) & 1) == 1
+            psi = (psi[np.where(held, i ^ (1 << op["target"]), i)] if op["kind"] == "cx" else
+                   np.where(held & (((i >> op["target"]) & 1) == 1), -psi, psi))
+            continue
+        half = op.get("theta", op.get("phi", 0.0)) / 2
+        co, si = np.cos(half), np.sin(half)
+        m = {"h": [[r, r], [r, -r]], "ry": [[co, -si], [si, co]],
+             "rz": [[complex(co, -si), 0], [0, complex(co, si)]]}[op["kind"]]
+        v = psi.reshape(1 << (n - 1 - op["qubit"]), 2, 1 << op["qubit"])
+        x, y = v[:, 0].copy(), v[:, 1].copy()
+        v[:, 0] = np.clongdouble(m[0][0]) * x + np.clongdouble(m[0][1]) * y
+        v[:, 1] = np.clongdouble(m[1][0]) * x + np.clongdouble(m[1][1]) * y
+    return psi
+
+
+@pytest.mark.parametrize("gate", [{"kind": "h"}], ids=lambda g: g["kind"])
+def test_the_scale_of_rounded_entries_is_kept(gate):
+    """2,400 times one gate, whose entries' norm is 7e-17 (H) off one: 1.6e-13 in all.
+    The rounding of 2,400 gates (three roundings of 1.1e-16, signs at random) is some 1.6e-14."""
+    n = 12
+    ins = []
+    for layer in range(200):
+        ins += [inst(gate["kind"], qubit=q, **{k: v for k, v in gate.items() if k != "kind"}) for q in range(n)]
+        ins += [inst("cx", control=q, target=q + 1) for q in range(layer % 2, n - 1, 2)]
+    c = Circuit(n, ins)
+    got = replay(_core.rotation_plan_dump(c.model_dump_json(), n))
+    assert np.linalg.norm((got - product_of_entries(c)).astype(np.complex128)) <= 4e-14
+
+
+# A U3 whose angles' sum is rounded to 1e-11: its entries are 1e-12 from a unitary matrix.
+FAR = [inst("ry", qubit=0, theta=0.77), inst("cx", control=0, target=1),
+       inst("u3", qubit=0, theta=-1.348, phi=1e-12, lam=98103.878)]
+
+
+def test_matrices_further_from_unitary_than_rounding_have_no_rotation_form():
+    assert not any(p["ok"] for p in _core.rotation_plan_dump(Circuit(5, FAR).model_dump_json(), 5)["passes"])
+
+
+@pytest.mark.gpu
+def test_matrices_further_from_unitary_than_rounding_are_applied_as_they_are():
+    c = Circuit(5, FAR)
+    assert np.max(np.abs(dqsim.StatevectorSimulator(seed=1).simulate(c).statevector - oracle_state(c))) <= 1e-15
