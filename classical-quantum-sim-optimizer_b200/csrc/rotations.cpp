@@ -935,6 +935,33 @@ class Scheduler {
                 }
                 b->second.push_back(i);
             }
+            // The slots' data first: what its rounding misses on average is settled by the table.
+            struct SlotStep {
+                uint32_t parity, kind;
+                std::vector<int> terms;
+                std::vector<uint4> factors;
+            };
+            std::vector<SlotStep> steps;
+            for (auto& b : by) {
+                SlotStep angles{b.first, kRotSlots, {}, {}}, moduli{b.first, kRotSlotModuli, {}, {}};
+                for (int i : b.second) {
+                    const Item& x = *it[size_t(i)];
+                    if (x.a != 0.0) {
+                        ld off[2] = {};
+                        angles.terms.push_back(i);
+                        angles.factors.push_back(factor_word(factor(0.0L, x.a), off));
+                        uniform_ -= off[0];
+                    }
+                    if (x.b != 0.0) {
+                        const ld up = std::exp(x.b), down = std::exp(-x.b);
+                        moduli.terms.push_back(i);
+                        moduli.factors.push_back(word(double(up), double(down)));
+                        uniform_ -= 0.5L * ((double(up) - up) / up + (double(down) - down) / down);
+                    }
+                }
+                if (!angles.terms.empty()) steps.push_back(std::move(angles));
+                if (!moduli.terms.empty()) steps.push_back(std::move(moduli));
+            }
             ld G = 0.0;
             if (final) {
                 G = std::remainder(lw_.global, 2 * kPiL);
@@ -944,44 +971,24 @@ class Scheduler {
                 table = table || uniform_ != 0.0;
             }
             if (table) emit_table(here, G);
-            for (auto& b : by) {
-                const std::vector<int>& terms = b.second;
-                auto part_of = [&](uint32_t kind, const std::vector<int>& t) {
-                    Part part;
-                    part.place = 6;
-                    part.kind = kind;
-                    part.signs = signs(b.first);
-                    part.data = uint32_t(tables_.size());
-                    part.count = uint32_t(t.size());
-                    parts_.push_back(part);
-                    for (size_t i = 0; i < t.size(); i += 4) {
-                        uint32_t m4[4] = {};
-                        for (size_t j = i; j < std::min(t.size(), i + 4); j++) m4[j - i] = slots(it[size_t(t[j])]->mask);
-                        tables_.push_back(word(m4[0], m4[1], m4[2], m4[3]));
-                    }
-                };
-                std::vector<int> angles, moduli;
-                for (int i : terms) {
-                    if (it[size_t(i)]->a != 0.0) angles.push_back(i);
-                    if (it[size_t(i)]->b != 0.0) moduli.push_back(i);
+            for (const SlotStep& step : steps) {
+                const size_t count = step.terms.size();
+                Part part;
+                part.place = 6;
+                part.kind = step.kind;
+                part.signs = signs(step.parity);
+                part.data = uint32_t(tables_.size());
+                part.count = uint32_t(count);
+                parts_.push_back(part);
+                for (size_t i = 0; i < count; i += 4) {
+                    uint32_t m4[4] = {};
+                    for (size_t j = i; j < std::min(count, i + 4); j++) m4[j - i] = slots(it[size_t(step.terms[j])]->mask);
+                    tables_.push_back(word(m4[0], m4[1], m4[2], m4[3]));
                 }
-                if (!angles.empty()) {
-                    part_of(kRotSlots, angles);
-                    ld off[2] = {};
-                    for (int i : angles) tables_.push_back(factor_word(factor(0.0L, it[size_t(i)]->a), off));
-                    uniform_ -= off[0];
-                    out_.slot_phases++;
-                    fma_ += 6.0 + 6.0 * double(angles.size()) / kRotEntries;
-                }
-                if (!moduli.empty()) {
-                    part_of(kRotSlotModuli, moduli);
-                    for (int i : moduli) {
-                        const ld x = it[size_t(i)]->b;
-                        tables_.push_back(word(double(std::exp(x)), double(std::exp(-x))));
-                    }
-                    out_.slot_phases++;
-                    fma_ += 2.0 + 2.0 * double(moduli.size()) / kRotEntries;
-                }
+                tables_.insert(tables_.end(), step.factors.begin(), step.factors.end());
+                out_.slot_phases++;
+                const double each = step.kind == kRotSlots ? 6.0 : 2.0;
+                fma_ += each + each * double(count) / kRotEntries;
             }
         };
         // The coordinate functional of register bit j: a mask that vanishes on the slots.
@@ -1041,7 +1048,7 @@ class Scheduler {
                     }
                 if (part.kind == kRotKept) {
                     part.u = double(1.0L + ld(x.t) * x.t);
-                    uniform_ -= lost;
+                    uniform_ -= 0.5L * std::log(ld(part.u));  // the pair's determinant as it is rounded
                 } else {
                     pend[low] -= lost;
                 }

@@ -397,9 +397,9 @@ def product_of_entries(c):
     return psi
 
 
-@pytest.mark.parametrize("gate", [{"kind": "h"}], ids=lambda g: g["kind"])
+@pytest.mark.parametrize("gate", [{"kind": "h"}, {"kind": "ry", "theta": 0.3}], ids=lambda g: g["kind"])
 def test_the_scale_of_rounded_entries_is_kept(gate):
-    """2,400 times one gate, whose entries' norm is 7e-17 (H) off one: 1.6e-13 in all.
+    """2,400 times one gate, whose entries' norm is 7e-17 (H) and 5e-17 (RY) off one: 1.6e-13 and 1.2e-13 in all.
     The rounding of 2,400 gates (three roundings of 1.1e-16, signs at random) is some 1.6e-14."""
     n = 12
     ins = []
