@@ -23,6 +23,7 @@ constexpr ld kUnitaryTol = 2e-15L;
 constexpr ld kScaleTol = 1e-12L;  // a scale further from one is no rounding
 // No turn, or a quarter turn, to the rounding of the product of matrices that gives it.
 constexpr ld kAngleTol = 1.2e-16L;
+constexpr ld kExactTol = 1e-18L;  // the same, to the rounding of the numbers here
 constexpr int kMaxDiagQubits = 6;
 
 int parity64(uint64_t x) { return __builtin_parityll(x); }
@@ -101,6 +102,12 @@ bool mean_modulus(const std::vector<cplx>& values, ld& mean) {
     return true;
 }
 
+// x + a, kept below a turn: a sum of 1,000 angles would lose 2e-14 to its own size.
+void turn(ld& x, ld a) {
+    x += a;
+    if (std::fabs(x) > kPiL) x = std::remainder(x, 2 * kPiL);
+}
+
 // The gates of a pass as items, with the frame that relabels places.
 class Lowering {
   public:
@@ -132,7 +139,6 @@ class Lowering {
     }
 
     std::vector<Item> items;
-    // Sums hundreds of angles: a 64-bit mantissa keeps its rounding below the amplitudes'.
     ld global = 0.0;           // phase of the whole state
     ld norm = 0.0;             // logarithm of a modulus of the whole state
     uint64_t sign = 0;         // Z^sign still to be applied
@@ -148,25 +154,25 @@ class Lowering {
     std::vector<uint32_t> dir_;
     std::vector<size_t> open_;  // phases that every later rotation commutes with
 
-    // exp(i a Z^mask (-1)^cons)
-    void phase(uint64_t mask, int cons, ld a) {
+    // exp(i a Z^mask (-1)^cons); `tol`: what an angle may be off a multiple of pi/2 and count as one.
+    void phase(uint64_t mask, int cons, ld a, ld tol = kExactTol) {
         if (cons) a = -a;
         if (mask == 0) {
-            global += a;
+            turn(global, a);
             return;
         }
         const ld r = std::nearbyint(a / kPiL);
         a -= r * kPiL;
-        if (std::fmod(std::fabs(r), 2.0L) == 1.0L) global += kPiL;
-        if (std::fabs(a) <= kAngleTol) return;
-        if (std::fabs(std::fabs(a) - kPiL / 2) <= kAngleTol) {  // +-i Z^mask
-            global += a > 0 ? kPiL / 2 : -kPiL / 2;
+        if (std::fmod(std::fabs(r), 2.0L) == 1.0L) turn(global, kPiL);
+        if (std::fabs(a) <= tol) return;
+        if (std::fabs(std::fabs(a) - kPiL / 2) <= tol) {  // +-i Z^mask
+            turn(global, a > 0 ? kPiL / 2 : -kPiL / 2);
             sign ^= mask;
             return;
         }
         for (size_t i : open_)
             if (items[i].mask == mask) {
-                items[i].a += a;
+                turn(items[i].a, a);
                 return;
             }
         Item it;
@@ -194,7 +200,7 @@ class Lowering {
         const bool imag = ny % 2 == 0;
         if ((ny / 2) % 2) cons ^= 1;  // i^ny = +-1 or +-i
         if (c < 0) {
-            global += kPiL;
+            turn(global, kPiL);
             c = -c;
             s = -s;
         }
@@ -205,12 +211,12 @@ class Lowering {
             // (the phases and rotations before see the place, so P comes last).
             ld c2 = s, s2 = -c;
             if (c2 < 0) {
-                global += kPiL;
+                turn(global, kPiL);
                 c2 = -c2;
                 s2 = -s2;
             }
             if (s2 != 0.0) emit(v, mask, imag, c2, s2);
-            if (imag) global -= kPiL / 2;
+            if (imag) turn(global, -(kPiL / 2));
             sign ^= mask;
             for (size_t q = 0; q < mask_.size(); q++) cons_[q] ^= parity64(mask_[q] & v);
             return;
@@ -298,20 +304,20 @@ class Lowering {
         const ld beta = B - A, gamma = D - B, alpha = A + (beta + gamma) / 2;
         norm += p.scale / ld(size_t(1) << controls.size());  // where controls hold only: its mean
         if (controls.empty()) {
-            global += alpha;
+            turn(global, alpha);
             // RZ(-+pi/2) RY(theta) RZ(+-pi/2) = RX(+-theta)
             const ld turns = std::nearbyint((beta + gamma) / (2 * kPiL));
             const ld quarter = std::fabs(std::remainder(beta, 2 * kPiL));
             if (s > 0 && std::fabs(beta + gamma - turns * 2 * kPiL) <= kAngleTol &&
                 std::fabs(quarter - kPiL / 2) <= kAngleTol) {
                 // RZ(gamma) = RZ(-beta) (-1)^turns; beta = +-pi/2 up to whole turns, which cancel in the pair.
-                if (std::fmod(std::fabs(turns), 2.0L) == 1.0L) global += kPiL;
+                if (std::fmod(std::fabs(turns), 2.0L) == 1.0L) turn(global, kPiL);
                 rotation({target}, {}, c, std::remainder(beta, 2 * kPiL) < 0 ? s : -s);
                 return;
             }
-            phase(mask_[size_t(target)], cons_[size_t(target)], -gamma / 2);
+            phase(mask_[size_t(target)], cons_[size_t(target)], -gamma / 2, kAngleTol);
             rotation({target}, {target}, c, s);
-            phase(mask_[size_t(target)], cons_[size_t(target)], -beta / 2);
+            phase(mask_[size_t(target)], cons_[size_t(target)], -beta / 2, kAngleTol);
             return;
         }
         std::vector<uint64_t> q;
@@ -355,7 +361,7 @@ class Lowering {
             const ld r = std::sqrt(0.5L);
             auto h = [&] {  // H = RY(pi/2) Z
                 phase(mask_[size_t(target)], cons_[size_t(target)], -kPiL / 2);  // -i Z
-                global += kPiL / 2;
+                turn(global, kPiL / 2);
                 rotation({target}, {target}, r, r);
             };
             h();

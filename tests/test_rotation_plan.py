@@ -411,6 +411,16 @@ def test_the_scale_of_rounded_entries_is_kept(gate):
     assert np.linalg.norm((got - product_of_entries(c)).astype(np.complex128)) <= 4e-14
 
 
+def test_angles_below_the_rounding_of_one_add_up():
+    """1,000 turns of 2e-16 with gates between that keep them apart: 1e-13 in an amplitude."""
+    ins = [inst("h", qubit=q) for q in range(5)]
+    for k in range(1000):
+        ins += [inst("rz", qubit=0, phi=2e-16), inst("cz", control=0, target=1 + k % 4)]
+    c = Circuit(5, ins)
+    got = replay(_core.rotation_plan_dump(c.model_dump_json(), 5))
+    assert np.max(np.abs(got - product_of_entries(c))) <= 2e-15
+
+
 # A U3 whose angles' sum is rounded to 1e-11: its entries are 1e-12 from a unitary matrix.
 FAR = [inst("ry", qubit=0, theta=0.77), inst("cx", control=0, target=1),
        inst("u3", qubit=0, theta=-1.348, phi=1e-12, lam=98103.878)]
