@@ -271,11 +271,17 @@ Device::Device(int ord) : ordinal(ord) {
 }
 
 void* Device::take_block(size_t bytes) {
-    std::lock_guard<std::mutex> l(block_mu_);
-    if (!block_ || block_bytes_ != bytes) return nullptr;
-    void* p = block_;
-    block_ = nullptr;
-    return p;
+    void* p = nullptr;
+    bool fits = false;
+    {
+        std::lock_guard<std::mutex> l(block_mu_);
+        p = block_;
+        fits = p && block_bytes_ == bytes;
+        block_ = nullptr;
+    }
+    if (fits) return p;
+    if (p) cudaFree(p);  // before the new one is made: the two are never held together
+    return nullptr;
 }
 
 void Device::keep_block(void* p, size_t bytes) {

