@@ -689,6 +689,9 @@ void BatchRun::enqueue(bool capturing) {
     if (capturing && sides_ > 0) {
         std::vector<cudaGraphNode_t> all = chains.at();
         for (const auto& t : tails) all.insert(all.end(), t.begin(), t.end());
+        // (a circuit without gates leaves its chain at the fork: each node counts once)
+        std::sort(all.begin(), all.end());
+        all.erase(std::unique(all.begin(), all.end()), all.end());
         chains.go(all);
     } else if (sides_ > 0) {
         for (cudaEvent_t e : join_) cuda_check(cudaStreamWaitEvent(s, e, 0), "join");

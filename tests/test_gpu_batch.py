@@ -110,3 +110,27 @@ def test_tensor_core_batch_matches_oracle_and_replays_identically():
         b.run(use_graph=True)
     assert [b.counts(i) for i in range(len(cs))] == direct
     np.testing.assert_array_equal(b.expect_zz(), zz)
+
+
+@pytest.mark.parametrize("precision", ["complex128", "complex64"])
+@pytest.mark.parametrize("sizes", [[6], [6, 13, 5], [13, 12]])
+@pytest.mark.parametrize("gates", [False, True])
+def test_circuits_without_gates(sizes, gates, precision):
+    """Measurements only, alone or beside a circuit with gates, launched directly and as a graph."""
+    cs = [workloads.TransportCircuit(n, [{"kind": "measure", "qubit": q, "cbit": q} for q in range(n)], n) for n in sizes]
+    if gates:
+        cs.insert(1, workloads.hea(13, 3, seed=2, measure=True))
+    b = _core.BatchedCircuits(dqsim.StatevectorSimulator(seed=4, precision=precision), cs, shots=100,
+                              tensor_cores=precision == "complex64")
+    for use_graph in (False, True):
+        b.run(use_graph=use_graph)
+        zz = b.expect_zz()
+        for i, c in enumerate(cs):
+            n = c.num_qubits
+            if len(c.data["instructions"]) == n:
+                assert zz[i] == 1.0
+                assert b.counts(i) == {"0" * n: 100}
+            else:
+                want = zz_of(b.statevector(i, n))
+                assert abs(zz[i] - want) <= (1e-12 if precision == "complex128" else 1e-6)
+                assert sum(b.counts(i).values()) == 100
