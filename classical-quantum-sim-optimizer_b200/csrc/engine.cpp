@@ -335,32 +335,42 @@ void Device::activate() const { cuda_check(cudaSetDevice(ordinal), "cudaSetDevic
 void Device::sync() { cuda_check(cudaStreamSynchronize(stream), "stream synchronize"); }
 
 void StateBatch::allocate(int n_, uint64_t W_, uint64_t ncb_, bool c64_, Device& d) {
-    amps.alloc_cached((size_t(W_) << n_) * (c64_ ? 8 : 16), d, "the statevector");
-    allocate(n_, W_, ncb_, c64_, d.stream);
+    shape(n_, W_, ncb_, c64_);
+    amps.alloc_cached((size_t(W) << n) * (c64 ? 8 : 16), d, "the statevector");
+    allocate_rest(d.stream);
 }
 
 void StateBatch::allocate(int n_, uint64_t W_, uint64_t ncb_, bool c64_, cudaStream_t pool_stream) {
+    shape(n_, W_, ncb_, c64_);
+    get(amps, (size_t(W) << n) * (c64 ? 8 : 16), pool_stream, "the statevector");
+    allocate_rest(pool_stream);
+}
+
+void StateBatch::shape(int n_, uint64_t W_, uint64_t ncb_, bool c64_) {
     n = n_;
     W = W_;
     ncb = ncb_;
     c64 = c64_;
     cwords = int(std::max<uint64_t>(1, (ncb + 63) / 64));
-    // With a stream, every buffer comes from the engine's pool: freeing them
-    // is stream-ordered and never waits for the device.
-    auto get = [&](DevMem& m, size_t bytes, const char* what) {
-        if (pool_stream)
-            m.alloc_on(bytes, pool_stream, what);
-        else
-            m.alloc(bytes, what);
-    };
-    if (!amps.home) get(amps, (size_t(W) << n) * (c64 ? 8 : 16), "the statevector");
-    get(cbits, size_t(W) * cwords * 8, "classical bits");
-    get(seeds, size_t(W) * 8, "rng seeds");
-    get(draws, size_t(W) * 8, "rng counters");
-    get(outcome, size_t(W) * 4, "measurement outcomes");
-    get(scale, size_t(W) * 8, "measurement scales");
-    get(partial, size_t(W) * k::kMaxChunks * 2 * 8, "measurement partial sums");
-    get(err, 16, "error flag");
+}
+
+// With a stream, every buffer comes from the engine's pool: freeing them
+// is stream-ordered and never waits for the device.
+void StateBatch::get(DevMem& m, size_t bytes, cudaStream_t pool_stream, const char* what) {
+    if (pool_stream)
+        m.alloc_on(bytes, pool_stream, what);
+    else
+        m.alloc(bytes, what);
+}
+
+void StateBatch::allocate_rest(cudaStream_t s) {
+    get(cbits, size_t(W) * cwords * 8, s, "classical bits");
+    get(seeds, size_t(W) * 8, s, "rng seeds");
+    get(draws, size_t(W) * 8, s, "rng counters");
+    get(outcome, size_t(W) * 4, s, "measurement outcomes");
+    get(scale, size_t(W) * 8, s, "measurement scales");
+    get(partial, size_t(W) * k::kMaxChunks * 2 * 8, s, "measurement partial sums");
+    get(err, 16, s, "error flag");
 }
 
 k::Batch StateBatch::view(cudaStream_t s, uint64_t W_active) const {

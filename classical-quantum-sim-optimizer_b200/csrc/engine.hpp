@@ -94,6 +94,11 @@ struct StateBatch {
     void allocate(int n, uint64_t W, uint64_t ncb, bool c64, Device& d);
     k::Batch view(cudaStream_t s, uint64_t W_active) const;
     size_t amp_bytes() const { return size_t(1) << n; }
+
+  private:
+    void shape(int n, uint64_t W, uint64_t ncb, bool c64);
+    void allocate_rest(cudaStream_t pool_stream);  // all but the statevector
+    static void get(DevMem& m, size_t bytes, cudaStream_t pool_stream, const char* what);
 };
 
 struct ProfileAcc {
