@@ -20,13 +20,13 @@ constexpr size_t kMaxTileBytes = size_t(1) << 17;  // 14 tile qubits of complex6
 // 0.97 and 0.21 ms; 256 circuits of 12-22 qubits 11.7 and 11.5 ms).
 constexpr size_t kSideStreams = 64;
 // Tile groups a CTA of a fused pass takes at least, for circuits of at least
-// kShareQuads groups in a batch of at least kFullQuads: there the passes of
+// kShareQuads groups in a batch of at least kFullQuads to an SM: there the passes of
 // other circuits fill the device and a CTA's set-up is worth sharing (256
 // circuits of 12-22 qubits 11.5 ms at 1, 10.6 at 3, 10.9 at 4); where they do
 // not, fewer CTAs only take longer (12 circuits of 12-20 qubits 0.31 ms at 1,
 // 0.60 at 3).
 constexpr int kShare = 3;
-constexpr uint64_t kShareQuads = 32, kFullQuads = 148 * 8;
+constexpr uint64_t kShareQuads = 32, kFullQuads = 8;
 // Spin limit of one dependency wait: 2^24 polls of >= 256 ns, several seconds.
 constexpr uint64_t kMaxSpins = uint64_t(1) << 24;
 
@@ -323,13 +323,6 @@ __global__ void k_seg_sample(const double* __restrict__ scan, const double* __re
     out[g] = idx < e - b - 1 ? idx : e - b - 1;
 }
 
-int sm_count() {
-    int dev = 0, c = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    return c > 0 ? c : 148;
-}
-
 }  // namespace
 
 BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64_t shots, const BatchTuning& tuning)
@@ -548,7 +541,7 @@ k::Batch BatchRun::circuit_view(const Circ& c, cudaStream_t s) const {
     b.W = 1;
     b.err = err_.as<int>();
     const uint64_t quads = c.n > uint64_t(kFusedM) ? uint64_t(1) << (c.n - kFusedM) >> 2 : 1;
-    if (fused_quads_ >= kFullQuads && quads >= kShareQuads) b.fused_quads = kShare;
+    if (fused_quads_ >= kFullQuads * uint64_t(k::sm_count()) && quads >= kShareQuads) b.fused_quads = kShare;
     return b;
 }
 
@@ -672,7 +665,7 @@ void BatchRun::enqueue(bool capturing) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<double2>, kBatchThreads, smem);
     if (per_sm < 1) per_sm = 1;
     // Every CTA is resident at once, so a claimed item never waits on an unclaimed one.
-    const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(total_items_, uint64_t(sm_count()) * per_sm)));
+    const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(total_items_, uint64_t(k::sm_count()) * per_sm)));
     if (total_items_ > 0) {
         if (c64_)
             k_batch<float2><<<grid, kBatchThreads, smem, s>>>(amps_.as<float2>(), recs_.as<PassRec>(),

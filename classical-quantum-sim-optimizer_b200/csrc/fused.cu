@@ -665,13 +665,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-int sm_count() {
-    int dev = 0, c = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    return c > 0 ? c : 148;
-}
-
 // Tile norms per partial: block (state st, part p) sums tiles
 // [p * kNormChunk, (p + 1) * kNormChunk) of state st in a fixed order, so the
 // state's norm (the sum of its parts in order) is the same on every run.

@@ -1039,6 +1039,13 @@ void measure(const Batch& b, int qubit, int64_t cbit, bool reset, const CondList
         measure_t<double2>(b, qubit, cbit, reset, cond);
 }
 
+int sm_count() {
+    int dev = 0, c = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+    return c > 0 ? c : 148;
+}
+
 int measure_chain_max() { return kChainMax; }
 
 bool measure_chain_applies(const Batch& b, int count) {
@@ -1046,7 +1053,7 @@ bool measure_chain_applies(const Batch& b, int count) {
     // at about 60 GB/s, up to four a SM at a time; separate measurements take three
     // launches and 2.5 passes at 5.5 TB/s.
     const double bytes = double(uint64_t(1) << b.n) * (b.c64 ? 8.0 : 16.0);
-    const double rounds = std::ceil(double(b.W) / 592.0);
+    const double rounds = std::ceil(double(b.W) / (4.0 * sm_count()));
     const double chain = 4.0 + 1.5 * count + rounds * 3.0 * bytes / 60e3;
     const double separate = count * (12.0 + 2.5 * bytes * double(b.W) / 5.5e6);
     return chain < separate && b.W <= 0x7fffffffULL;

@@ -40,6 +40,9 @@ struct Batch {
 
 constexpr int kMaxChunks = 1024;
 
+// SMs of the current device.
+int sm_count();
+
 struct Ctl {
     int qubit;
     bool value;

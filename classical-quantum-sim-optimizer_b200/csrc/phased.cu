@@ -578,17 +578,6 @@ __global__ void __launch_bounds__(kPhaseThreads, phase_min_ctas<V>())
     phased_body<V>(s, n, m, tq, nphases, total_tiles, ArgWords{&args});
 }
 
-int sm_count() {
-    static int c = 0;
-    if (!c) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-        if (c <= 0) c = 148;
-    }
-    return c;
-}
-
 template <typename Kernel>
 uint64_t configure(Kernel kernel, size_t smem, size_t& configured, uint64_t total) {
     if (smem > configured) {

@@ -1603,17 +1603,6 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_tile(V* __restrict__ s, int
     }
 }
 
-int sm_count() {
-    static int c = 0;
-    if (!c) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-        if (c <= 0) c = 148;
-    }
-    return c;
-}
-
 template <typename V, bool TIMED>
 void tile_pass_t(const Batch& b, int m, const TileOp* ops, int nops, const double2* pool, const TilePass& hp,
                  unsigned long long* cycles) {
