@@ -697,14 +697,6 @@ __global__ void k_scan_add(double* __restrict__ x, uint64_t len, const double* _
     }
 }
 
-__global__ void k_cdf_normalize(double* __restrict__ cdf, uint64_t len, double total, int clamp) {
-    for (uint64_t g = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < len; g += uint64_t(gridDim.x) * blockDim.x) {
-        double v = cdf[g] / total;
-        if (clamp) v = fmin(v, 1.0);
-        cdf[g] = (g == len - 1) ? 1.0 : v;
-    }
-}
-
 // Entry i of running sums kept in two levels: tile-local sums x plus the
 // inclusive sums of whole tiles before it (the same addition k_scan_add makes).
 __device__ __forceinline__ double two_level(const double* __restrict__ x, const double* __restrict__ tiles,
@@ -721,38 +713,22 @@ __global__ void k_take_total(const double* __restrict__ cdf, uint64_t len, const
     if (!(isfinite(t) && t > 0.0)) *err = 1;
 }
 
-__global__ void k_cdf_normalize_dev(double* __restrict__ cdf, uint64_t len, const double* __restrict__ scalar,
-                                    int clamp) {
-    const double total = *scalar;
-    for (uint64_t g = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < len; g += uint64_t(gridDim.x) * blockDim.x) {
-        double v = cdf[g] / total;
-        if (clamp) v = fmin(v, 1.0);
-        cdf[g] = (g == len - 1) ? 1.0 : v;
-    }
-}
-
-// With `total` (device scalar, or host value when total_dev is null and
-// total_host > 0) the table holds the unnormalised running sums and each
-// probe normalises the entry it reads exactly as k_cdf_normalize would have
-// stored it (cdf[i] / total, clamped to 1 when clamp, the last entry 1).
+// The table holds unnormalised running sums; each probe normalises the entry it
+// reads (by the total, clamped to 1 when clamp, the last entry 1).
 __global__ void k_sample(const double* __restrict__ cdf, uint64_t len, uint64_t seed, uint64_t shots, int per_shot,
-                         const double* __restrict__ tiles, const double* __restrict__ total_dev, double total_host,
-                         int clamp, uint64_t* __restrict__ out) {
+                         const double* __restrict__ tiles, const double* __restrict__ total_dev, int clamp,
+                         uint64_t* __restrict__ out) {
     uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= shots) return;
-    const bool scaled = total_dev != nullptr || total_host > 0.0;
-    const double total = total_dev ? *total_dev : total_host;
+    const double total = *total_dev;
     uint64_t v = per_shot ? dev::chacha8_u64(seed + t, 0) : dev::chacha8_u64(seed, t);
     double draw = dev::u64_to_unit(v);
     uint64_t lo = 0, hi = len;
     while (lo < hi) {
         uint64_t mid = lo + (hi - lo) / 2;
-        double c = two_level(cdf, tiles, mid);
-        if (scaled) {
-            c = c / total;
-            if (clamp) c = fmin(c, 1.0);
-            if (mid == len - 1) c = 1.0;
-        }
+        double c = two_level(cdf, tiles, mid) / total;
+        if (clamp) c = fmin(c, 1.0);
+        if (mid == len - 1) c = 1.0;
         if (c <= draw)
             lo = mid + 1;
         else
@@ -1246,37 +1222,16 @@ void scan_states(cudaStream_t s, bool c64, const void* amps, uint64_t len, doubl
     if (nb > 1) scan(s, tmp, nb, tmp + nb);
 }
 
-uint64_t scan_tile_of(uint64_t i) { return i / uint64_t(kScanTile); }
-
 void take_total(cudaStream_t s, const double* cdf, uint64_t len, const double* tiles, double* scalar, int* err) {
     k_take_total<<<1, 1, 0, s>>>(cdf, len, tiles, scalar, err);
     check_launch("take_total");
 }
 
-void cdf_normalize(cudaStream_t s, double* cdf, uint64_t len, double total, bool clamp) {
-    k_cdf_normalize<<<stream_grid(len), 256, 0, s>>>(cdf, len, total, clamp ? 1 : 0);
-    check_launch("cdf_normalize");
-}
-
-void cdf_normalize_device(cudaStream_t s, double* cdf, uint64_t len, double* scalar, int* err, bool clamp) {
-    k_take_total<<<1, 1, 0, s>>>(cdf, len, nullptr, scalar, err);
-    k_cdf_normalize_dev<<<stream_grid(len), 256, 0, s>>>(cdf, len, scalar, clamp ? 1 : 0);
-    check_launch("cdf_normalize_device");
-}
-
-void sample(cudaStream_t s, const double* cdf, uint64_t len, uint64_t seed, uint64_t shots, bool per_shot_seed,
-            uint64_t* out) {
-    if (shots == 0) return;
-    k_sample<<<blocks_for(shots, 128), 128, 0, s>>>(cdf, len, seed, shots, per_shot_seed ? 1 : 0, nullptr, nullptr,
-                                                     0.0, 0, out);
-    check_launch("sample");
-}
-
 void sample_sums(cudaStream_t s, const double* sums, const double* tiles, uint64_t len, const double* total_dev,
-                 double total_host, bool clamp, uint64_t seed, uint64_t shots, bool per_shot_seed, uint64_t* out) {
+                 bool clamp, uint64_t seed, uint64_t shots, bool per_shot_seed, uint64_t* out) {
     if (shots == 0) return;
     k_sample<<<blocks_for(shots, 128), 128, 0, s>>>(sums, len, seed, shots, per_shot_seed ? 1 : 0, tiles, total_dev,
-                                                     total_host, clamp ? 1 : 0, out);
+                                                     clamp ? 1 : 0, out);
     check_launch("sample");
 }
 

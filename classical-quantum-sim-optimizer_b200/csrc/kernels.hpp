@@ -100,22 +100,14 @@ size_t scan_tmp_size(uint64_t len);
 // Kernel launches scan (and scan_probs) makes for `len` entries.
 int scan_launches(uint64_t len);
 void scan(cudaStream_t s, double* x, uint64_t len, double* tmp);
-// cdf[i] = cdf[i] / total (clamped to 1 when clamp), cdf[len-1] = 1.
-void cdf_normalize(cudaStream_t s, double* cdf, uint64_t len, double total, bool clamp);
-// Same with the total taken from cdf[len-1] on the device (copied to `scalar`
-// first); sets *err when the total is not finite and positive.
-void cdf_normalize_device(cudaStream_t s, double* cdf, uint64_t len, double* scalar, int* err, bool clamp);
-// out[t] = min(partition_point(cdf, draw_t), len-1); per_shot_seed: draw_t is the
-// first draw of seed+t, otherwise draw t of the stream `seed`.
-void sample(cudaStream_t s, const double* cdf, uint64_t len, uint64_t seed, uint64_t shots, bool per_shot_seed,
-            uint64_t* out);
-// The same over unnormalised running sums: every probe normalises the entry it
-// reads exactly as cdf_normalize would have (by *total_dev when given, else by
-// total_host), so no normalising pass over the table is needed.  With `tiles`
-// the sums are in two levels (scan_local): entry i is sums[i] plus
+// out[t] = min(partition_point(cdf, draw_t), len-1) over unnormalised running
+// sums: every probe normalises the entry it reads (sums[i] / *total_dev, clamped
+// to 1 when clamp, the last entry 1), so no pass over the table does.  per_shot_seed:
+// draw_t is the first draw of seed+t, otherwise draw t of the stream `seed`.  With
+// `tiles` the sums are in two levels (scan_local): entry i is sums[i] plus
 // tiles[i / 2048 - 1], the addition scan would have stored.
 void sample_sums(cudaStream_t s, const double* sums, const double* tiles, uint64_t len, const double* total_dev,
-                 double total_host, bool clamp, uint64_t seed, uint64_t shots, bool per_shot_seed, uint64_t* out);
+                 bool clamp, uint64_t seed, uint64_t shots, bool per_shot_seed, uint64_t* out);
 // Inclusive running sums of state 0's squared magnitudes (in index order, the
 // same values as norm2 then scan) into x; `tmp` needs scan_tmp_size(2^n)
 // doubles.  add_tiles = false leaves them in two levels (see scan_local).
@@ -127,7 +119,6 @@ void scan_local(cudaStream_t s, double* x, uint64_t len, double* tmp);
 constexpr int kScanTileEntries = 2048;
 // scan_local of the squared magnitudes of `len` amplitudes (any number).
 void scan_states(cudaStream_t s, bool c64, const void* amps, uint64_t len, double* x, double* tmp);
-uint64_t scan_tile_of(uint64_t i);
 // *scalar = entry len-1 of the (two-level when tiles) sums; *err = 1 when it is
 // not finite and positive.
 void take_total(cudaStream_t s, const double* cdf, uint64_t len, const double* tiles, double* scalar, int* err);

@@ -142,7 +142,7 @@ double Plan::run(bool record) {
             k::scan_local(s, cdf_.as<double>(), clen, tmp_.as<double>());
         }
         k::take_total(s, cdf_.as<double>(), clen, tmp_.as<double>(), scalar_.as<double>(), st_.err.as<int>());
-        k::sample_sums(s, cdf_.as<double>(), tmp_.as<double>(), clen, scalar_.as<double>(), 0.0, false, seed_,
+        k::sample_sums(s, cdf_.as<double>(), tmp_.as<double>(), clen, scalar_.as<double>(), false, seed_,
                        shots_, true, idx_.as<uint64_t>());
         if (record) rec.end();
     }

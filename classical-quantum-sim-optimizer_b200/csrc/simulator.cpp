@@ -343,7 +343,7 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
                 cuda_check(cudaEventRecord(ev[1], s), "cudaEventRecord");
                 phase(kPhRun);
                 build_sums(b, qubits, cdf.as<double>(), clen, tmp, total_dev);
-                k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), clen, &total_dev->total, 0.0, false, seed, shots,
+                k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), clen, &total_dev->total, false, seed, shots,
                                true, idx.as<uint64_t>());
                 cuda_check(cudaEventSynchronize(ev[1]), "cudaEventSynchronize");
                 phase(kPhSums);
@@ -585,7 +585,7 @@ std::unordered_map<uint64_t, uint64_t> Result::counts(uint64_t shots, const std:
     SumTotal* total_dev = reinterpret_cast<SumTotal*>(idx.as<uint64_t>() + shots);
     k::Batch b = state.view(s, 1);
     build_sums(b, qubits, cdf.as<double>(), m, tmp, total_dev);
-    k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), m, &total_dev->total, 0.0, true, seed, shots, false,
+    k::sample_sums(s, cdf.as<double>(), tmp.as<double>(), m, &total_dev->total, true, seed, shots, false,
                    idx.as<uint64_t>());
     std::vector<uint64_t> h(shots + kTotalBytes / 8);
     cuda_check(cudaMemcpyAsync(h.data(), idx.p, shots * 8 + kTotalBytes, cudaMemcpyDeviceToHost, s), "read samples");
