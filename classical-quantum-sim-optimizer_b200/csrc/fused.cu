@@ -671,7 +671,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Up to kNormDirect tiles the next pass sums the tile norms itself: the sum's kernel
 // was 3 of the 28 us of a small circuit's pass and near half of a batch's launches (14-qubit
 // ansatz 0.068 -> 0.060 ms, 18 qubits 0.111 -> 0.099, 64 circuits of 12 to 15
-// qubits 0.156 -> 0.140; 256 of 12 to 22 qubits, which fill the device, 12.05 -> 12.2).
+// qubits 0.156 -> 0.140). Where other circuits fill the device it gives little: 256 of 12 to 22
+// qubits 10.94 -> 10.97, but 128 of 12 to 20 qubits 1.91 -> 1.81, so batches take the same rule.
 constexpr uint64_t kNormChunk = 2048, kNormDirect = 64;
 __global__ void k_state_norm(const double* __restrict__ tile_norm, uint64_t tiles_per_state, int parts,
                              double* __restrict__ norm) {
