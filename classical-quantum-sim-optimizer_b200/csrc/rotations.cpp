@@ -334,9 +334,14 @@ class Lowering {
         };
         const ld half = std::atan2(s, c) / 2;  // theta / 4
         crz(gamma);
-        controlled_z(controls, target);
-        rotation({target}, {target}, std::cos(half), -std::sin(half));
-        controlled_z(controls, target);
+        if (nc == 1) {
+            // CZ RY CZ is the rotation about Z Y (its negative where the control holds at 0): no phases.
+            rotation({target}, {target, q[0]}, std::cos(half), controls[0].value ? -std::sin(half) : std::sin(half));
+        } else {
+            controlled_z(controls, target);
+            rotation({target}, {target}, std::cos(half), -std::sin(half));
+            controlled_z(controls, target);
+        }
         rotation({target}, {target}, std::cos(half), std::sin(half));
         crz(beta);
         std::vector<ld> phi(size_t(1) << nc, 0.0);

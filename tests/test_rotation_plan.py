@@ -434,3 +434,15 @@ def test_matrices_further_from_unitary_than_rounding_have_no_rotation_form():
 def test_matrices_further_from_unitary_than_rounding_are_applied_as_they_are():
     c = Circuit(5, FAR)
     assert np.max(np.abs(dqsim.StatevectorSimulator(seed=1).simulate(c).statevector - oracle_state(c))) <= 1e-15
+
+
+@pytest.mark.parametrize("tile,tables", [(6, 4), (5, 5)])
+def test_controlled_rotations_take_no_phases_between(tile, tables):
+    """A ring of CRY as rotations about Y and Z Y, controls in the tile and outside: the tables settle what rotations owe."""
+    c = Circuit(6, [inst("ry", qubit=q, theta=0.3 + q) for q in range(6)] +
+                [inst("cry", control=q, target=(q + 1) % 6, theta=0.9 + q) for q in range(6)])
+    error, plan = replay_error(c, tile)
+    assert error <= 1e-15
+    assert sum(p["slot_phases"] for p in plan["passes"]) == 0
+    assert sum(p["rotations"] for p in plan["passes"]) == 18
+    assert sum(p["tables"] for p in plan["passes"]) <= tables
