@@ -978,22 +978,36 @@ int dq_rotation_plan_dump(const char* json, size_t len, int tile_qubits, char** 
             for (auto i = begin; i != end; ++i) s += (i == begin ? "" : ",") + std::to_string(*i);
             s += "]";
         };
-        for (size_t pi = 0; pi < passes.size(); pi++) {
-            const TilePass& p = passes[pi];
-            RotProgram r;
-            const bool ok = build_rotation_pass(p.raw, p.qubits, int(n), r);
-            s += std::string(pi ? ",{" : "{") + "\"ok\":" + (ok ? "true" : "false") +
-                 ",\"raw\":" + std::to_string(p.raw_ops) + ",\"data\":" + std::to_string(r.data) + ",\"phases\":" + std::to_string(r.nphases) +
+        auto program = [&](const RotProgram& r) {
+            s += "\"data\":" + std::to_string(r.data) + ",\"phases\":" + std::to_string(r.nphases) +
                  ",\"rotations\":" + std::to_string(r.rotations) + ",\"tables\":" + std::to_string(r.tables) +
                  ",\"slot_phases\":" + std::to_string(r.slot_phases) + ",\"out_const\":" +
                  std::to_string(r.out_const) + ",\"sign_local\":" + std::to_string(r.sign_local) +
                  ",\"sign_outer\":" + std::to_string(r.sign_outer) + ",\"sign_const\":" + std::to_string(r.sign_const);
-            list("qubits", p.qubits.begin(), p.qubits.end());
             list("out_dir", r.out_dir, r.out_dir + r.m);
             list("out_outer", r.out_outer, r.out_outer + kRotMaxOuter);
             std::vector<uint32_t> flat;
             for (const uint4& w : r.words) flat.insert(flat.end(), {w.x, w.y, w.z, w.w});
             list("words", flat.begin(), flat.end());
+        };
+        for (size_t pi = 0; pi < passes.size(); pi++) {
+            const TilePass& p = passes[pi];
+            RotProgram r;
+            const bool ok = build_rotation_pass(p.raw, p.qubits, int(n), r);
+            s += std::string(pi ? ",{" : "{") + "\"ok\":" + (ok ? "true" : "false") +
+                 ",\"raw\":" + std::to_string(p.raw_ops) + ",";
+            program(r);
+            list("qubits", p.qubits.begin(), p.qubits.end());
+            if (r.words.size() > size_t(kRotParamWords)) {  // as it is launched
+                s += ",\"parts\":[";
+                const std::vector<RotProgram> parts = split_rotation_pass(std::move(r));
+                for (size_t i = 0; i < parts.size(); i++) {
+                    s += i ? ",{" : "{";
+                    program(parts[i]);
+                    s += "}";
+                }
+                s += "]";
+            }
             s += "}";
         }
         s += "]}";

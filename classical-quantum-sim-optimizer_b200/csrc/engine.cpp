@@ -639,33 +639,31 @@ void Executor::lower_segment(const std::vector<Operation>& ops, size_t begin, si
         for (auto& p : ps) add_tile_pass(std::move(p));
         return;
     }
-    std::vector<RotProgram> programs(ps.size());
-    std::vector<char> ok(ps.size(), 0);
+    std::vector<std::vector<RotProgram>> programs(ps.size());  // none: no rotation form
     parallel_for(ps.size(), [&](size_t i) {
-        ok[i] = char(build_rotation_pass(ps[i].raw, ps[i].qubits, cfg_.n, programs[i]));
+        RotProgram p;
+        if (build_rotation_pass(ps[i].raw, ps[i].qubits, cfg_.n, p)) programs[i] = split_rotation_pass(std::move(p));
     });
     for (size_t i = 0; i < ps.size(); i++) {
         TilePass& p = ps[i];
-        if (!ok[i]) {
+        if (programs[i].empty()) {
             lower_pass_ops(p.raw, p.qubits, cfg_.n, cfg_.fuse, pool_host_, p.ops);
             p.raw.clear();
             add_tile_pass(std::move(p));
             continue;
         }
-        RotStep r;
-        r.qubits = p.qubits;
-        r.raw_ops = p.raw_ops;
-        r.program = std::move(programs[i]);
-        if (r.program.words.size() > size_t(kRotParamWords)) {
-            r.words_at = rot_words_host_.size();
-            rot_words_host_.insert(rot_words_host_.end(), r.program.words.begin(), r.program.words.end());
+        for (size_t part = 0; part < programs[i].size(); part++) {
+            RotStep r;
+            r.qubits = p.qubits;
+            r.raw_ops = part == 0 ? p.raw_ops : 0;
+            r.program = std::move(programs[i][part]);
+            Step s;
+            s.rot = int(rots_.size());
+            s.type = Operation::Dense;
+            s.category = 1;
+            rots_.push_back(std::move(r));
+            steps_.push_back(std::move(s));
         }
-        Step s;
-        s.rot = int(rots_.size());
-        s.type = Operation::Dense;
-        s.category = 1;
-        rots_.push_back(std::move(r));
-        steps_.push_back(std::move(s));
     }
 }
 
@@ -891,12 +889,6 @@ void Executor::upload(cudaStream_t stream) {
                                    cudaMemcpyHostToDevice, stream),
                    "upload tile phases");
     }
-    if (!rot_words_host_.empty()) {
-        get(rot_words_, rot_words_host_.size() * sizeof(uint4), stream, "rotation passes");
-        cuda_check(cudaMemcpyAsync(rot_words_.p, rot_words_host_.data(), rot_words_host_.size() * sizeof(uint4),
-                                   cudaMemcpyHostToDevice, stream),
-                   "upload rotation passes");
-    }
     if (!fused_blocks_host_.empty()) {
         get(fused_blocks_, fused_blocks_host_.size() * sizeof(FusedBlock), stream, "fused block descriptors");
         get(upool_, upool_host_.size() * sizeof(uint16_t), stream, "fused block gate images");
@@ -990,8 +982,7 @@ void Executor::run(const k::Batch& b, ProfileAcc* profile, EventRecorder* rec, b
             if (rec) rec->begin(kcTile, step_bytes(si, b));
             if (s.rot >= 0) {
                 const RotStep& r = rots_[size_t(s.rot)];
-                k::rotation_pass(b, r.qubits, r.program,
-                                 rot_words_.p ? rot_words_.as<uint4>() + r.words_at : nullptr, from_basis && si == 0);
+                k::rotation_pass(b, r.qubits, r.program, from_basis && si == 0);
                 if (rec) rec->end();
                 finish_tile_step(profile, b.stream, t0);
                 continue;

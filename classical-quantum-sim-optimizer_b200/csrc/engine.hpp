@@ -258,12 +258,9 @@ class Executor {
     struct RotStep {
         std::vector<int> qubits;
         RotProgram program;
-        size_t words_at = 0;  // of its words in rot_words_host_ (programs larger than a launch argument)
         int raw_ops = 0;
     };
     std::vector<RotStep> rots_;
-    std::vector<uint4> rot_words_host_;
-    DevMem rot_words_;
     DevMem pool_, tile_ops_, fused_blocks_, upool_, norm_tiles_, norm_states_, phase_words_;
     bool uploaded_ = false;
     ExecConfig cfg_;

@@ -37,7 +37,7 @@ struct RotWords {
 };
 
 // Programs: steps from the launch argument (uniform loads from the constant
-// bank) and their data from shared memory, or all of it in device memory.
+// bank) and their data from shared memory.
 struct ArgWords {
     const RotWords* a;
     const uint4* table;
@@ -45,13 +45,6 @@ struct ArgWords {
     __device__ __forceinline__ uint4 data(uint32_t i) const { return table[i]; }
     // (as doubles: taken apart from a uint4, each factor cost two register moves, a quarter of a table's instructions)
     __device__ __forceinline__ double2 factor(uint32_t i) const { return reinterpret_cast<const double2*>(table)[i]; }
-};
-struct DevWords {
-    const uint4* __restrict__ w;
-    const uint4* __restrict__ table;
-    __device__ __forceinline__ uint4 operator()(uint32_t i) const { return __ldg(w + i); }
-    __device__ __forceinline__ uint4 data(uint32_t i) const { return __ldg(table + i); }
-    __device__ __forceinline__ double2 factor(uint32_t i) const { return __ldg(reinterpret_cast<const double2*>(table) + i); }
 };
 
 __device__ __forceinline__ double lo_hi(uint32_t lo, uint32_t hi) { return __hiloint2double(int(hi), int(lo)); }
@@ -347,12 +340,6 @@ __global__ void __launch_bounds__(kRotThreads, 1)
     rotation_body(s, n, p, pack, total_tiles, basis, ArgWords{&w, table});
 }
 
-__global__ void __launch_bounds__(kRotThreads, 1)
-    k_rotations_dev(double2* __restrict__ s, int n, int pack, uint64_t total_tiles, int basis,
-                    const __grid_constant__ RotPass p, const uint4* __restrict__ w) {
-    rotation_body(s, n, p, pack, total_tiles, basis, DevWords{w, w + p.data});
-}
-
 constexpr int kTeamTile = 12;      // qubits of a team's tile
 constexpr int kTeamThreads = 256;  // one thread per 16 amplitudes
 constexpr int kTeamBuffers = 3;
@@ -610,8 +597,7 @@ uint64_t resident_ctas(Kernel kernel, int threads, size_t smem) {
 
 }  // namespace
 
-void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const RotProgram& r, const uint4* words_dev,
-                   bool basis) {
+void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const RotProgram& r, bool basis) {
     if (b.c64) fail(kValueError, "rotation passes run on complex128 states");
     const bool swaps = r.nphases == 0 && !basis && (tile_qubits[0] > 0 || (b.W << b.n) <= kSwapStates);
     if (StateMap map; swaps && own_inverse(r, tile_qubits, b.n, map) && map.to[0] == 1) {
@@ -652,30 +638,22 @@ void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const Ro
     int pack = 0;
     while (tbits + pack < 6 && (uint64_t(2) << pack) <= total) pack++;
     const int threads = 1 << (tbits + pack);
-    const bool as_argument = r.words.size() <= size_t(kRotParamWords);
+    if (r.words.size() > size_t(kRotParamWords)) fail(kValueError, "rotation program larger than a launch argument");
     p.data = r.data;
     p.ndata = int(r.words.size()) - r.data;
-    const size_t smem = rotation_tile_smem(r.m, pack) + (as_argument ? size_t(p.ndata) * sizeof(uint4) : 0);
+    const size_t smem = rotation_tile_smem(r.m, pack) + size_t(p.ndata) * sizeof(uint4);
     const uint64_t ctas = (total + (uint64_t(1) << pack) - 1) >> pack;
-    if (as_argument) {
-        static thread_local RotWords args;
-        std::memcpy(args.w, r.words.data(), r.words.size() * sizeof(uint4));
-        const size_t team_smem = team_tile_smem() + size_t(p.ndata) * sizeof(uint4);
-        const bool teams = r.m == kTeamTile && r.tell >= 0;
-        const uint64_t sms = teams ? resident_ctas(k_rotations_team, 2 * kTeamThreads, team_smem) : 0;
-        if (teams && total >= kTeamTiles * sms) {
-            k_rotations_team<<<unsigned(sms), 2 * kTeamThreads, team_smem, b.stream>>>(static_cast<double2*>(b.amps), b.n, total, basis ? 1 : 0, p, args);
-        } else {
-            k_rotations_arg<<<unsigned(std::min(ctas, resident_ctas(k_rotations_arg, threads, smem))), unsigned(threads), smem,
-                              b.stream>>>(
-                static_cast<double2*>(b.amps), b.n, pack, total, basis ? 1 : 0, p, args);
-        }
-    } else {
-        if (!words_dev) fail(kValueError, "rotation pass without its device words");
-        k_rotations_dev<<<unsigned(std::min(ctas, resident_ctas(k_rotations_dev, threads, smem))), unsigned(threads), smem,
+    static thread_local RotWords args;
+    std::memcpy(args.w, r.words.data(), r.words.size() * sizeof(uint4));
+    const size_t team_smem = team_tile_smem() + size_t(p.ndata) * sizeof(uint4);
+    const bool teams = r.m == kTeamTile && r.tell >= 0;
+    const uint64_t sms = teams ? resident_ctas(k_rotations_team, 2 * kTeamThreads, team_smem) : 0;
+    if (teams && total >= kTeamTiles * sms)
+        k_rotations_team<<<unsigned(sms), 2 * kTeamThreads, team_smem, b.stream>>>(static_cast<double2*>(b.amps), b.n, total, basis ? 1 : 0, p, args);
+    else
+        k_rotations_arg<<<unsigned(std::min(ctas, resident_ctas(k_rotations_arg, threads, smem))), unsigned(threads), smem,
                           b.stream>>>(
-            static_cast<double2*>(b.amps), b.n, pack, total, basis ? 1 : 0, p, words_dev);
-    }
+            static_cast<double2*>(b.amps), b.n, pack, total, basis ? 1 : 0, p, args);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) fail(kCudaError, std::string("rotation pass: ") + cudaGetErrorString(e));
 }

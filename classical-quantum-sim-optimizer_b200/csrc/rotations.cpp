@@ -466,6 +466,11 @@ struct Span {
 
 constexpr ld kMaxOwed = 200.0L;  // rotations may leave amplitudes e^200 too large before a table
 constexpr int kWindow = 128;  // items a phase chooses among
+// Rotations a phase may hold: its words then fit a launch argument whatever the
+// circuit. A rotation takes at most 20 (its own two, a step, a table before it
+// with another), each other item of the window 6, the phase itself 39.
+constexpr int kPhaseRotations = 83;
+static_assert(20 * kPhaseRotations + 6 * (kWindow - kPhaseRotations) + 39 <= kRotParamWords);
 // Below this many qubits half of them: planning then takes a third less time,
 // where it is most of a call, for at most 3 % longer programs (either way).
 constexpr int kWideQubits = 20;
@@ -522,6 +527,29 @@ uint4 factor_word(const Factor& f, ld off[2]) {
     return word(best[0], best[1]);
 }
 
+// The phase after which a team's fetch counts as done (RotProgram::tell), by the
+// SM cycles of a 12-qubit tile's phases as measured step by step.
+int teller(const RotProgram& p) {
+    const double rotation[4] = {0, 135, 300, 340};
+    std::vector<double> upto;  // the work up to each phase's end
+    for (int ph = 0; ph < p.nphases; ph++) {
+        const uint4 head = p.words[size_t(3 * ph)];
+        double cycles = 1100;
+        for (uint32_t i = 0; i < head.y; i++) {
+            const uint4 s = p.words[head.x + i];
+            cycles += 75 + (s.x & 0xF00u ? 300 : 0) + (s.x & kRotTable ? 300 : 0);
+            for (int j = 0; j < 4; j++) cycles += rotation[(s.x >> (2 * j)) & 3u];
+            if (s.x & (kRotSlots | kRotSlotModuli)) cycles += 370 + 73.0 * double(s.w & 0xFFFFu);
+        }
+        upto.push_back((upto.empty() ? 0.0 : upto.back()) + cycles);
+    }
+    if (upto.empty()) return -1;
+    const double half = 0.55 * (upto.back() + 3000.0);  // (the rest: stores and fetches)
+    int tell = std::min(1, (p.nphases - 1) / 2);
+    while (tell >= 0 && upto[size_t(tell)] > half) tell--;
+    return tell;
+}
+
 class Scheduler {
   public:
     Scheduler(std::vector<Item> items, int m, int n, Lowering& lw, RotProgram& out)
@@ -535,13 +563,18 @@ class Scheduler {
             std::vector<uint4> steps, rots;
         };
         std::vector<Ph> phases;
+        std::vector<int> data_at;
         do {
             Ph p;
+            data_at.push_back(int(tables_.size()));
             one_phase(p.head);
             pack(p.steps, p.rots);
             phases.push_back(std::move(p));
         } while (!active_.empty());
-        if (phases.size() == 1 && phases[0].steps.empty()) phases.clear();  // relabellings only
+        if (phases.size() == 1 && phases[0].steps.empty()) {  // relabellings only
+            phases.clear();
+            data_at.clear();
+        }
         size_t step_at = phases.size() * 3, rot_at = step_at;
         for (const Ph& p : phases) rot_at += p.steps.size();
         out_.words.clear();
@@ -560,26 +593,11 @@ class Scheduler {
         // The kernel fetches a step and a rotation ahead.
         out_.words.insert(out_.words.end(), 2, make_uint4(0, 0, 0, 0));
         out_.nphases = int(phases.size());
-        std::vector<double> upto;  // the work up to each phase's end
-        for (const Ph& p : phases) upto.push_back((upto.empty() ? 0.0 : upto.back()) + phase_work(p.steps));
-        const double half = phases.empty() ? 0.0 : 0.55 * (upto.back() + 3000.0);  // (the rest: stores and fetches)
-        out_.tell = phases.empty() ? -1 : std::min(1, int(phases.size() - 1) / 2);
-        while (out_.tell >= 0 && upto[size_t(out_.tell)] > half) out_.tell--;
+        out_.phase_data = data_at;
+        out_.tell = teller(out_);
     }
 
   private:
-    // SM cycles of a 12-qubit tile's phase, as measured step by step.
-    static double phase_work(const std::vector<uint4>& steps) {
-        const double rotation[4] = {0, 135, 300, 340};
-        double cycles = 1100;
-        for (const uint4& s : steps) {
-            cycles += 75 + (s.x & 0xF00u ? 300 : 0) + (s.x & kRotTable ? 300 : 0);
-            for (int j = 0; j < 4; j++) cycles += rotation[(s.x >> (2 * j)) & 3u];
-            if (s.x & (kRotSlots | kRotSlotModuli)) cycles += 370 + 73.0 * double(s.w & 0xFFFFu);
-        }
-        return cycles;
-    }
-
     std::vector<Item> items_;
     int m_, window_;
     Lowering& lw_;
@@ -648,6 +666,7 @@ class Scheduler {
             exec = Bits{};
             for (int i = 0; i < W; i++) {
                 if ((red[i] && red[i] != more) || !pred[i].within(exec)) continue;
+                if (dir[i] && rots == kPhaseRotations) continue;
                 rots += dir[i] ? 1 : 0;
                 exec.set(i);
             }
@@ -1209,6 +1228,76 @@ bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<in
         if (bit) out.sign_outer |= 1u << j;
     }
     return true;
+}
+
+std::vector<RotProgram> split_rotation_pass(RotProgram&& p, size_t most) {
+    std::vector<RotProgram> parts;
+    if (p.words.size() <= most) {
+        parts.push_back(std::move(p));
+        return parts;
+    }
+    const int end = int(p.words.size()) - 2 - p.data;
+    auto rots_end = [&](int ph) { return ph + 1 < p.nphases ? p.words[size_t(3 * ph + 5)].y : uint32_t(p.data); };
+    auto data_end = [&](int ph) { return ph + 1 < p.nphases ? p.phase_data[size_t(ph + 1)] : end; };
+    auto size = [&](int ph) {
+        const uint4 *h = &p.words[size_t(3 * ph)];
+        return size_t(3 + h[0].y + rots_end(ph) - h[2].y) + size_t(data_end(ph) - p.phase_data[size_t(ph)]);
+    };
+    for (int first = 0; first < p.nphases;) {
+        int last = first;
+        for (size_t total = 2 + size(first); last + 1 < p.nphases; last++) {
+            total += size(last + 1);
+            if (total > most) break;
+        }
+        RotProgram part;
+        part.m = p.m;
+        part.nphases = last + 1 - first;
+        const int base = p.phase_data[size_t(first)];
+        uint32_t step_at = uint32_t(3 * part.nphases), rot_at = step_at;
+        for (int ph = first; ph <= last; ph++) rot_at += p.words[size_t(3 * ph)].y;
+        for (int ph = first; ph <= last; ph++) {
+            const uint4 *h = &p.words[size_t(3 * ph)];
+            part.words.insert(part.words.end(), h, h + 3);
+            uint4* own = &part.words[part.words.size() - 3];
+            own[0].x = step_at;
+            own[2].y = rot_at;
+            step_at += h[0].y;
+            rot_at += rots_end(ph) - h[2].y;
+        }
+        for (int ph = first; ph <= last; ph++) {
+            const uint4 head = p.words[size_t(3 * ph)];
+            for (uint32_t i = 0; i < head.y; i++) {
+                uint4 s = p.words[head.x + i];
+                if (s.x & kRotTable) s.y -= uint32_t(base);
+                if (s.x & (kRotSlots | kRotSlotModuli)) s.z -= uint32_t(base);
+                part.words.push_back(s);
+            }
+        }
+        auto take = [&](size_t from, size_t to) {
+            part.words.insert(part.words.end(), p.words.begin() + long(from), p.words.begin() + long(to));
+        };
+        take(p.words[size_t(3 * first + 2)].y, rots_end(last));
+        part.data = int(part.words.size());
+        take(size_t(p.data + base), size_t(p.data + data_end(last)));
+        part.words.insert(part.words.end(), 2, make_uint4(0, 0, 0, 0));
+        part.tell = teller(part);
+        // Places stay as they are between the parts; the last one leaves the frame.
+        for (int q = 0; q < p.m; q++) part.out_dir[q] = uint16_t(rot_swizzle(1u << q));
+        parts.push_back(std::move(part));
+        first = last + 1;
+    }
+    RotProgram& out = parts.back();
+    std::copy(std::begin(p.out_dir), std::end(p.out_dir), out.out_dir);
+    std::copy(std::begin(p.out_outer), std::end(p.out_outer), out.out_outer);
+    out.out_const = p.out_const;
+    out.sign_local = p.sign_local;
+    out.sign_outer = p.sign_outer;
+    out.sign_const = p.sign_const;
+    out.flops_per_amp = p.flops_per_amp;
+    out.rotations = p.rotations;
+    out.tables = p.tables;
+    out.slot_phases = p.slot_phases;
+    return parts;
 }
 
 }  // namespace dq

@@ -48,7 +48,7 @@ constexpr int kRotSlotBits = kRotMaxTile - kRotRegBits;
 // Parity masks of the kernel hold the slot (thread) bits below bit kRotSlotBits
 // and the bits of the tile's index above.
 constexpr int kRotMaxOuter = 32 - kRotSlotBits;
-constexpr int kRotParamWords = 1980;  // largest program passed as a launch argument (31,680 bytes)
+constexpr int kRotParamWords = 1980;  // largest program, a launch argument (31,680 bytes)
 
 // A pass's program, in 16-byte words:
 //   phase p at 3p: {first step word, steps, v0 | v1 << 16, v2 | v3 << 16}, then the
@@ -76,6 +76,7 @@ struct RotProgram {
     int nphases = 0;
     std::vector<uint4> words;
     int data = 0;                    // first word of the steps' data
+    std::vector<int> phase_data;     // where each phase's data begin among them
     int tell = -1;                   // phase after which a team's fetch counts as done (rotation_pass.cu); -1: no teams
     // Where the last sweep finds the amplitude of tile index e: XOR of
     // out_dir[q] over e's set bits, out_outer[j] over the set bits of the
@@ -125,13 +126,18 @@ int rotation_pinned_low(const std::vector<Operation>& ops, size_t begin, size_t 
 bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<int>& tile_qubits, int n,
                          RotProgram& out);
 
+// A program as programs of at most `most` words, to be run one after another: cut
+// between phases.  A launch argument's steps and rotations come through the constant
+// bank.  Read from device memory instead, 40 layers of 8-qubit brickwork (2,686
+// words) took 0.222 ms, as two launches 0.159; 60 layers on 12 of 26 qubits (4
+// launches, each a sweep of the state) 41.1 and 26.3.
+std::vector<RotProgram> split_rotation_pass(RotProgram&& p, size_t most = kRotParamWords);
+
 namespace k {
-// One pass over every tile of every state (complex128).  `words_dev`: the
-// program's words on the device, read when they exceed kRotParamWords.
+// One pass over every tile of every state (complex128), of at most kRotParamWords words.
 // `basis`: every state is |0...0> on entry; the pass builds its input tiles
 // itself and reads nothing of the state.
-void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const RotProgram& p, const uint4* words_dev,
-                   bool basis);
+void rotation_pass(const Batch& b, const std::vector<int>& tile_qubits, const RotProgram& p, bool basis);
 }  // namespace k
 
 }  // namespace dq

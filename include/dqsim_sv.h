@@ -400,7 +400,8 @@ DQ_API int dq_compile_dump(const char* json, size_t json_len, char** out_text);
  * counterpart in the reference; it exposes the planner for inspection. */
 DQ_API int dq_tile_plan_dump(const char* json, size_t json_len, int tile_qubits, int fusion_width, char** out_text);
 /* Host-only: the complex128 rotation passes of the circuit's unitary operations
- * (per pass its tile qubits, program words and output map) as JSON text. */
+ * (per pass its tile qubits, program words and output map, and the parts a program
+ * larger than a launch argument is launched as) as JSON text. */
 DQ_API int dq_rotation_plan_dump(const char* json, size_t json_len, int tile_qubits, char** out_text);
 /* Host-only: the tensor-core fused plan (12-qubit passes of 32x32 blocks: layout
  * tables, f16 hi/lo gate images and each pass's TMA box plan) as JSON text.  No

@@ -446,3 +446,30 @@ def test_controlled_rotations_take_no_phases_between(tile, tables):
     assert sum(p["slot_phases"] for p in plan["passes"]) == 0
     assert sum(p["rotations"] for p in plan["passes"]) == 18
     assert sum(p["tables"] for p in plan["passes"]) <= tables
+
+
+@pytest.mark.parametrize("maker", [lambda: brickwork(5, 90, seed=1, measure=False), lambda: brickwork(9, 60, seed=2, measure=False),
+                                   lambda: mixed_layers(8, 90, 3, ("rx", "ry"), "cx"), lambda: form_circuit(4, 9, 900)])
+def test_programs_larger_than_a_launch_argument_in_parts(maker):
+    """Cut between phases: each part fits, and run one after another they are the whole."""
+    c = maker()
+    n = c.data["qregs"]["q"]["size"]
+    for tile in {5, n}:
+        plan = _core.rotation_plan_dump(c.model_dump_json(), tile)
+        assert tile < n or any("parts" in p for p in plan["passes"])
+        parts = [dict(part, qubits=p["qubits"]) for p in plan["passes"] for part in p.get("parts", [p])]
+        assert all(len(p["words"]) // 4 <= 1980 for p in parts)
+        for p in plan["passes"]:
+            assert sum(part["phases"] for part in p.get("parts", [p])) == p["phases"]
+        np.testing.assert_allclose(replay({"n": n, "passes": parts}), oracle_state(c), atol=1e-13, rtol=0)
+
+
+def test_a_phase_fits_a_launch_argument():
+    """The longest phases: many rotations that commute, each with a table before it (X X on all pairs), on 20 qubits."""
+    n = 20
+    rng = np.random.default_rng(1)
+    ins = [inst("rxx", a=a, b=b, theta=float(rng.uniform(-3, 3))) for _ in range(3) for a in range(8) for b in range(a)]
+    ins += [inst("ry", qubit=q, theta=0.1 + q) for q in range(n)]
+    for p in _core.rotation_plan_dump(Circuit(n, ins + ins).model_dump_json(), 12)["passes"]:
+        assert p["ok"]
+        assert all(len(part["words"]) // 4 <= 1980 for part in p.get("parts", [p]))
