@@ -3,6 +3,7 @@
 #include "rotations.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 
@@ -27,6 +28,7 @@ constexpr ld kExactTol = 1e-18L;  // the same, to the rounding of the numbers he
 constexpr int kMaxDiagQubits = 6;
 
 int parity64(uint64_t x) { return __builtin_parityll(x); }
+int parity(uint32_t x) { return __builtin_parity(x); }  // (of directions and what lies on them: tile bits)
 
 struct Item {
     bool rot = false;
@@ -152,7 +154,11 @@ class Lowering {
     std::vector<uint64_t> mask_;
     std::vector<int> cons_;
     std::vector<uint32_t> dir_;
-    std::vector<size_t> open_;  // phases that every later rotation commutes with
+    struct Open {
+        uint64_t mask;
+        size_t item;
+    };
+    std::vector<Open> open_;  // phases that every later rotation commutes with
 
     // exp(i a Z^mask (-1)^cons); `tol`: what an angle may be off a multiple of pi/2 and count as one.
     void phase(uint64_t mask, int cons, ld a, ld tol = kExactTol) {
@@ -161,30 +167,36 @@ class Lowering {
             turn(global, a);
             return;
         }
-        const ld r = std::nearbyint(a / kPiL);
-        a -= r * kPiL;
-        if (std::fmod(std::fabs(r), 2.0L) == 1.0L) turn(global, kPiL);
+        if (std::fabs(a) > kPiL / 2) {
+            const ld r = std::nearbyint(a / kPiL);
+            a -= r * kPiL;
+            if (std::fmod(r, 2.0L) != 0.0L) turn(global, kPiL);
+        }
         if (std::fabs(a) <= tol) return;
         if (std::fabs(std::fabs(a) - kPiL / 2) <= tol) {  // +-i Z^mask
             turn(global, a > 0 ? kPiL / 2 : -kPiL / 2);
             sign ^= mask;
             return;
         }
-        for (size_t i : open_)
-            if (items[i].mask == mask) {
-                turn(items[i].a, a);
+        for (const Open& o : open_)
+            if (o.mask == mask) {
+                turn(items[o.item].a, a);
                 return;
             }
         Item it;
         it.mask = mask;
         it.a = a;
-        open_.push_back(items.size());
+        open_.push_back({mask, items.size()});
         items.push_back(it);
     }
 
     // exp(-i theta/2 P) with (c, s) = (cos, sin)(theta/2), P the product over the
     // qubits of X (bit of xs), Z (of zs) or Y (both).
-    void rotation(const std::vector<uint64_t>& xs, const std::vector<uint64_t>& zs, ld c, ld s) {
+    void rotation(std::initializer_list<uint64_t> xs, std::initializer_list<uint64_t> zs, ld c, ld s) {
+        rotation_of<std::initializer_list<uint64_t>>(xs, zs, c, s);
+    }
+    template <class Qubits>
+    void rotation_of(const Qubits& xs, const Qubits& zs, ld c, ld s) {
         uint32_t v = 0;
         uint64_t mask = 0;
         int cons = 0, ny = 0;
@@ -234,7 +246,7 @@ class Lowering {
         norm += 0.5L * (c * c + s * s - 1.0L);  // (an RXX's entries as they are rounded)
         if (parity64(sign & v)) it.t = -it.t;
         open_.erase(std::remove_if(open_.begin(), open_.end(),
-                                   [&](size_t i) { return parity64(items[i].mask & v) != 0; }),
+                                   [&](const Open& o) { return parity(uint32_t(o.mask) & v) != 0; }),
                     open_.end());
         items.push_back(it);
     }
@@ -306,10 +318,9 @@ class Lowering {
         if (controls.empty()) {
             turn(global, alpha);
             // RZ(-+pi/2) RY(theta) RZ(+-pi/2) = RX(+-theta)
-            const ld turns = std::nearbyint((beta + gamma) / (2 * kPiL));
-            const ld quarter = std::fabs(std::remainder(beta, 2 * kPiL));
+            const ld turns = std::fabs(beta + gamma) < kPiL ? 0.0L : std::nearbyint((beta + gamma) / (2 * kPiL));
             if (s > 0 && std::fabs(beta + gamma - turns * 2 * kPiL) <= kAngleTol &&
-                std::fabs(quarter - kPiL / 2) <= kAngleTol) {
+                std::fabs(std::fabs(std::remainder(beta, 2 * kPiL)) - kPiL / 2) <= kAngleTol) {
                 // RZ(gamma) = RZ(-beta) (-1)^turns; beta = +-pi/2 up to whole turns, which cancel in the pair.
                 if (std::fmod(std::fabs(turns), 2.0L) == 1.0L) turn(global, kPiL);
                 rotation({target}, {}, c, std::remainder(beta, 2 * kPiL) < 0 ? s : -s);
@@ -437,7 +448,7 @@ class Lowering {
                 if (X & 1) xs.push_back(lo);
                 if (Z & 2) zs.push_back(hi);
                 if (Z & 1) zs.push_back(lo);
-                rotation(xs, zs, c, s);
+                rotation_of(xs, zs, c, s);
                 return;
             }
         throw Unsupported{};
@@ -479,8 +490,20 @@ struct Bits {
     uint64_t w[2] = {0, 0};
     void set(int i) { w[i >> 6] |= uint64_t(1) << (i & 63); }
     bool get(int i) const { return (w[i >> 6] >> (i & 63)) & 1; }
-    bool within(const Bits& o) const { return !(w[0] & ~o.w[0]) && !(w[1] & ~o.w[1]); }
+    bool within(const Bits& o) const { return !((w[0] & ~o.w[0]) | (w[1] & ~o.w[1])); }
+    bool any() const { return (w[0] | w[1]) != 0; }
+    int count() const { return __builtin_popcountll(w[0]) + __builtin_popcountll(w[1]); }
+    // f(i) for every member in order.
+    template <class F>
+    void each(F&& f) const {
+        for (int k = 0; k < 2; k++)
+            for (uint64_t r = w[k]; r; r &= r - 1) f(64 * k + __builtin_ctzll(r));
+    }
 };
+Bits operator&(const Bits& a, const Bits& b) { return {{a.w[0] & b.w[0], a.w[1] & b.w[1]}}; }
+Bits operator|(const Bits& a, const Bits& b) { return {{a.w[0] | b.w[0], a.w[1] | b.w[1]}}; }
+Bits operator^(const Bits& a, const Bits& b) { return {{a.w[0] ^ b.w[0], a.w[1] ^ b.w[1]}}; }
+Bits without(const Bits& a, const Bits& b) { return {{a.w[0] & ~b.w[0], a.w[1] & ~b.w[1]}}; }
 
 uint4 word(uint32_t x, uint32_t y, uint32_t z, uint32_t w) { return make_uint4(x, y, z, w); }
 uint4 word(double a, double b) {
@@ -502,28 +525,61 @@ struct Factor {
     }
 };
 
-Factor factor(ld b, ld a) {
-    const ld g = b == 0.0L ? 1.0L : std::exp(b);
-    return a == 0.0L ? Factor{g, 0.0L} : Factor{g * std::cos(a), g * std::sin(a)};
+// e^{ia} for |a| <= 2 pi: of the nearest multiple of pi/64, from a table, times
+// that of the rest, below pi/128, by the power series to its 10th term (1e-23).
+Factor turned(ld a) {
+    static const std::vector<Factor> table = [] {
+        std::vector<Factor> t;
+        for (int k = -129; k <= 129; k++) t.push_back({std::cos(ld(k) * kPiL / 64), std::sin(ld(k) * kPiL / 64)});
+        return t;
+    }();
+    const int k = int(std::lrint(double(a) * (64 / 3.14159265358979323846)));
+    const ld x = a - ld(k) * (kPiL / 64), y = x * x;
+    Factor f{1.0L - y / 2 * (1.0L - y / 12 * (1.0L - y / 30 * (1.0L - y / 56 * (1.0L - y / 90)))),
+             x * (1.0L - y / 6 * (1.0L - y / 20 * (1.0L - y / 42 * (1.0L - y / 72))))};
+    f.times(table[size_t(k + 129)]);
+    return f;
+}
+
+ld grown(ld b) { return std::fabs(b) < 1e-10L ? 1.0L + b : std::exp(b); }
+
+// The neighbours of a double away from zero and towards it (zero has none).
+double outward(double x) {
+    if (x == 0.0) return x;
+    uint64_t u;
+    std::memcpy(&u, &x, 8);
+    u++;
+    std::memcpy(&x, &u, 8);
+    return x;
+}
+double inward(double x) {
+    if (x == 0.0) return x;
+    uint64_t u;
+    std::memcpy(&u, &x, 8);
+    u--;
+    std::memcpy(&x, &u, 8);
+    return x;
 }
 
 uint4 factor_word(const Factor& f, ld off[2]) {
     const ld re = f.re, im = f.im, S2 = re * re + im * im;
     const double x = double(re), y = double(im);
     double best[2] = {x, y};
-    ld miss = std::fabs(ld(x) * x + ld(y) * y - S2);
-    const double tries[4][2] = {{std::nextafter(x, 4.0 * x), y}, {std::nextafter(x, 0.0), y},
-                                {x, std::nextafter(y, 4.0 * y)}, {x, std::nextafter(y, 0.0)}};
-    for (const auto& t : tries) {
-        const ld m = std::fabs(ld(t[0]) * t[0] + ld(t[1]) * t[1] - S2);
+    const ld x2 = ld(x) * x, y2 = ld(y) * y;
+    ld miss = std::fabs(x2 + y2 - S2);
+    const double tries[4][2] = {{outward(x), y}, {inward(x), y}, {x, outward(y)}, {x, inward(y)}};
+    for (int i = 0; i < 4; i++) {
+        const double* t = tries[i];
+        const ld m = std::fabs(i < 2 ? ld(t[0]) * t[0] + y2 - S2 : x2 + ld(t[1]) * t[1] - S2);
         if (m < miss) {
             miss = m;
             best[0] = t[0];
             best[1] = t[1];
         }
     }
-    off[0] += ((best[0] - re) * re + (best[1] - im) * im) / S2;
-    off[1] += ((best[1] - im) * re - (best[0] - re) * im) / S2;
+    const ld dx = best[0] - re, dy = best[1] - im, inv = 1.0L / S2;
+    off[0] += (dx * re + dy * im) * inv;
+    off[1] += (dy * re - dx * im) * inv;
     return word(best[0], best[1]);
 }
 
@@ -642,103 +698,113 @@ class Scheduler {
         const int W = int(std::min<size_t>(active_.size(), size_t(window_)));
         std::vector<const Item*> it(static_cast<size_t>(W));
         for (int i = 0; i < W; i++) it[size_t(i)] = &items_[size_t(active_[size_t(i)])];
-        // Earlier items an item does not commute with (phases have no direction).
-        Bits pred[kWindow];
+        // Earlier items an item does not commute with: by the parity of one's mask on
+        // the other's direction, both ways (phases have no direction), a tile bit for
+        // all items at a time.
+        Bits pred[kWindow], all, rot_bits;
         uint32_t dir[kWindow];
         {
-            uint32_t mask[kWindow];  // directions are tile-local
+            Bits mask_has[kRotMaxTile], dir_has[kRotMaxTile];
+            const uint32_t local = (1u << m_) - 1;
             for (int j = 0; j < W; j++) {
-                dir[j] = it[size_t(j)]->v;
-                mask[j] = uint32_t(it[size_t(j)]->mask);
-                for (int i = 0; i < j; i++)
-                    pred[j].w[i >> 6] |= uint64_t(__builtin_parity((mask[i] & dir[j]) ^ (mask[j] & dir[i]))) << (i & 63);
+                const Item& x = *it[size_t(j)];
+                dir[j] = x.v;
+                Bits sum;
+                for (uint32_t r = x.v; r; r &= r - 1) sum = sum ^ mask_has[__builtin_ctz(r)];
+                for (uint32_t r = uint32_t(x.mask) & local; r; r &= r - 1) sum = sum ^ dir_has[__builtin_ctz(r)];
+                pred[j] = sum;
+                for (uint32_t r = x.v; r; r &= r - 1) dir_has[__builtin_ctz(r)].set(j);
+                for (uint32_t r = uint32_t(x.mask) & local; r; r &= r - 1) mask_has[__builtin_ctz(r)].set(j);
+                all.set(j);
+                if (x.rot) rot_bits.set(j);
             }
         }
         // Directions modulo V: a rotation can run when its own is 0, or the one
         // direction `more` that V is tried with.
         Span V;
         uint32_t red[kWindow];
-        auto reduce = [&] {
-            for (int i = 0; i < W; i++) red[i] = dir[i] ? V.reduce(dir[i]) : 0;
+        for (int i = 0; i < W; i++) red[i] = dir[i];
+        auto widen = [&](uint32_t v) {  // v into V, and its top bit out of the directions
+            v = V.reduce(v);
+            if (!V.add(v)) return;
+            const uint32_t top = uint32_t(1) << (31 - __builtin_clz(v));
+            for (int i = 0; i < W; i++)
+                if (red[i] & top) red[i] ^= v;
         };
-        auto closure = [&](uint32_t more, Bits& exec) {
-            int rots = 0;
-            exec = Bits{};
-            for (int i = 0; i < W; i++) {
-                if ((red[i] && red[i] != more) || !pred[i].within(exec)) continue;
-                if (dir[i] && rots == kPhaseRotations) continue;
+        // `exec` and what can run after it among `some`.
+        auto closure = [&](const Bits& some, Bits exec) {
+            int rots = (exec & rot_bits).count();
+            without(some, exec).each([&](int i) {
+                if (!pred[i].within(exec) || (dir[i] && rots == kPhaseRotations)) return;
                 rots += dir[i] ? 1 : 0;
                 exec.set(i);
-            }
-            return rots;
+            });
+            return exec;
         };
         // Directions one at a time: the one that lets the most rotations in,
         // among those of the first rotations that only lack their direction.
-        Bits exec;
-        reduce();
-        closure(0, exec);
+        Bits inside = without(all, rot_bits);  // items without a direction outside V
+        Bits exec = closure(inside, Bits{});
         while (V.dim < kRotRegBits) {
             uint32_t cand[8];
+            Bits has[8];
             int count = 0;
-            for (int i = 0; i < W && count < 8; i++)
-                if (red[i] && !exec.get(i) && pred[i].within(exec) && std::find(cand, cand + count, red[i]) == cand + count)
+            const Bits waiting = without(rot_bits, exec);
+            waiting.each([&](int i) {
+                if (count < 8 && red[i] && pred[i].within(exec) && std::find(cand, cand + count, red[i]) == cand + count)
                     cand[count++] = red[i];
+            });
+            waiting.each([&](int i) {
+                const int k = int(std::find(cand, cand + count, red[i]) - cand);
+                if (k < count) has[k].set(i);
+            });
             if (count == 0) break;
-            int best = -1;
-            uint32_t bestv = 0;
+            int best = -1, take = 0;
             Bits bestE;
             for (int k = 0; k < count; k++) {
-                Bits e;
-                const int r = closure(cand[k], e);
+                const Bits e = closure(inside | has[k], exec);
+                const int r = (e & rot_bits).count();
                 if (r > best) {
                     best = r;
-                    bestv = cand[k];
+                    take = k;
                     bestE = e;
                 }
             }
-            V.add(bestv);
+            widen(cand[take]);
+            inside = inside | has[take];
             exec = bestE;
-            reduce();
         }
-        for (int b = m_ - 1; b >= 0 && V.dim < kRotRegBits; b--) V.add(1u << b);
-        reduce();
-        closure(0, exec);
-        bool last = int(active_.size()) == W;
-        for (int i = 0; i < W && last; i++)
-            if (it[size_t(i)]->rot && !exec.get(i)) last = false;
+        for (int b = m_ - 1; b >= 0 && V.dim < kRotRegBits; b--) widen(1u << b);
+        for (int i = 0; i < W; i++)
+            if (!red[i]) inside.set(i);
+        exec = closure(inside, exec);
+        const bool last = int(active_.size()) == W && rot_bits.within(exec);
 
         // Order: rotations as far as they go, then the phases that hold the
         // next ones back, and so on.  `flush[f]` comes before the rotations of group f.
         std::vector<std::vector<int>> groups, flush;
-        Bits done, rot_bits;
-        for (int i = 0; i < W; i++)
-            if (dir[i]) rot_bits.set(i);
+        Bits done;
         while (true) {
             std::vector<int> g;
-            for (int i = 0; i < W; i++)
-                if (it[size_t(i)]->rot && exec.get(i) && !done.get(i) && pred[i].within(done)) {
-                    done.set(i);
-                    g.push_back(i);
-                }
-            groups.push_back(g);
+            without(rot_bits & exec, done).each([&](int i) {
+                if (!pred[i].within(done)) return;
+                done.set(i);
+                g.push_back(i);
+            });
+            groups.push_back(std::move(g));
             Bits needed;
-            for (int j = 0; j < W; j++) {
-                if (!it[size_t(j)]->rot || !exec.get(j) || done.get(j)) continue;
+            without(rot_bits & exec, done).each([&](int j) {
                 // Held back by phases only?
-                Bits missing;
-                for (int w = 0; w < 2; w++) missing.w[w] = pred[j].w[w] & ~done.w[w];
-                if ((missing.w[0] & rot_bits.w[0]) || (missing.w[1] & rot_bits.w[1])) continue;
-                for (int w = 0; w < 2; w++) needed.w[w] |= missing.w[w];
-            }
-            std::vector<int> need;
-            for (int i = 0; i < W; i++)
-                if (needed.get(i)) need.push_back(i);
-            if (need.empty()) break;
+                const Bits missing = without(pred[j], done);
+                if (!(missing & rot_bits).any()) needed = needed | missing;
+            });
+            if (!needed.any()) break;
             std::vector<int> ready;
-            for (int i : need)
+            needed.each([&](int i) {
                 if (pred[i].within(done)) ready.push_back(i);
+            });
             for (int i : ready) done.set(i);
-            flush.push_back(ready);
+            flush.push_back(std::move(ready));
         }
         // V's basis: the directions of the first rotations, whose signs then
         // follow their own register bit where they commute.
@@ -767,7 +833,7 @@ class Scheduler {
         int nm = 0;
         auto on_V = [&](uint64_t mask) {
             uint32_t r = 0;
-            for (int j = 0; j < kRotRegBits; j++) r |= uint32_t(parity64(mask & basis[j])) << j;
+            for (int j = 0; j < kRotRegBits; j++) r |= uint32_t(parity(uint32_t(mask) & basis[j])) << j;
             return r;
         };
         uint32_t ech[kRotRegBits] = {};
@@ -857,24 +923,34 @@ class Scheduler {
             for (uint32_t p : unit)
                 if (int(U.size()) < m_ - kRotRegBits && p && independent(p, true)) U.push_back(p);
         }
-        auto slots = [&](uint64_t mask) {  // kernel parity mask
-            uint32_t s = 0;
-            for (size_t i = 0; i < U.size(); i++) s |= uint32_t(parity64(mask & U[i])) << i;
-            return s | uint32_t(mask >> m_) << kRotSlotBits;
+        uint32_t slots_of[kWindow];
+        Bits slots_known;
+        auto slots = [&](int item) {  // kernel parity mask
+            if (!slots_known.get(item)) {
+                const uint64_t mask = it[size_t(item)]->mask;
+                uint32_t s = uint32_t(mask >> m_) << kRotSlotBits;
+                for (size_t i = 0; i < U.size(); i++) s |= uint32_t(parity(uint32_t(mask) & U[i])) << i;
+                slots_of[item] = s;
+                slots_known.set(item);
+            }
+            return slots_of[item];
         };
-        auto signs = [&](uint32_t r) {
-            uint32_t s = 0;
-            for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) s |= uint32_t(__builtin_parity(r & v)) << v;
-            return s;
-        };
+        static const std::array<uint32_t, kRotEntries> sign_bits = [] {
+            std::array<uint32_t, kRotEntries> all{};
+            for (uint32_t r = 0; r < uint32_t(kRotEntries); r++)
+                for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) all[r] |= uint32_t(parity(r & v)) << v;
+            return all;
+        }();
+        auto signs = [&](uint32_t r) { return sign_bits[r]; };
         uint32_t combined[kRotEntries] = {};  // the places of the register entries
         for (uint32_t d = 1; d < uint32_t(kRotEntries); d++)
             combined[d] = combined[d & (d - 1)] ^ basis[__builtin_ctz(d)];
-        auto direction = [&](uint32_t v) {  // v on the basis
+        uint32_t on_basis[kWindow];  // directions on the basis
+        (rot_bits & exec).each([&](int i) {
             uint32_t d = 1;
-            while (d < uint32_t(kRotEntries) && combined[d] != v) d++;
-            return d & uint32_t(kRotEntries - 1);
-        };
+            while (d < uint32_t(kRotEntries) && combined[d] != dir[i]) d++;
+            on_basis[i] = d & uint32_t(kRotEntries - 1);
+        });
 
         // Emission.  pend[j]: logarithm of the factor still owed by the entries
         // with register bit j clear (the others owe its negative).
@@ -887,15 +963,32 @@ class Scheduler {
             part.data = uint32_t(tables_.size());
             parts_.push_back(part);
             Factor T[kRotEntries];
-            T[0] = factor(uniform_, std::remainder(G, 2 * kPiL));
-            for (int v = 1; v < kRotEntries; v++) T[v] = T[0];
-            auto spread = [&](uint32_t r, ld b, ld a) {  // e^{b + ia}, inverted by the parity of r
-                const Factor plus = factor(b, a), minus = b == 0.0L ? Factor{plus.re, -plus.im} : factor(-b, -a);
-                for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) T[v].times(__builtin_parity(r & v) ? minus : plus);
+            ld g[kRotEntries];
+            T[0] = turned(std::remainder(G, 2 * kPiL));
+            g[0] = grown(uniform_);
+            for (int v = 1; v < kRotEntries; v++) {
+                T[v] = T[0];
+                g[v] = g[0];
+            }
+            auto grow = [&](uint32_t r, ld b) {  // e^b, inverted by the parity of r
+                const ld up = grown(b), down = 1.0L / up;
+                for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) g[v] *= __builtin_parity(r & v) ? down : up;
             };
             for (int j = 0; j < kRotRegBits; j++)
-                if (pend[j] != 0.0L) spread(1u << j, pend[j], 0.0L);
-            for (int i : f) spread(on_V(it[size_t(i)]->mask), it[size_t(i)]->b, it[size_t(i)]->a);
+                if (pend[j] != 0.0L) grow(1u << j, pend[j]);
+            for (int i : f) {
+                const Item& x = *it[size_t(i)];
+                const uint32_t r = on_V(x.mask);
+                if (x.a != 0.0L) {
+                    const Factor plus = turned(x.a), minus{plus.re, -plus.im};
+                    for (uint32_t v = 0; v < uint32_t(kRotEntries); v++) T[v].times(__builtin_parity(r & v) ? minus : plus);
+                }
+                if (x.b != 0.0L) grow(r, x.b);
+            }
+            for (int v = 0; v < kRotEntries; v++) {
+                T[v].re *= g[v];
+                T[v].im *= g[v];
+            }
             ld off[2] = {};
             for (const Factor& t : T) tables_.push_back(factor_word(t, off));
             for (ld& p : pend) p = 0.0;
@@ -917,7 +1010,7 @@ class Scheduler {
                     bool free = true;
                     for (size_t j = 0; j < i && free; j++) free = !pred[size_t(left[i])].get(left[j]);
                     if (!free) continue;
-                    const uint32_t d = direction(it[size_t(left[i])]->v);
+                    const uint32_t d = on_basis[left[i]];
                     const int p = (d & (d - 1)) == 0 && !it[size_t(left[i])]->imag ? __builtin_ctz(d) : 4;
                     if (p > at && p < place) {
                         place = p;
@@ -937,14 +1030,16 @@ class Scheduler {
         auto emit_flush = [&](std::vector<int> f, bool final) {
             // Phases that need no slot parity come along for nothing.
             bool free_table = final;
-            for (int i : f) free_table = free_table || slots(it[size_t(i)]->mask) == 0;
-            if (free_table)
-                for (int i = 0; i < W; i++)
-                    if (!it[size_t(i)]->rot && !done.get(i) && pred[i].within(applied_) &&
-                        slots(it[size_t(i)]->mask) == 0 && std::find(f.begin(), f.end(), i) == f.end()) {
-                        f.push_back(i);
-                        done.set(i);
-                    }
+            for (int i : f) free_table = free_table || slots(i) == 0;
+            if (free_table) {
+                Bits listed = done | rot_bits;
+                for (int i : f) listed.set(i);
+                without(all, listed).each([&](int i) {
+                    if (!pred[i].within(applied_) || slots(i) != 0) return;
+                    f.push_back(i);
+                    done.set(i);
+                });
+            }
             std::vector<std::pair<uint32_t, std::vector<int>>> by;  // register parity -> phases
             std::vector<int> here;  // of the table
             bool table = false;
@@ -953,7 +1048,7 @@ class Scheduler {
                 if (applied_.get(i)) continue;
                 applied_.set(i);
                 const uint32_t r = on_V(x.mask);
-                if (slots(x.mask) == 0) {
+                if (slots(i) == 0) {
                     table = true;
                     here.push_back(i);
                     continue;
@@ -979,11 +1074,11 @@ class Scheduler {
                     if (x.a != 0.0) {
                         ld off[2] = {};
                         angles.terms.push_back(i);
-                        angles.factors.push_back(factor_word(factor(0.0L, x.a), off));
+                        angles.factors.push_back(factor_word(turned(x.a), off));
                         uniform_ -= off[0];
                     }
                     if (x.b != 0.0) {
-                        const ld up = std::exp(x.b), down = std::exp(-x.b);
+                        const ld up = grown(x.b), down = 1.0L / up;
                         moduli.terms.push_back(i);
                         moduli.factors.push_back(word(double(up), double(down)));
                         uniform_ -= 0.5L * ((double(up) - up) / up + (double(down) - down) / down);
@@ -1012,7 +1107,7 @@ class Scheduler {
                 parts_.push_back(part);
                 for (size_t i = 0; i < count; i += 4) {
                     uint32_t m4[4] = {};
-                    for (size_t j = i; j < std::min(count, i + 4); j++) m4[j - i] = slots(it[size_t(step.terms[j])]->mask);
+                    for (size_t j = i; j < std::min(count, i + 4); j++) m4[j - i] = slots(step.terms[j]);
                     tables_.push_back(word(m4[0], m4[1], m4[2], m4[3]));
                 }
                 tables_.insert(tables_.end(), step.factors.begin(), step.factors.end());
@@ -1034,14 +1129,14 @@ class Scheduler {
         for (size_t g = groups.size(); g-- > 0;) {
             bool table = g + 1 == groups.size() && last;
             if (g < flush.size())
-                for (int i : flush[g]) table = table || slots(it[size_t(i)]->mask) == 0;
+                for (int i : flush[g]) table = table || slots(i) == 0;
             table_at[g] = table ? g : table_at[g + 1];
         }
         for (size_t g = 0; g < groups.size(); g++) {
             for (size_t gi = 0; gi < groups[g].size(); gi++) {
                 const int i = groups[g][gi];
                 const Item& x = *it[size_t(i)];
-                const uint32_t d = direction(x.v), r = on_V(x.mask);
+                const uint32_t d = on_basis[i], r = on_V(x.mask);
                 const int low = __builtin_ctz(d);
                 // In place where a table comes before the next rotation that mixes
                 // this register bit, or where the factors owed can join a phase
@@ -1049,7 +1144,7 @@ class Scheduler {
                 bool in_place = table_at[g] < groups.size();
                 for (size_t h = g; h < groups.size() && h <= table_at[g] && in_place; h++)
                     for (size_t hi = h == g ? gi + 1 : 0; hi < groups[h].size() && in_place; hi++)
-                        in_place = !((direction(it[size_t(groups[h][hi])]->v) >> low) & 1);
+                        in_place = !((on_basis[groups[h][hi]] >> low) & 1);
                 if (!in_place && table_at[g] == groups.size()) {
                     const uint64_t f = functional(low);
                     for (int j = 0; j < W && !in_place; j++)
@@ -1057,16 +1152,16 @@ class Scheduler {
                                    pred[j].within(done);
                     for (size_t h = g; h < groups.size() && in_place; h++)
                         for (size_t hi = h == g ? gi + 1 : 0; hi < groups[h].size() && in_place; hi++)
-                            in_place = !((direction(it[size_t(groups[h][hi])]->v) >> low) & 1);
+                            in_place = !((on_basis[groups[h][hi]] >> low) & 1);
                 }
                 const ld lost = 0.5L * std::log1p(ld(x.t) * x.t);
                 Part part;
                 part.place = (d & (d - 1)) == 0 && !x.imag ? low : 4;
                 part.d = d;
                 part.kind = x.imag ? kRotImag : !in_place ? kRotKept
-                            : part.place < 4 && r == (1u << low) && slots(x.mask) == 0 ? kRotPlain : kRotSigned;
+                            : part.place < 4 && r == (1u << low) && slots(i) == 0 ? kRotPlain : kRotSigned;
                 part.signs = signs(r);
-                part.mask = slots(x.mask);
+                part.mask = slots(i);
                 part.t = x.t;
                 part.u = double(ld(x.t) / (1.0L + ld(x.t) * x.t));
                 // Entries that owe different factors must not mix, whatever the kind: those
@@ -1078,7 +1173,7 @@ class Scheduler {
                     }
                 if (part.kind == kRotKept) {
                     part.u = double(1.0L + ld(x.t) * x.t);
-                    uniform_ -= 0.5L * std::log(ld(part.u));  // the pair's determinant as it is rounded
+                    uniform_ -= lost + 0.5L * (part.u / (1.0L + ld(x.t) * x.t) - 1.0L);  // the determinant as it is rounded
                 } else {
                     pend[low] -= lost;
                 }

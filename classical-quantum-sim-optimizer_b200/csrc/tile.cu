@@ -1291,7 +1291,15 @@ std::vector<TilePass> plan_tiles(const std::vector<Operation>& ops, size_t begin
     // A seed's own qubits are always allowed; the cap applies to the rest.
     TileShape sh{m, n, pinned, std::max(opt.spread_bit, 0), opt.max_spread >= 0 ? opt.max_spread : INT_MAX,
                  std::max(opt.inflight_bits, 0), size_t(std::max(opt.max_pass_ops, 0))};
-    const std::vector<PassChoice> chosen = choose_passes(g, sh, std::max(1, opt.seeds), beam);
+    std::vector<PassChoice> chosen;
+    if (m == n && sh.max_ops == 0 && opt.max_spread < 0) {
+        // The tile is the register: one pass takes every operation.
+        chosen.resize(1);
+        chosen[0].T = n == 64 ? ~uint64_t(0) : (uint64_t(1) << n) - 1;
+        for (size_t i = 0; i < N; i++) chosen[0].taken.push_back(i);
+    } else {
+        chosen = choose_passes(g, sh, std::max(1, opt.seeds), beam);
+    }
     for (const PassChoice& pc : chosen) {
         std::vector<char> inT(size_t(n), 0);
         for (int q = 0; q < n; q++) inT[size_t(q)] = char((pc.T >> q) & 1);
