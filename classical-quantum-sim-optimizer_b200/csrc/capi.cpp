@@ -972,7 +972,8 @@ int dq_rotation_plan_dump(const char* json, size_t len, int tile_qubits, char** 
         o.pinned_low = rotation_pinned_low(ops, 0, ops.size(), int(n), tile_qubits);
         std::vector<double2> pool;
         auto passes = plan_tiles(ops, 0, ops.size(), int(n), o, &pool);
-        std::string s = "{\"n\":" + std::to_string(n) + ",\"passes\":[";
+        std::string s = "{\"n\":" + std::to_string(n) + ",\"register_phases_quicker\":" +
+                        (register_phases_quicker(ops, 0, ops.size(), int(n)) ? "true" : "false") + ",\"passes\":[";
         auto list = [&](const char* name, auto begin, auto end) {
             s += std::string(",\"") + name + "\":[";
             for (auto i = begin; i != end; ++i) s += (i == begin ? "" : ",") + std::to_string(*i);

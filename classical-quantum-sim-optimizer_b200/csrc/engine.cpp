@@ -630,7 +630,8 @@ void Executor::lower_segment(const std::vector<Operation>& ops, size_t begin, si
         }
         return;
     }
-    const bool rotations = cfg_.rotations && !cfg_.c64 && !cfg_.model;
+    const bool rotations = cfg_.rotations && !cfg_.c64 && !cfg_.model &&
+                           !(cfg_.one_state && register_phases_quicker(ops, begin, end, cfg_.n));
     o.keep_raw = rotations;
     o.targets_only = rotations && rotation_targets_only(ops, begin, end, cfg_.n, cfg_.tile_m);
     if (rotations) o.pinned_low = rotation_pinned_low(ops, begin, end, cfg_.n, cfg_.tile_m);

@@ -168,6 +168,9 @@ struct ExecConfig {
     // complex128 passes run as Pauli rotations (rotations.hpp) wherever every
     // operation of the pass has that form; the others in register phases.
     bool rotations = false;
+    // It runs on one state at a time, in tiles of the default size: small registers then
+    // take whichever form has the shorter chain (register_phases_quicker).
+    bool one_state = false;
     // Gate images and scratch from the pool on the stream the executor runs
     // on (which must outlive it): no device-wide wait when it goes.
     bool pooled = false;

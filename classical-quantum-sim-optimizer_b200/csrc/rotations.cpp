@@ -1285,6 +1285,55 @@ int rotation_pinned_low(const std::vector<Operation>& ops, size_t begin, size_t 
     return kPinnedLow;
 }
 
+bool register_phases_quicker(const std::vector<Operation>& ops, size_t begin, size_t end, int n) {
+    if (n > 11) return false;
+    // Microseconds of both forms beyond a launch, fitted to the device times of 18
+    // families of circuits (5 to 11 qubits, 10 and 30 layers, one B200).
+    double rotations = 0.0, ones = 0.0, multi = 0.0, size = 0.0;
+    std::vector<size_t> last(size_t(n), end);  // the last many-qubit operation on each qubit
+    for (size_t i = begin; i < end; i++) {
+        const Operation& op = ops[i];
+        const size_t nc = std::min<size_t>(op.controls.size(), 4);
+        switch (op.type) {
+            case Operation::One: {
+                if (nc > 0) {
+                    rotations += 0.8 * double(nc);
+                    break;
+                }
+                // Z rotations on both sides of the Y rotation, or one.
+                const cplx left = op.m[0][0] * cplx(op.m[1][0].re, -op.m[1][0].im);
+                const cplx right = op.m[0][0] * cplx(op.m[0][1].re, -op.m[0][1].im);
+                rotations += std::fabs(left.im) > 1e-15 && std::fabs(right.im) > 1e-15 ? 0.31 : 0.2;
+                break;
+            }
+            case Operation::X: {
+                const double by_controls[5] = {0.0, 0.0, 0.55, 1.7, 3.7};
+                rotations += by_controls[nc];
+                break;
+            }
+            case Operation::Swap: rotations += nc == 0 ? 0.0 : nc == 1 ? 0.65 : 1.7; break;
+            case Operation::Diagonal: rotations += 0.06 * double(op.qubits.size()); break;
+            default: rotations += 0.4; break;
+        }
+        const std::vector<uint64_t> qubits = op.touched();
+        size += double(qubits.size());
+        if (qubits.size() == 1) {
+            ones += 1.0;
+            continue;
+        }
+        // (one on the qubits of the one before is fused with it)
+        const size_t before = last[size_t(qubits[0])];
+        bool same = before != end && ops[before].touched().size() == qubits.size();
+        for (uint64_t q : qubits) same = same && last[size_t(q)] == before;
+        if (!same) multi += 1.0;
+        for (uint64_t q : qubits) last[size_t(q)] = i;
+    }
+    // Phases larger than a launch argument are read from device memory.
+    const double phases = (0.4 * multi + 0.12 * ones) * (size > 410.0 ? 1.75 : 1.0);
+    const double share = n <= 7 ? 0.86 : n <= 9 ? 0.9 : n == 10 ? 1.04 : 1.35;  // matrices take longer as the tile grows
+    return rotations > share * phases;
+}
+
 bool build_rotation_pass(const std::vector<Operation>& ops, const std::vector<int>& tile_qubits, int n,
                          RotProgram& out) {
     const int m = int(tile_qubits.size());

@@ -118,6 +118,16 @@ bool rotation_targets_only(const std::vector<Operation>& ops, size_t begin, size
 // where an operation has no rotation form or touches more than the tile has left.
 int rotation_pinned_low(const std::vector<Operation>& ops, size_t begin, size_t end, int n, int m);
 
+// Whether register phases (phased.hpp) are expected to take less time than rotation
+// passes for ops[begin, end) on one state of n qubits that is a single tile. One or
+// two warps then run all of it, and what counts is the number of rotations and
+// tables in their chain against the number of fused two-qubit matrices. Register
+// phases and rotations on 9 qubits in 30 layers: CU3 0.074 and 0.133 ms, C4X and RY 0.092
+// and 0.194, CX and U3 0.150 and 0.124, CZ and RY RZ 0.278 and 0.102. From 12 qubits on, and where
+// several states fill the device, rotations are quicker or within 3 % (12-qubit CU3 of
+// 30 layers excepted, 0.178 and 0.209).
+bool register_phases_quicker(const std::vector<Operation>& ops, size_t begin, size_t end, int n);
+
 // Plans the pass `ops` over `tile_qubits` (ascending) of an n-qubit state.
 // Targets and swapped qubits are tile qubits; controls and diagonal qubits may
 // lie outside, where the tile's index gives their value.  False when an

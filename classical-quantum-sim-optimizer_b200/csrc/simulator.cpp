@@ -154,6 +154,7 @@ ExecConfig exec_config(const Options& o, uint64_t n, bool force_per_gate, const 
     // The default complex128 passes are Pauli rotations; an explicit fusion
     // width asks for fused matrices of that width.
     c.rotations = !c.c64 && o.fusion_width == 0;
+    c.one_state = o.tile_qubits == 0;
     c.pooled = true;  // a simulator's executors run on its device's stream
     c.n = int(n);
     return c;
@@ -463,7 +464,9 @@ ShotOutput Simulator::run_shots(const std::vector<Operation>& ops, uint64_t n, u
     st.allocate(int(n), workers, ncb, c64, *dev_);
     const size_t begin = cache_prefix ? prefix_end : 0;
     if (!sp.rest || sp.rest_begin != begin) {
-        sp.rest = std::make_unique<Executor>(ops, begin, ops.size(), exec_config(opt_, n));
+        ExecConfig c = exec_config(opt_, n);
+        c.one_state = false;
+        sp.rest = std::make_unique<Executor>(ops, begin, ops.size(), c);
         sp.rest_begin = begin;
     }
     Executor& ex = *sp.rest;

@@ -473,3 +473,33 @@ def test_a_phase_fits_a_launch_argument():
     for p in _core.rotation_plan_dump(Circuit(n, ins + ins).model_dump_json(), 12)["passes"]:
         assert p["ok"]
         assert all(len(part["words"]) // 4 <= 1980 for part in p.get("parts", [p]))
+
+
+def ring(n, layers, kind):
+    """Layers of RY on every qubit and one gate of `kind` on every third (of three qubits: neighbours)."""
+    ins = []
+    for layer in range(layers):
+        ins += [inst("ry", qubit=q, theta=0.3 + q + layer) for q in range(n)]
+        for q in range(layer % 3, n - 2, 3):
+            ins.append({"cz": inst("cz", control=q, target=q + 1), "cu3": inst("cu3", control=q, target=q + 2, theta=0.4, phi=1.1, lam=q),
+                        "ccx": inst("ccx", control1=q, control2=q + 1, target=q + 2),
+                        "rxx": inst("rxx", a=q, b=q + 2, theta=0.7)}[kind])
+    return Circuit(n, ins)
+
+
+@pytest.mark.parametrize("n,kind,quicker", [(5, "cu3", True), (9, "cu3", True), (11, "cu3", True), (12, "cu3", False),
+                                            (20, "cu3", False), (8, "ccx", True), (8, "rxx", True), (9, "cz", False)])
+def test_the_form_of_small_registers(n, kind, quicker):
+    assert _core.rotation_plan_dump(ring(n, 6, kind).model_dump_json(), 12)["register_phases_quicker"] == quicker
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [5, 8, 9, 10, 11, 12])
+@pytest.mark.parametrize("kind", ["cu3", "ccx", "rxx", "cz"])
+def test_both_forms_of_small_registers(n, kind):
+    """The default against register phases (an explicit fusion width), rotations (an explicit tile) and the oracle."""
+    c = ring(n, 6, kind)
+    want = oracle_state(c)
+    for options in ({}, {"fusion_width": 2}, {"tile_qubits": 12}):
+        got = dqsim.StatevectorSimulator(seed=1, **options).simulate(c).statevector
+        assert np.max(np.abs(got - want)) <= 1e-13, options
