@@ -592,6 +592,42 @@ __global__ void __launch_bounds__(kMargThreads, 2)
     }
 }
 
+// Small states, which L2 holds and which few CTAs would read by chunks: a group of
+// 2^G_bits threads per output gathers its terms, then adds them in a fixed order.
+// A query of 8 of 16 qubits takes 45 us, 55 by chunks, of 2 of 12 qubits 35 and 42, of 10 of
+// 20 qubits 96 and 105. Up to four terms a thread; with eight (1 of 12 qubits, 4 of 15) the
+// chunks are 1 to 3 us quicker, and from 21 qubits on they are for nearly all selections.
+constexpr int kGatherQubits = 20, kGatherBits = 8;
+constexpr uint64_t kGatherTerms = 4;
+
+struct GatherPlan {
+    int k, G_bits;
+    uint8_t q[64];   // selected qubits, output bit k - 1 first
+    uint64_t rest;   // the others
+};
+
+template <typename V>
+__global__ void __launch_bounds__(256) k_marginal_gather(const V* __restrict__ s, int n, const __grid_constant__ GatherPlan p,
+                                                        double* __restrict__ out, uint64_t nout) {
+    __shared__ double sm[256];
+    const int G = 1 << p.G_bits, lane = threadIdx.x & (G - 1);
+    const uint64_t j = (uint64_t(blockIdx.x) * 256 + threadIdx.x) >> p.G_bits;
+    double acc = 0.0;
+    if (j < nout) {
+        uint64_t base = 0;
+        for (int t = 0; t < p.k; t++) base |= ((j >> (p.k - 1 - t)) & 1) << p.q[t];
+        const uint64_t terms = uint64_t(1) << (n - p.k);
+        for (uint64_t r = lane; r < terms; r += G) acc += dev::norm2(s[base | deposit_mask(r, p.rest)]);
+    }
+    sm[threadIdx.x] = acc;
+    __syncthreads();
+    for (int w = G >> 1; w > 0; w >>= 1) {
+        if (lane < w) sm[threadIdx.x] += sm[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (lane == 0 && j < nout) out[j] = sm[threadIdx.x];
+}
+
 // A CTA adds 32 outputs, eight threads each: thread y the parts y, y + 8, ...,
 // then the eight in order (one thread each took 17 us for 256 outputs of 1,024 parts).
 __global__ void __launch_bounds__(256) k_marginal_parts(const double* __restrict__ parts, uint64_t nout, int count,
@@ -1141,14 +1177,39 @@ MarginalPlan marginal_plan(int n, const std::vector<int>& qubits) {
 }
 }  // namespace
 
+namespace {
+bool gathers(int n, const std::vector<int>& qubits) {
+    const int free = n - int(qubits.size());
+    return n <= kGatherQubits && (uint64_t(1) << std::max(0, free - kGatherBits)) <= kGatherTerms;
+}
+}  // namespace
+
 size_t marginal_scratch(int n, const std::vector<int>& qubits) {
+    if (gathers(n, qubits)) return 0;
     const MarginalPlan p = marginal_plan(n, qubits);
     return p.parts_bits ? size_t(1) << (p.parts_bits + int(qubits.size())) : 0;
 }
 
 void marginal(const Batch& b, const std::vector<int>& qubits, double* out, double* scratch) {
-    const MarginalPlan p = marginal_plan(b.n, qubits);
     const uint64_t nout = uint64_t(1) << qubits.size();
+    if (gathers(b.n, qubits)) {
+        GatherPlan g{};
+        g.k = int(qubits.size());
+        g.G_bits = std::min(kGatherBits, b.n - g.k);
+        g.rest = (uint64_t(1) << b.n) - 1;
+        for (int t = 0; t < g.k; t++) {
+            g.q[t] = uint8_t(qubits[size_t(t)]);
+            g.rest &= ~(uint64_t(1) << qubits[size_t(t)]);
+        }
+        const unsigned grid = blocks_for(nout << g.G_bits, 256);
+        if (b.c64)
+            k_marginal_gather<float2><<<grid, 256, 0, b.stream>>>(static_cast<const float2*>(b.amps), b.n, g, out, nout);
+        else
+            k_marginal_gather<double2><<<grid, 256, 0, b.stream>>>(static_cast<const double2*>(b.amps), b.n, g, out, nout);
+        check_launch("marginal");
+        return;
+    }
+    const MarginalPlan p = marginal_plan(b.n, qubits);
     const unsigned grid = blocks_for(uint64_t(1) << (p.kh + p.parts_bits), 1);
     double* to = p.parts_bits ? scratch : out;
     if (b.c64)

@@ -47,3 +47,15 @@ def test_marginals(n, precision):
         table = r.probabilities(qubits)
         got[list(table)] = list(table.values())
         np.testing.assert_allclose(got, reference(psi, n, qubits), atol=1e-13, rtol=0, err_msg=str(qubits))
+
+
+@pytest.mark.parametrize("n,k", [(3, 3), (10, 0), (11, 1), (12, 1), (12, 2), (13, 3), (14, 3), (18, 8), (20, 10), (20, 9), (21, 11)])
+def test_marginals_where_gathering_meets_chunks(n, k):
+    """Up to 20 qubits and ten unselected ones, and just beyond either."""
+    r = dqsim.StatevectorSimulator(seed=1).simulate(hea(n, 2, seed=n))
+    psi = r.statevector
+    qubits = [int(q) for q in np.random.default_rng(100 * n + k).choice(n, size=k, replace=False)]
+    got = np.zeros(1 << k)
+    table = r.probabilities(qubits)
+    got[list(table)] = list(table.values())
+    np.testing.assert_allclose(got, reference(psi, n, qubits), atol=1e-13, rtol=0)
