@@ -372,8 +372,12 @@ BatchRun::BatchRun(Simulator& sim, const std::vector<std::string>& texts, uint64
             cfg.c64 = true;
             cfg.n = int(c.n);
             c.fused = std::make_unique<Executor>(ops, 0, prefix, cfg);
-        } else if (c.fuse == kTuneRotations && !c64_ && c.n >= uint64_t(kRotMinTile)) {
-            // Rotation passes, run the same way.
+        } else if (c.fuse == kTuneRotations && !c64_ && c.n >= uint64_t(kRotMinTile) &&
+                   !register_phases_quicker(ops, 0, prefix, int(c.n))) {
+            // Rotation passes, run the same way, but for small circuits of long chains of
+            // rotations: those stay in the persistent kernel. 40 CU3 circuits of 4 to 8 qubits
+            // 53 us there, 67 on the side streams, 200 of 6 to 12 qubits 110 and 212 (each form where
+            // it is the quicker one: 94); 64 CZ ansatz circuits of 6 to 11 qubits 170 and 69.
             ExecConfig cfg;
             cfg.tiled = true;
             cfg.rotations = true;

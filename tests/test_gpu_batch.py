@@ -134,3 +134,27 @@ def test_circuits_without_gates(sizes, gates, precision):
                 want = zz_of(b.statevector(i, n))
                 assert abs(zz[i] - want) <= (1e-12 if precision == "complex128" else 1e-6)
                 assert sum(b.counts(i).values()) == 100
+
+
+def test_small_circuits_in_either_form():
+    """Rotation passes on side streams and, where their chain is the longer one, the persistent kernel, in one batch."""
+    from helpers import Circuit, inst
+
+    cs = []
+    for n in (5, 8, 11, 12, 13):
+        for kind in ("cu3", "cz"):
+            ins = [inst("ry", qubit=q, theta=0.3 + q) for q in range(n)]
+            for q in range(n - 1):
+                ins.append(inst("cu3", control=q, target=q + 1, theta=0.4, phi=1.1, lam=q) if kind == "cu3" else
+                           inst("cz", control=q, target=q + 1))
+            cs.append(Circuit(n, ins + ins + [inst("measure", qubit=q, cbit=q) for q in range(n)], n))
+    quicker = [_core.rotation_plan_dump(Circuit(n, c.data["instructions"][:-n]).model_dump_json())["register_phases_quicker"]
+               for c, n in zip(cs, (5, 5, 8, 8, 11, 11, 12, 12, 13, 13))]
+    assert quicker == [True, False] * 3 + [False] * 4
+    b = _core.BatchedCircuits(dqsim.StatevectorSimulator(seed=9), cs, shots=100)
+    for use_graph in (False, True):
+        b.run(use_graph=use_graph)
+        for i, c in enumerate(cs):
+            n = c.data["qregs"]["q"]["size"]
+            want = o.OracleSimulator(seed=1).simulate(Circuit(n, c.data["instructions"][:-n])).statevector
+            assert np.max(np.abs(b.statevector(i, n) - want)) <= 1e-12
