@@ -479,9 +479,10 @@ constexpr ld kMaxOwed = 200.0L;  // rotations may leave amplitudes e^200 too lar
 constexpr int kWindow = 128;  // items a phase chooses among
 // Rotations a phase may hold: its words then fit a launch argument whatever the
 // circuit. A rotation takes at most 20 (its own two, a step, a table before it
-// with another), each other item of the window 6, the phase itself 39.
-constexpr int kPhaseRotations = 83;
-static_assert(20 * kPhaseRotations + 6 * (kWindow - kPhaseRotations) + 39 <= kRotParamWords);
+// with another), each other item of the window 6 (an angle and a modulus of a slot: a mask
+// word, a factor and a step each), the phase itself 56 (its head, three more tables, two to fetch ahead).
+constexpr int kPhaseRotations = 82;
+static_assert(20 * kPhaseRotations + 6 * (kWindow - kPhaseRotations) + 56 <= kRotParamWords);
 // Below this many qubits half of them: planning then takes a third less time,
 // where it is most of a call, for at most 3 % longer programs (either way).
 constexpr int kWideQubits = 20;
@@ -1317,8 +1318,8 @@ bool register_phases_quicker(const std::vector<Operation>& ops, size_t begin, si
         }
         const std::vector<uint64_t> qubits = op.touched();
         size += double(qubits.size());
-        if (qubits.size() == 1) {
-            ones += 1.0;
+        if (qubits.size() <= 1) {
+            ones += double(qubits.size());
             continue;
         }
         // (one on the qubits of the one before is fused with it)

@@ -503,3 +503,12 @@ def test_both_forms_of_small_registers(n, kind):
     for options in ({}, {"fusion_width": 2}, {"tile_qubits": 12}):
         got = dqsim.StatevectorSimulator(seed=1, **options).simulate(c).statevector
         assert np.max(np.abs(got - want)) <= 1e-13, options
+
+
+@pytest.mark.gpu
+def test_parts_of_a_program_with_many_tiles_to_an_sm():
+    """40 layers on 12 of 22 qubits: parts with and without teams, intermediate ones in place."""
+    c = Circuit(22, brickwork(12, 40, seed=3, measure=False).data["instructions"])
+    passes = _core.rotation_plan_dump(c.model_dump_json(), 12)["passes"]
+    assert any(len(p.get("parts", [])) > 1 for p in passes)
+    assert np.max(np.abs(dqsim.StatevectorSimulator(seed=1).simulate(c).statevector - oracle_state(c))) <= 1e-12
